@@ -7,7 +7,7 @@
 // epilogue read tile t while the MMAs of tile t+1 run.  Nothing of the n x n
 // score matrix is written to HBM: each epilogue thread owns one query row,
 // reads its 256 scores straight from TMEM and offers the few that beat its
-// row threshold to a thread-private candidate buffer (common.cuh).
+// row threshold to a thread-private key set (common.cuh).
 //
 // Warp roles (192 threads):
 //   warp 0      TMA producer (one elected lane, no multicast)
@@ -45,6 +45,7 @@
 // src/nndescent/int8.rs:15-21 for the int8 dissimilarity).
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -142,8 +143,8 @@ constexpr int kModeJaccard = 2;  // 0/1 int8 rows: intersection counts, -(inter 
 // -2^30 keeps score - threshold free of overflow.
 constexpr int32_t kIntOpen = -(1 << 30);
 
-template <int MODE>
-__device__ __forceinline__ uint32_t pass_threshold(const KeyHeap& heap, int32_t pa) {
+template <int MODE, class Keys>
+__device__ __forceinline__ uint32_t pass_threshold(const Keys& heap, int32_t pa) {
   const uint64_t t = heap.threshold();
   if (MODE == kModeInt8) {
     if (t == kKeyInf) return uint32_t(kIntOpen);
@@ -201,9 +202,9 @@ __device__ __forceinline__ uint32_t pick(const uint32_t (&v)[32], int j) {
 // chunk's values stay in registers; a survivor's value is picked by a select
 // tree (survivors are rare once the heap is full).  Bit 31 - j of `mask`
 // stands for column j (the order chunk_mask builds).
-template <int MODE>
+template <int MODE, class Keys>
 __device__ __forceinline__ void offer_chunk(const uint32_t (&v)[32], uint32_t mask, int64_t col0, int64_t n_k,
-                                            bool self_mode, int64_t q, KeyHeap& heap, uint32_t& thr, int32_t pa,
+                                            bool self_mode, int64_t q, Keys& heap, uint32_t& thr, int32_t pa,
                                             const int32_t* __restrict__ pc, const int32_t* ids = nullptr,
                                             float seed = -__builtin_huge_valf()) {
   while (mask) {
@@ -700,7 +701,8 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       const int64_t qg = v.q_self ? (valid ? v.q_self_base + v.q_self[q] : -1) : v.q_row0 + q;
       // symmetric mode: qg is the scanned row, qd its row of the data set (keys and outputs)
       const int32_t qd = kSym ? (valid ? p.sym_perm[q] : -1) : int32_t(qg);
-      KeyHeap heap;
+      // four groups: a binary heap, the other's registers would not fit
+      std::conditional_t<GROUPS == 4, KeyHeap, KeySet> heap;
       heap.init(hstore, v.keep);
       if (valid && v.self_mode && group == 0) heap.offer(make_key(-1.0f, qd));
       const int32_t pa = (MODE == kModeJaccard && valid) ? v.pc[qg] : 0;
@@ -733,8 +735,6 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           __syncwarp();
           tth = sthr + (ti & 1) * kTileThr;
         }
-        uint32_t va[32], vb[32];
-        tmem_ld_32x32b_x32(tbase, va);
         // One chunk of 32 columns.  Symmetric mode: key rows before the
         // block's own (the first tile of an odd block) belong to the block
         // before; those past the block also feed their own rows' mailboxes.
@@ -753,19 +753,30 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             offer_chunk<MODE>(vv, chunk_mask<MODE>(vv, thr), col, v.n_k, v.self_mode, qg, heap, thr, pa, v.pc);
           }
         };
+        // One group: a chunk is processed while the next is read.  Several
+        // groups: their warps hide each other's TMEM latency, and a second
+        // chunk's registers would not fit (a register that a TMEM load is
+        // still writing must not be spilled).
+        uint32_t va[32];
+        if constexpr (GROUPS == 1) {
+          uint32_t vb[32];
+          tmem_ld_32x32b_x32(tbase, va);
 #pragma unroll 1
-        for (int c = 0; c < NCH; c += 2) {
-          float um0 = 0.0f, um1 = 0.0f;
-          if (kSym) {
-            um0 = tth[BN + col_base / 32 + c];
-            um1 = tth[BN + col_base / 32 + c + 1];
+          for (int c = 0; c < NCH; c += 2) {
+            tmem_ld_wait();
+            tmem_ld_32x32b_x32(tbase + (c + 1) * 32, vb);
+            chunk(va, c, kSym ? tth[BN + col_base / 32 + c] : 0.0f);
+            tmem_ld_wait();
+            if (c + 2 < NCH) tmem_ld_32x32b_x32(tbase + (c + 2) * 32, va);
+            chunk(vb, c + 1, kSym ? tth[BN + col_base / 32 + c + 1] : 0.0f);
           }
-          tmem_ld_wait();
-          tmem_ld_32x32b_x32(tbase + (c + 1) * 32, vb);
-          chunk(va, c, um0);
-          tmem_ld_wait();
-          if (c + 2 < NCH) tmem_ld_32x32b_x32(tbase + (c + 2) * 32, va);
-          chunk(vb, c + 1, um1);
+        } else {
+#pragma unroll 1
+          for (int c = 0; c < NCH; c++) {
+            tmem_ld_32x32b_x32(tbase + c * 32, va);
+            tmem_ld_wait();
+            chunk(va, c, kSym ? tth[BN + col_base / 32 + c] : 0.0f);
+          }
         }
         tc_fence_before();
         if (kPair && !leader) mbar_arrive_cluster(a ? tempty_c1 : tempty_c0);
@@ -792,7 +803,10 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
       }
       if (group == 0 && valid) {
-        const int got = heap.finish();
+        // The rerank takes candidates in any order: only final output, and the
+        // mailbox merge's input, is sorted (60 keys took ~45k cycles a block).
+        const uint64_t worst = heap.threshold();
+        const int got = v.final_mode || kSym ? heap.finish() : heap.size;
         const int64_t orow = (kSym ? int64_t(qd) : q) * v.keep;  // symmetric mode: rows of the data set
         for (int j = 0; j < v.keep; j++) {
           float raw = kHeapInf;
@@ -808,8 +822,8 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           v.out_idx[orow + j] = idx;
           if (v.out_raw) v.out_raw[orow + j] = raw;
           if (v.final_mode && v.out_dist) v.out_dist[orow + j] = transform_raw(v.dtype, raw);
-          if (v.out_bound && j == v.keep - 1) v.out_bound[q] = raw;
         }
+        if (v.out_bound) v.out_bound[q] = got == v.keep ? from_orderable(uint32_t(worst >> 32)) : kHeapInf;
       }
       if (GROUPS > 1) epilogue_sync(GROUPS * 128);  // heaps are reused by the next block
     }
