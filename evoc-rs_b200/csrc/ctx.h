@@ -72,6 +72,7 @@ struct evoc_gpu_ctx {
   evoc::DevBuf sym;
   int64_t sym_min_rows = 0;
   int64_t sym_sample = 0, sym_cap = 0, sym_max_offers = 0, sym_overflow = 0;
+  evoc::DevBuf prune;  // exact self-joins over tile lists (prune.cu): rows in scanned order, centres, lists
   evoc::DevBuf batch_ws, batch_tab;  // batches: per-request work arena, device tables
   void* batch_host = nullptr;  // pinned staging of the tables
   size_t batch_host_bytes = 0;

@@ -28,6 +28,7 @@ enum CtxBuf {
   kBufCert,      // 16-bit form: certificate norms, bounds, failed-row lists
   kBufRepair,    // 16-bit form: rescan arena for rows that failed the certificate
   kBufSym,       // 16-bit form: symmetric scan arena (mailboxes, thresholds, sample rows)
+  kBufPrune,     // exact self-joins over tile lists: rows in scanned order, centres, lists
   kBufCount
 };
 

@@ -143,22 +143,33 @@ int64_t pivot_count(int64_t n) {
   return n_piv;
 }
 
-int locality_order(evoc_gpu_ctx* ctx, const Job& j, const void* rows, int64_t row_bytes, bool int8,
-                   bool sorted_cells, int half_type = evoc::kHalfF16) {
-  Stage st(ctx, "pivot_order");
-  const int64_t n_piv = pivot_count(j.n);
+// n_piv evenly spaced rows as pivots (ctx->pivots, room for more_rows rows past them).
+int gather_pivots(evoc_gpu_ctx* ctx, int64_t n, const void* rows, int64_t row_bytes, int64_t n_piv,
+                  int64_t more_rows = 0) {
   const int64_t piv_rows = evoc::padded_rows(n_piv);
-  EVOC_TRY(ctx->pivots.ensure(size_t(piv_rows * row_bytes)), "alloc pivots");
+  EVOC_TRY(ctx->pivots.ensure(size_t((piv_rows + more_rows) * row_bytes)), "alloc pivots");
   EVOC_TRY(cudaMemsetAsync(ctx->pivots.p, 0, size_t(piv_rows * row_bytes), ctx->stream), "clear pivots");
-  EVOC_TRY(evoc::launch_gather_pivots(rows, row_bytes, j.n, n_piv, ctx->pivots.p, ctx->sms, ctx->stream),
+  EVOC_TRY(evoc::launch_gather_pivots(rows, row_bytes, n, n_piv, ctx->pivots.p, ctx->sms, ctx->stream),
            "gather pivots");
-  const int grid = scan_grid(ctx, j.nq);
-  EVOC_TRY(ctx->labels.ensure(size_t(j.nq) * 4), "alloc labels");
-  EVOC_TRY(evoc::launch_tc_scan(int8 ? evoc::kScanInt8 : evoc::kScanHalf, rows, evoc::padded_rows(j.n), j.r0, j.nq,
-                                ctx->pivots.p, piv_rows, n_piv,
-                                row_bytes, 1, nullptr, grid, 0, 0, 0, ctx->labels.as<int32_t>(), nullptr, nullptr,
-                                j.status, ctx->timeout_ns, nullptr, ctx->stream, -1, half_type),
+  ctx->launches += 1;
+  return EVOC_OK;
+}
+
+// The nearest of n_piv pivots at `pivots` for rows r0 .. r0+nq-1 of a rows_mem-row matrix, with the
+// dissimilarities where raw is given.
+int nearest_pivots(evoc_gpu_ctx* ctx, const void* rows, int64_t rows_mem, int64_t r0, int64_t nq, int64_t row_bytes,
+                   bool int8, int half_type, const void* pivots, int64_t n_piv, int32_t* label, float* raw,
+                   int* status) {
+  EVOC_TRY(evoc::launch_tc_scan(int8 ? evoc::kScanInt8 : evoc::kScanHalf, rows, rows_mem, r0, nq, pivots,
+                                evoc::padded_rows(n_piv), n_piv, row_bytes, 1, nullptr, scan_grid(ctx, nq), 0, 0, 0,
+                                label, raw, nullptr, status, ctx->timeout_ns, nullptr, ctx->stream, -1, half_type),
            "pivot scan");
+  ctx->launches += 1;
+  return EVOC_OK;
+}
+
+// Counting sort of the rows by label into ctx->order.
+int order_by_pivot(evoc_gpu_ctx* ctx, const Job& j, int64_t n_piv, bool sorted_cells) {
   EVOC_TRY(ctx->order.ensure(size_t(j.nq) * 4), "alloc order");
   EVOC_TRY(ctx->hist.ensure(size_t(n_piv) * 4), "alloc hist");
   EVOC_TRY(ctx->cursor.ensure(size_t(n_piv) * 4), "alloc cursor");
@@ -166,7 +177,244 @@ int locality_order(evoc_gpu_ctx* ctx, const Job& j, const void* rows, int64_t ro
                                        ctx->cursor.as<int32_t>(), ctx->order.as<int32_t>(), sorted_cells, ctx->sms,
                                        ctx->stream),
            "order by pivot");
-  ctx->launches += sorted_cells ? 6 : 5;
+  ctx->launches += sorted_cells ? 4 : 3;
+  return EVOC_OK;
+}
+
+int locality_order(evoc_gpu_ctx* ctx, const Job& j, const void* rows, int64_t row_bytes, bool int8,
+                   bool sorted_cells, int half_type = evoc::kHalfF16) {
+  Stage st(ctx, "pivot_order");
+  const int64_t n_piv = pivot_count(j.n);
+  int rc = gather_pivots(ctx, j.n, rows, row_bytes, n_piv);
+  if (rc) return rc;
+  EVOC_TRY(ctx->labels.ensure(size_t(j.nq) * 4), "alloc labels");
+  rc = nearest_pivots(ctx, rows, evoc::padded_rows(j.n), j.r0, j.nq, row_bytes, int8, half_type, ctx->pivots.p, n_piv,
+                      ctx->labels.as<int32_t>(), nullptr, j.status);
+  return rc ? rc : order_by_pivot(ctx, j, n_piv, sorted_cells);
+}
+
+int32_t read_count(evoc_gpu_ctx* ctx, const int32_t* d_count, int* rc) {
+  int32_t v = 0;
+  cudaError_t e = cudaMemcpyAsync(&v, d_count, 4, cudaMemcpyDeviceToHost, ctx->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  if (e != cudaSuccess) *rc = cuda_fail(ctx, e, "read count");
+  return v;
+}
+
+// Exact self-joins over tile lists (prune.cu): at least kPruneMinRows rows, a
+// pivot per 512, at most 2,048, and as many more for the strays.
+constexpr int64_t kPruneMinRows = 16384;
+constexpr int64_t kStrayPivots = 2048;
+
+int64_t list_pivots(int64_t n) { return std::max<int64_t>(2, std::min<int64_t>(n / 512, 2048)); }
+
+// Tiles per group as a power of two: at most kPruneGroups groups.
+int prune_lg(int64_t n) {
+  int lg = 0;
+  while ((((n + 255) / 256 + (int64_t(1) << lg) - 1) >> lg) > evoc::kPruneGroups) lg++;
+  return lg;
+}
+
+struct PruneLayout {
+  size_t rows, centres, u, g, list, len, blocks, stats, seed, sq, rank, cells, second, total;
+  int lg;
+  int64_t groups, ld, group_rows;
+};
+
+// row_bytes: of the operand rows; xs_bytes: of the rows copied into scanned
+// order (the operand rows; binary data: the packed rows).
+PruneLayout prune_layout(int64_t n, int64_t row_bytes, int64_t xs_bytes) {
+  PruneLayout L{};
+  const int64_t piv = list_pivots(n) + kStrayPivots;
+  L.lg = prune_lg(n);
+  L.group_rows = int64_t(256) << L.lg;
+  L.groups = (n + L.group_rows - 1) / L.group_rows;
+  L.ld = round_up(std::max(L.groups, piv), 256);
+  size_t off = 0;
+  auto take = [&](size_t bytes) {
+    const size_t at = off;
+    off += (bytes + 255) / 256 * 256;
+    return at;
+  };
+  L.rows = take(size_t(evoc::padded_rows(n) * xs_bytes));
+  L.centres = take(size_t(round_up(L.groups, 256) * row_bytes));
+  L.u = take(size_t(L.groups * L.ld) * 4);
+  L.g = take(size_t(std::max(L.groups, piv) * L.ld) * 4);  // the pivots' similarities first
+  L.list = take(size_t(L.groups * L.groups) * 4);
+  L.len = take(size_t(L.groups) * 4);
+  L.blocks = take(size_t((n + 127) / 128) * 4);
+  L.stats = take(size_t(4 * L.groups) * 4 + 256);
+  L.seed = take(size_t(n) * 4);    // the pivot scan's dissimilarities first
+  L.sq = take(size_t(n) * 4);      // int8: squared norms; binary: popcounts in scanned order
+  L.rank = take(size_t(piv) * 4);
+  L.cells = take(size_t(2 * piv) * 4 + 256);
+  L.second = take(size_t(n) * 4);  // the strays' second labels
+  L.total = off;
+  return L;
+}
+
+// Whether a whole-graph request may take the lists: enough rows for them to
+// pay (16,384: 1.1 ms against 1.3 for the full scan at 384 features; below,
+// the plan's launches cost more than the scan), heaps in shared memory, rows
+// short enough for the group statistics.
+bool use_lists(int64_t n, int64_t r0, int64_t nq, int64_t keep, int64_t row_elems) {
+  return r0 == 0 && nq == n && n >= kPruneMinRows && keep <= n && evoc::tc_scan_list_feasible(int(keep)) &&
+         row_elems <= 51200;
+}
+
+// The lists are taken when a quarter of a sample of rows reaches this cosine
+// with its nearest pivot.  With a the cosine of a row and its group's centre,
+// the bound is at least 1 - a^2 and the rows' neighbours score about a^2, and
+// a^2 is about the cosine with a pivot of the same cluster: below a half
+// nothing can be skipped.  Binary rows differ from their centre by single bits,
+// whose number varies from row to row; their bound needs 0.8 (bit rows that
+// keep 0.66, 1,024 bits with a twentieth flipped, skip no tile at all).
+constexpr int64_t kFitSample = 2048;
+constexpr float kFitCosine = 0.5f, kFitCosineBits = 0.8f;
+
+// Plans the lists of a self-join of all rows and scans over them; *taken is
+// false when the rows call for the full scan.  rows: the operand rows in data-set order (binary
+// data: the 0/1 expansion in ctx->xb, which is rewritten in scanned order from
+// the packed rows `packed`).  final_mode etc. as launch_tc_scan's; bound: by
+// data-set row, or null.
+int list_scan(evoc_gpu_ctx* ctx, const Job& j, int mode, const void* rows, int64_t row_bytes, int half, int keep,
+              int final_mode, int dtype, int32_t* idx, float* raw, float* dist, float* bound, const char* stage,
+              bool* taken, const void* packed = nullptr, int64_t ldp = 0, int64_t nbytes = 0) {
+  *taken = false;
+  const bool binary = mode == evoc::kScanJaccard;
+  const int64_t n = j.n, rows_mem = evoc::padded_rows(n);
+  const PruneLayout L = prune_layout(n, row_bytes, binary ? ldp : row_bytes);
+  EVOC_TRY(ctx->prune.ensure(L.total), "alloc tile lists");
+  uint8_t* b = ctx->prune.as<uint8_t>();
+  auto f = [&](size_t off) { return reinterpret_cast<float*>(b + off); };
+  auto i32 = [&](size_t off) { return reinterpret_cast<int32_t*>(b + off); };
+  const int gemm = mode == evoc::kScanHalf ? evoc::kScanHalf : evoc::kScanInt8;
+  const int64_t piv1 = list_pivots(n);
+  int64_t piv2 = 0;
+  {
+    Stage st(ctx, "scan_order");
+    const bool int8 = gemm == evoc::kScanInt8;
+    int rc = gather_pivots(ctx, n, rows, row_bytes, piv1, kStrayPivots + 256);
+    if (rc) return rc;
+    const int32_t* sq = nullptr;
+    if (mode == evoc::kScanInt8) {
+      EVOC_TRY(evoc::launch_int8_sq(rows, row_bytes, n, i32(L.sq), ctx->sms, ctx->stream), "row norms");
+      ctx->launches += 1;
+      sq = i32(L.sq);
+    } else if (binary) {
+      sq = ctx->popc.as<int32_t>();
+    }
+    EVOC_TRY(cudaMemsetAsync(b + L.cells, 0, size_t(2 * piv1 + 2) * 4, ctx->stream), "clear cells");
+    EVOC_TRY(ctx->labels.ensure(size_t(n) * 4), "alloc labels");
+    int32_t* label = ctx->labels.as<int32_t>();
+    // the sample's rows pass through the place of the scanned rows
+    const int64_t stride = n / kFitSample;
+    EVOC_TRY(evoc::launch_gather_strided_rows(rows, row_bytes, stride, kFitSample, kFitSample, b + L.rows, ctx->sms,
+                                              ctx->stream),
+             "sample rows");
+    rc = nearest_pivots(ctx, b + L.rows, kFitSample, 0, kFitSample, row_bytes, int8, half, ctx->pivots.p, piv1, label,
+                        f(L.seed), j.status);
+    if (rc) return rc;
+    EVOC_TRY(evoc::launch_sample_fit(label, f(L.seed), int(kFitSample), stride, n, int(piv1), sq,
+                                     binary ? kFitCosineBits : kFitCosine, i32(L.cells), ctx->stream),
+             "sample fit");
+    ctx->launches += 2;
+    const int32_t close = read_count(ctx, i32(L.cells), &rc);
+    if (rc || close < kFitSample / 4) return rc;
+    *taken = true;
+    rc = nearest_pivots(ctx, rows, rows_mem, 0, n, row_bytes, int8, half, ctx->pivots.p, piv1, label, f(L.seed),
+                        j.status);
+    if (rc) return rc;
+    EVOC_TRY(ctx->order.ensure(size_t(n) * 4), "alloc order");
+    int32_t* strays = ctx->order.as<int32_t>();  // until the order is known
+    const evoc::CellFit fit{f(L.cells) + 2, i32(L.cells) + 2 + piv1, i32(L.cells) + 1};
+    EVOC_TRY(evoc::launch_cell_fit(label, f(L.seed), n, int(piv1), sq, fit, strays, ctx->sms, ctx->stream), "cell fit");
+    ctx->launches += 2;
+    const int32_t n_strays = read_count(ctx, i32(L.cells) + 1, &rc);
+    if (rc) return rc;
+    // their operand rows are gathered in the arena's place for the scanned rows (binary data: packed
+    // rows' place, which holds an eighth of the 0/1 rows; strays past that keep their first cell)
+    const int64_t room = rows_mem * (binary ? ldp : row_bytes) / row_bytes / 256 * 256;
+    const int64_t count = std::min<int64_t>(std::max(n_strays, 0), std::min(n, room));
+    uint8_t* p2 = ctx->pivots.as<uint8_t>() + piv1 * row_bytes;  // right after the first pivots
+    if (count >= 32) {
+      piv2 = std::max<int64_t>(2, std::min<int64_t>(count / 64, kStrayPivots));
+      const int64_t crows = evoc::padded_rows(count);
+      void* q = b + L.rows;
+      EVOC_TRY(evoc::launch_gather_rows_list(rows, row_bytes, 0, strays, count, crows, q, ctx->sms, ctx->stream),
+               "stray rows");
+      EVOC_TRY(cudaMemsetAsync(p2, 0, size_t(evoc::padded_rows(piv2) * row_bytes), ctx->stream), "clear pivots");
+      EVOC_TRY(evoc::launch_gather_pivots(q, row_bytes, count, piv2, p2, ctx->sms, ctx->stream), "gather pivots");
+      rc = nearest_pivots(ctx, q, crows, 0, count, row_bytes, int8, half, p2, piv2, i32(L.second), nullptr, j.status);
+      if (rc) return rc;
+      EVOC_TRY(evoc::launch_stray_labels(strays, i32(L.second), count, int(piv1), int(piv2), label, ctx->sms,
+                                         ctx->stream),
+               "stray labels");
+      ctx->launches += 3;
+    }
+    const int64_t piv = piv1 + piv2, piv_mem = evoc::padded_rows(piv);
+    if (piv2 > 0 || piv_mem > evoc::padded_rows(piv1)) {
+      const int64_t end = piv1 + (piv2 > 0 ? evoc::padded_rows(piv2) : 0);
+      if (piv_mem > end)
+        EVOC_TRY(cudaMemsetAsync(ctx->pivots.as<uint8_t>() + end * row_bytes, 0, size_t((piv_mem - end) * row_bytes),
+                                 ctx->stream),
+                 "clear pivots");
+    }
+    EVOC_TRY(evoc::launch_centre_products(gemm, ctx->pivots.p, piv_mem, piv, ctx->pivots.p, piv_mem, row_bytes, half,
+                                          true, 256, f(L.g), L.ld, j.status, ctx->timeout_ns, ctx->sms, ctx->stream),
+             "pivot similarities");
+    EVOC_TRY(evoc::launch_prim_order(f(L.g), L.ld, int(piv), i32(L.rank), label, n, ctx->sms, ctx->stream),
+             "pivot order");
+    rc = order_by_pivot(ctx, j, piv, false);
+    if (rc) return rc;
+    EVOC_TRY(evoc::launch_gather_rows_list(binary ? packed : rows, binary ? ldp : row_bytes, 0,
+                                           ctx->order.as<int32_t>(), n, rows_mem, b + L.rows, ctx->sms, ctx->stream),
+             "rows in scanned order");
+    ctx->launches += 4;
+    if (binary) {
+      EVOC_TRY(evoc::launch_popcount_rows(b + L.rows, n, int(ldp / 4), i32(L.sq), ctx->sms, ctx->stream), "popcounts");
+      EVOC_TRY(evoc::launch_expand_bits(b + L.rows, n, ldp, nbytes, ctx->xb.p, rows_mem, row_bytes, ctx->sms,
+                                        ctx->stream),
+               "expand bits");
+      ctx->launches += 2;
+    }
+  }
+  const void* xs = binary ? ctx->xb.p : b + L.rows;
+  const int32_t* pc = binary ? i32(L.sq) : nullptr;
+  const evoc::PruneStats ps{f(L.stats), f(L.stats) + L.groups, f(L.stats) + 2 * L.groups, f(L.stats) + 3 * L.groups,
+                            reinterpret_cast<unsigned int*>(f(L.stats) + 4 * L.groups)};
+  {
+    Stage st(ctx, "tile_lists");
+    const int64_t crows = round_up(L.groups, 256);
+    EVOC_TRY(cudaMemsetAsync(b + L.centres, 0, size_t(crows * row_bytes), ctx->stream), "clear centres");
+    EVOC_TRY(evoc::launch_group_stats(gemm, xs, row_bytes, n, L.group_rows, int(L.groups), half, b + L.centres, ps,
+                                      ctx->stream),
+             "group statistics");
+    EVOC_TRY(cudaMemsetAsync(b + L.u, 0, size_t(L.groups * L.ld) * 4, ctx->stream), "clear maxima");
+    EVOC_TRY(evoc::launch_centre_products(gemm, xs, rows_mem, n, b + L.centres, crows, row_bytes, half, false,
+                                          L.group_rows, i32(L.u), L.ld, j.status, ctx->timeout_ns, ctx->sms,
+                                          ctx->stream),
+             "group maxima");
+    EVOC_TRY(evoc::launch_centre_products(gemm, b + L.centres, crows, L.groups, b + L.centres, crows, row_bytes, half,
+                                          true, L.group_rows, f(L.g), L.ld, j.status, ctx->timeout_ns, ctx->sms,
+                                          ctx->stream),
+             "centre products");
+    EVOC_TRY(evoc::launch_seeds(mode, xs, rows_mem, n, row_bytes, keep, half, ps.top, pc, f(L.seed), j.status,
+                                ctx->timeout_ns, scan_grid(ctx, n), ctx->stream),
+             "seeds");
+    EVOC_TRY(evoc::launch_prune_lists(mode, n, L.group_rows, int(L.groups), L.ld, i32(L.u), f(L.g), ps, f(L.seed),
+                                      int(row_bytes / 2), i32(L.list), i32(L.len), i32(L.blocks), ctx->stream),
+             "tile lists");
+    ctx->launches += 6;
+  }
+  Stage st(ctx, stage);
+  const evoc::ScanLists lists{ctx->order.as<int32_t>(), i32(L.list), i32(L.len), i32(L.blocks), f(L.seed),
+                              ctx->popc.as<int32_t>(), int(L.groups), L.lg};
+  const int grid = ctx->scan_per_block ? int((n + 127) / 128) : scan_grid(ctx, n);
+  EVOC_TRY(evoc::launch_tc_scan_list(mode, xs, rows_mem, n, row_bytes, keep, grid, final_mode, dtype, idx, raw, dist,
+                                     bound, j.status, ctx->timeout_ns, pc, ctx->stream, half, lists, ctx->delay_ns),
+           "list scan");
+  ctx->launches += 1;
   return EVOC_OK;
 }
 
@@ -300,14 +548,6 @@ int exact_rows(evoc_gpu_ctx* ctx, const RescanJob& j, const int32_t* list, int64
     ctx->launches += 1;
   }
   return EVOC_OK;
-}
-
-int32_t read_count(evoc_gpu_ctx* ctx, const int32_t* d_count, int* rc) {
-  int32_t v = 0;
-  cudaError_t e = cudaMemcpyAsync(&v, d_count, 4, cudaMemcpyDeviceToHost, ctx->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-  if (e != cudaSuccess) *rc = cuda_fail(ctx, e, "read certificate count");
-  return v;
 }
 
 // Whether `rows` failed rows take the exact FP32 pass directly.  The 16-bit
@@ -542,10 +782,16 @@ int run_bf16_rerank(evoc_gpu_ctx* ctx, const evoc_gpu_opts& opts, const Job& j, 
   const int grid = main_scan_grid(ctx, j.nq, int(C), variant);
   EVOC_TRY(ctx->cand.ensure(size_t(j.nq * C) * 4), "alloc candidates");
   const bool sym = use_symmetric(ctx, certify, j.n, j.r0, j.nq, C);
+  bool lists = !sym && use_lists(j.n, j.r0, j.nq, C, ldb);
+  if (lists) {
+    int rc = list_scan(ctx, j, evoc::kScanHalf, ctx->xb.p, ldb * 2, half, int(C), 0, 0, ctx->cand.as<int32_t>(),
+                       nullptr, nullptr, certify ? cf(CL.bound) : nullptr, "bf16_scan", &lists);
+    if (rc) return rc;
+  }
   if (sym) {
     int rc = symmetric_scan(ctx, j, half, ldb, rows, C, cf(CL.bound), cf(CL.hnorm), maxes);
     if (rc) return rc;
-  } else {
+  } else if (!lists) {
     Stage st(ctx, "bf16_scan");
     EVOC_TRY(ctx->scratch.ensure(scan_scratch_bytes(ctx, j.nq, C)), "alloc scratch");
     EVOC_TRY(evoc::launch_tc_scan(evoc::kScanHalf, ctx->xb.p, rows, j.r0, j.nq, ctx->xb.p, rows, j.n, ldb * 2, int(C),
@@ -557,8 +803,8 @@ int run_bf16_rerank(evoc_gpu_ctx* ctx, const evoc_gpu_opts& opts, const Job& j, 
   }
   const int32_t* order = nullptr;
   if (j.nq >= 65536) {
-    // the order only schedules the rerank (the symmetric scan computed it already)
-    if (!sym) {
+    // the order only schedules the rerank (the symmetric and the list scan computed it already)
+    if (!sym && !lists) {
       int rc = locality_order(ctx, j, ctx->xb.p, ldb * 2, false, false, half);
       if (rc) return rc;
     }
@@ -600,6 +846,12 @@ int run_bf16_rerank(evoc_gpu_ctx* ctx, const evoc_gpu_opts& opts, const Job& j, 
 }
 
 int run_int8(evoc_gpu_ctx* ctx, const Job& j, int64_t ldb) {
+  if (use_lists(j.n, j.r0, j.nq, j.keff, ldb)) {
+    bool taken = false;
+    const int rc = list_scan(ctx, j, evoc::kScanInt8, ctx->x.p, ldb, evoc::kHalfF16, j.keff, 1, EVOC_DTYPE_I8, j.idx,
+                             j.raw, j.dist, nullptr, "int8_scan", &taken);
+    if (rc || taken) return rc;
+  }
   Stage st(ctx, "int8_scan");
   const int variant = tuned_variant(ctx, evoc::kScanInt8, j.keff, ldb, j.n);
   const int grid = main_scan_grid(ctx, j.nq, j.keff, variant);
@@ -631,6 +883,12 @@ int run_jaccard_tc(evoc_gpu_ctx* ctx, const Job& j, int64_t ldb, int64_t nbytes)
     EVOC_TRY(evoc::launch_expand_bits(ctx->x.p, j.n, ldb, nbytes, ctx->xb.p, rows, lde, ctx->sms, ctx->stream),
              "expand bits");
     ctx->launches += 2;
+  }
+  if (use_lists(j.n, j.r0, j.nq, j.keff, lde)) {
+    bool taken = false;
+    const int rc = list_scan(ctx, j, evoc::kScanJaccard, ctx->xb.p, lde, evoc::kHalfF16, j.keff, 1, EVOC_DTYPE_U8,
+                             j.idx, j.raw, j.dist, nullptr, "jaccard_scan", &taken, ctx->x.p, ldb, nbytes);
+    if (rc || taken) return rc;
   }
   Stage st(ctx, "jaccard_scan");
   const int grid = scan_grid(ctx, j.nq);
@@ -1626,7 +1884,7 @@ void evoc_gpu_ctx_destroy(evoc_gpu_ctx* ctx) {
                     &ctx->out_raw,  &ctx->out_dist, &ctx->xb,   &ctx->cand,   &ctx->labels,
                     &ctx->order,    &ctx->hist,    &ctx->cursor, &ctx->pivots, &ctx->popc,
                     &ctx->g_idx,    &ctx->g_dist,  &ctx->g_sigma, &ctx->g_rho, &ctx->g_indptr,
-                    &ctx->g_indices, &ctx->g_data, &ctx->g_work, &ctx->nnd_work, &ctx->cert, &ctx->repair};
+                    &ctx->g_indices, &ctx->g_data, &ctx->g_work, &ctx->nnd_work, &ctx->cert, &ctx->repair, &ctx->prune};
   for (DevBuf* b : bufs) b->release();
   for (auto& g : ctx->batch_graphs) cudaGraphExecDestroy(g.exec);
   ctx->batch_ws.release();
@@ -1779,6 +2037,17 @@ void knn_buffer_needs(const evoc_gpu_ctx* ctx, const evoc_gpu_opts& opts, int32_
     b[kBufHist] = size_t(n_piv) * 4;
     b[kBufCursor] = size_t(n_piv) * 4;
   };
+  auto list_plan = [&](int64_t keep, int64_t row_bytes, int64_t elems, int64_t xs_bytes) {
+    if (!use_lists(n, 0, n, keep, elems)) return;
+    const int64_t piv = list_pivots(n);
+    auto at_least = [&](int buf, size_t bytes) { b[buf] = std::max(b[buf], bytes); };
+    at_least(kBufPivots, size_t((padded_rows(piv) + kStrayPivots + 256) * row_bytes));
+    at_least(kBufLabels, size_t(n) * 4);
+    at_least(kBufOrder, size_t(n) * 4);
+    at_least(kBufHist, size_t(piv + kStrayPivots) * 4);
+    at_least(kBufCursor, size_t(piv + kStrayPivots) * 4);
+    b[kBufPrune] = prune_layout(n, row_bytes, xs_bytes).total;
+  };
   auto nnd = [&]() {
     size_t sizes[kNndParts];
     b[kBufNnd] = nnd_work_sizes(n, int(keff), nnd_max_candidates(opts, int(keff)), sizes);
@@ -1800,6 +2069,7 @@ void knn_buffer_needs(const evoc_gpu_ctx* ctx, const evoc_gpu_opts& opts, int32_
       b[kBufScratch] = size_t(grid) * 256 * size_t(C) * 8;
       if (n >= 65536) locality(ldb * 2);
       if (use_symmetric(ctx, opts.certify != 0, n, 0, n, C)) b[kBufSym] = sym_layout(n, C, ldb).total;
+      else list_plan(C, ldb * 2, ldb, ldb * 2);
       if (opts.certify) {
         // the certificate and, should rows fail it, their rescans (bounded chunks)
         const int64_t C2 = second_pass_candidates(n, 256);  // the largest second pass
@@ -1821,6 +2091,7 @@ void knn_buffer_needs(const evoc_gpu_ctx* ctx, const evoc_gpu_opts& opts, int32_
     b[kBufX] = size_t(rows * ldb);
     if (form == EVOC_FORM_EXACT_INT) {
       b[kBufScratch] = size_t(grid) * 256 * size_t(keff) * 8;
+      list_plan(keff, ldb, ldb, ldb);
     } else if (form == EVOC_FORM_NNDESCENT) {
       locality(ldb);
       nnd();
@@ -1831,6 +2102,7 @@ void knn_buffer_needs(const evoc_gpu_ctx* ctx, const evoc_gpu_opts& opts, int32_
       b[kBufPopc] = size_t(n) * 4;
       b[kBufXb] = size_t(rows * expanded_row_bytes(dim));
       b[kBufScratch] = size_t(grid) * 256 * size_t(keff) * 8;
+      list_plan(keff, expanded_row_bytes(dim), expanded_row_bytes(dim), round_up(dim, 64));
     } else if (form == EVOC_FORM_POPCOUNT) {
       b[kBufPopc] = size_t(n) * 4;
     } else if (form == EVOC_FORM_NNDESCENT) {
@@ -1877,7 +2149,7 @@ void ctx_buffer_sizes(const evoc_gpu_ctx* ctx, CtxSizes* cur) {
   const DevBuf* bufs[kBufCount] = {&ctx->x,      &ctx->scratch, &ctx->norms,    &ctx->flag,      &ctx->xb,
                                    &ctx->cand,   &ctx->labels,  &ctx->order,    &ctx->hist,      &ctx->cursor,
                                    &ctx->pivots, &ctx->popc,    &ctx->nnd_work, &ctx->batch_ws,  &ctx->batch_tab,
-                                   &ctx->cert,   &ctx->repair,  &ctx->sym};
+                                   &ctx->cert,   &ctx->repair,  &ctx->sym,      &ctx->prune};
   for (int i = 0; i < kBufCount; i++) cur->b[i] = bufs[i]->bytes;
 }
 
@@ -1895,7 +2167,7 @@ void ctx_release_buffers(evoc_gpu_ctx* ctx) {
   DevBuf* bufs[kBufCount] = {&ctx->x,      &ctx->scratch, &ctx->norms,    &ctx->flag,      &ctx->xb,
                              &ctx->cand,   &ctx->labels,  &ctx->order,    &ctx->hist,      &ctx->cursor,
                              &ctx->pivots, &ctx->popc,    &ctx->nnd_work, &ctx->batch_ws,  &ctx->batch_tab,
-                             &ctx->cert,   &ctx->repair,  &ctx->sym};
+                             &ctx->cert,   &ctx->repair,  &ctx->sym,      &ctx->prune};
   for (DevBuf* b : bufs) b->release();
   for (auto& g : ctx->batch_graphs) cudaGraphExecDestroy(g.exec);  // they name the freed tables
   ctx->batch_graphs.clear();

@@ -97,6 +97,72 @@ cudaError_t launch_tc_scan_sym(const void* X, int64_t rows, int64_t n, int64_t r
                                cudaStream_t stream, int half_type, const float* thr, const float* umin,
                                const int32_t* perm, int32_t* count, uint64_t* mail, int cap,
                                uint64_t delay_ns = 0);
+// Scan of n rows against themselves over tile lists (self rule): X holds the
+// rows in a scanned order, scanned row i being data-set row perm[i].  A query
+// block multiplies the groups of 2^lg tiles its group's list names (`list`,
+// `groups` entries per group, the first len[group] of them; blocks visited as
+// block_order says) and admits only scores reaching seed[row], a dissimilarity
+// no better than the row's keep-th; outputs go to data-set rows.  pc:
+// popcounts in scanned order, pc_rows by data-set row (Jaccard).
+struct ScanLists {
+  const int32_t* perm;
+  const int32_t* list;
+  const int32_t* len;
+  const int32_t* block_order;
+  const float* seed;
+  const int32_t* pc_rows;
+  int groups, lg;
+};
+bool tc_scan_list_feasible(int keep);
+cudaError_t launch_tc_scan_list(int mode, const void* X, int64_t rows, int64_t n, int64_t row_bytes, int keep,
+                                int grid, int final_mode, int dtype, int32_t* out_idx, float* out_raw,
+                                float* out_dist, float* out_bound, int* status, uint64_t timeout_ns,
+                                const int32_t* pc, cudaStream_t stream, int half_type, const ScanLists& lists,
+                                uint64_t delay_ns = 0);
+
+// prune.cu: the lists.  Groups of group_rows rows (a multiple of 256), at most kPruneGroups of them.
+constexpr int kPruneGroups = 4096;
+struct PruneStats {
+  float *a0, *a1, *rho, *sq0;  // per group: smallest / largest a_x, largest |x'|, smallest |x|^2
+  unsigned int* top;                 // largest |x|^2 of all rows (f32 bits)
+};
+// Products of the first `rows` rows of A with all rows of C (a multiple of 256): f32 out[row][ld], or
+// per group the column maxima with 0 (f32 / s32 patterns, out cleared by the caller).
+cudaError_t launch_centre_products(int mode, const void* A, int64_t a_rows_mem, int64_t rows, const void* C,
+                                   int64_t c_rows_mem, int64_t row_bytes, int half_type, bool store,
+                                   int64_t group_rows, void* out, int64_t ld, int* status, uint64_t timeout_ns,
+                                   int sms, cudaStream_t stream);
+// A seed per row (scanned order): a dissimilarity that keep other rows near it do not exceed.  top: the
+// largest |x|^2.
+cudaError_t launch_seeds(int mode, const void* X, int64_t rows_mem, int64_t n, int64_t row_bytes, int keep,
+                         int half_type, const unsigned int* top, const int32_t* pc, float* seed, int* status,
+                         uint64_t timeout_ns, int grid, cudaStream_t stream);
+cudaError_t launch_int8_sq(const void* rows, int64_t row_bytes, int64_t n, int32_t* sq, int sms, cudaStream_t stream);
+// *close += the sampled rows (sample i is row i * stride) whose cosine with their pivot reaches `least`.
+cudaError_t launch_sample_fit(const int32_t* label, const float* raw, int m, int64_t stride, int64_t n, int n_piv,
+                              const int32_t* sq, float least, int32_t* close, cudaStream_t stream);
+// How well the rows fit their pivots: per cell sum and count of the cosines, the rows that stray (listed in
+// any order).  All cleared by the caller.  raw: the pivot scan's dissimilarities; sq: squared norms of the
+// rows (null: unit rows).
+struct CellFit {
+  float* sum;
+  int32_t* count;
+  int32_t* strays;
+};
+cudaError_t launch_cell_fit(const int32_t* label, const float* raw, int64_t n, int n_piv, const int32_t* sq,
+                            const CellFit& f, int32_t* list, int sms, cudaStream_t stream);
+// label[list[i]] = first + second[i].
+cudaError_t launch_stray_labels(const int32_t* list, const int32_t* second, int64_t count, int first, int n_second,
+                                int32_t* label, int sms, cudaStream_t stream);
+// rank[p] = the pivot's place in the order; label[i] = rank[label[i]].
+cudaError_t launch_prim_order(const float* sim, int64_t ld, int n, int32_t* rank, int32_t* label, int64_t n_rows,
+                              int sms, cudaStream_t stream);
+cudaError_t launch_group_stats(int mode, const void* rows, int64_t row_bytes, int64_t n, int64_t group_rows,
+                               int groups, int half_type, void* centres, const PruneStats& st, cudaStream_t stream);
+cudaError_t launch_prune_lists(int mode, int64_t n, int64_t group_rows, int groups, int64_t ld, const int32_t* U,
+                               const float* G, const PruneStats& st, const float* T, int half_len, int32_t* list,
+                               int32_t* len, int32_t* block_order, cudaStream_t stream);
+
 // sym.cu.  Row j of dst = row j * stride of src for j < m, zero rows up to m_pad.
 cudaError_t launch_gather_strided_rows(const void* src, int64_t row_bytes, int64_t stride, int64_t m, int64_t m_pad,
                                        void* dst, int sms, cudaStream_t stream);

@@ -32,6 +32,11 @@
 // mailbox threshold it is staged in shared memory and appended to the row's
 // mailbox in HBM, 64 keys per warp at a time.
 //
+// List mode (prune.cu plans it): all rows are queries and keys, in an order
+// that puts like rows side by side; query block b multiplies only the key
+// tiles of its list, and a seed per row (a bound on its keep-th key) keeps
+// the heaps closed to what cannot stay.
+//
 // Three score modes share the kernel: 16-bit float dot products (cosine; FP16
 // or BF16 operands, the same instruction and rate), int8 dot products, and
 // binary Jaccard, where the packed bits are expanded to 0/1
@@ -115,6 +120,8 @@ struct ScanParams {
   // to whole tiles).  Keys, outputs and mailboxes use data-set rows;
   // sym_thr / sym_umin follow the scanned order.
   const int32_t* sym_perm;
+  // List mode: see ScanLists (kernels.h).
+  ScanLists lists;
   // Batch mode: the work-list of (request, query block) items and the
   // requests' tensor maps and parameters, all in device memory.
   const ScanJob* jobs;
@@ -143,34 +150,40 @@ constexpr int kModeJaccard = 2;  // 0/1 int8 rows: intersection counts, -(inter 
 // -2^30 keeps score - threshold free of overflow.
 constexpr int32_t kIntOpen = -(1 << 30);
 
-template <int MODE, class Keys>
-__device__ __forceinline__ uint32_t pass_threshold(const Keys& heap, int32_t pa) {
-  const uint64_t t = heap.threshold();
+template <int MODE>
+__device__ __forceinline__ uint32_t open_threshold() {
+  return MODE == kModeHalf ? 0xff800000u : uint32_t(kIntOpen);
+}
+
+template <int MODE>
+__device__ __forceinline__ uint32_t raw_threshold(float raw, int32_t pa) {
   if (MODE == kModeInt8) {
-    if (t == kKeyInf) return uint32_t(kIntOpen);
-    const float ts = -from_orderable(uint32_t(t >> 32));  // raw = -score
+    const float ts = -raw;  // raw = -score
     int32_t ti = int32_t(ts);
     if (!(fabsf(ts) < 16777216.0f)) ti -= 256;
     return uint32_t(ti);
   }
   if (MODE == kModeJaccard) {
-    if (t == kKeyInf) return uint32_t(kIntOpen);
-    const float sim = -from_orderable(uint32_t(t >> 32));  // raw = -J (or +0.0 for J = 0)
-    if (!(sim > 0.0f)) return uint32_t(kIntOpen);
+    const float sim = -raw;  // raw = -J (or +0.0 for J = 0)
+    if (!(sim > 0.0f)) return open_threshold<MODE>();
     return uint32_t(int32_t(floorf(sim * float(pa) * (1.0f - 1e-6f))));
   }
-  const uint32_t NEG_INF = 0xff800000u;
-  if (t == kKeyInf) return NEG_INF;
-  const float raw = from_orderable(uint32_t(t >> 32));
-  return raw < 0.0f ? __float_as_uint(-raw) : NEG_INF;  // raw = -score, or MIN_POSITIVE for scores <= 0
+  return raw < 0.0f ? __float_as_uint(-raw) : open_threshold<MODE>();  // raw = -score, or MIN_POSITIVE for scores <= 0
 }
 
-// The threshold with a row's seed (16-bit scores only; -inf: none): a score
-// below the seed provably cannot be among the row's kept keys, so the heap
-// admits only scores reaching both.
+template <int MODE, class Keys>
+__device__ __forceinline__ uint32_t pass_threshold(const Keys& heap, int32_t pa) {
+  const uint64_t t = heap.threshold();
+  return t == kKeyInf ? open_threshold<MODE>() : raw_threshold<MODE>(from_orderable(uint32_t(t >> 32)), pa);
+}
+
+// The threshold with a row's seed (the same pattern; open_threshold: none): a
+// score below the seed provably cannot be among the row's kept keys, so the
+// heap admits only scores reaching both.
 template <int MODE>
-__device__ __forceinline__ uint32_t seeded(uint32_t thr, float seed) {
-  return MODE == kModeHalf ? __float_as_uint(fmaxf(__uint_as_float(thr), seed)) : thr;
+__device__ __forceinline__ uint32_t seeded(uint32_t thr, uint32_t seed) {
+  if (MODE == kModeHalf) return __float_as_uint(fmaxf(__uint_as_float(thr), __uint_as_float(seed)));
+  return uint32_t(max(int32_t(thr), int32_t(seed)));
 }
 
 template <int MODE>
@@ -206,7 +219,7 @@ template <int MODE, class Keys>
 __device__ __forceinline__ void offer_chunk(const uint32_t (&v)[32], uint32_t mask, int64_t col0, int64_t n_k,
                                             bool self_mode, int64_t q, Keys& heap, uint32_t& thr, int32_t pa,
                                             const int32_t* __restrict__ pc, const int32_t* ids = nullptr,
-                                            float seed = -__builtin_huge_valf()) {
+                                            uint32_t seed = open_threshold<MODE>(), float seed_raw = kHeapInf) {
   while (mask) {
     const int j = __clz(mask);
     mask &= ~(0x80000000u >> j);
@@ -221,6 +234,8 @@ __device__ __forceinline__ void offer_chunk(const uint32_t (&v)[32], uint32_t ma
     } else {
       raw = MODE == kModeInt8 ? -__int2float_rn(int32_t(bits)) : raw_cosine(__uint_as_float(bits));
     }
+    // a Jaccard survivor's bound on the intersection is loose: the seed itself decides
+    if (MODE == kModeJaccard && raw > seed_raw) continue;
     heap.offer(make_key(raw, ids ? ids[j] : int32_t(key)));  // ids: the chunk's row indices of the data set
     thr = seeded<MODE>(pass_threshold<MODE>(heap, pa), seed);
   }
@@ -377,6 +392,7 @@ struct ItemView {
   const CUtensorMap* mb;
   int64_t qb, n_q, n_k, q_row0, n_ktiles;
   int64_t kt0;  // first key tile (symmetric mode: the tile holding the block's own rows)
+  const int32_t* list;  // list mode: the block's tile groups
   int n_kchunks, keep, self_mode, final_mode, dtype;
   int32_t* out_idx;
   float* out_raw;
@@ -397,7 +413,7 @@ __device__ __forceinline__ int64_t sym_block(int64_t it, int64_t n_blocks) {
   return it;
 }
 
-template <bool kBatch, bool kSym = false>
+template <bool kBatch, bool kSym = false, bool kList = false>
 __device__ __forceinline__ ItemView item_view(const ScanParams& p, const CUtensorMap* tmA, const CUtensorMap* tmB,
                                               int64_t it) {
   ItemView v;
@@ -426,6 +442,7 @@ __device__ __forceinline__ ItemView item_view(const ScanParams& p, const CUtenso
     v.ma = tmA;
     v.mb = tmB;
     v.qb = kSym ? sym_block(it, (p.n_q + BM - 1) / BM) : it;
+    if (kList) v.qb = p.lists.block_order[sym_block(it, (p.n_q + BM - 1) / BM)];
     v.n_q = p.n_q;
     v.n_k = p.n_k;
     v.q_row0 = p.q_row0;
@@ -444,6 +461,13 @@ __device__ __forceinline__ ItemView item_view(const ScanParams& p, const CUtenso
   }
   v.n_ktiles = (v.n_k + BN - 1) / BN;
   v.kt0 = kSym ? v.qb * BM / BN : 0;
+  v.list = nullptr;
+  if (kList) {
+    // tiles past the data in the last group read as zero rows and are not offered
+    const int64_t g = (v.qb * BM / BN) >> p.lists.lg;
+    v.list = p.lists.list + g * p.lists.groups;
+    v.n_ktiles = int64_t(p.lists.len[g]) << p.lists.lg;
+  }
   return v;
 }
 
@@ -452,8 +476,9 @@ __device__ __forceinline__ ItemView item_view(const ScanParams& p, const CUtenso
 // once), then the rest from the last tile down: the CTAs of a round of items
 // all start at the top and stream the same key tiles nearly in step, as in
 // the plain scan, so each tile is read from HBM once and then from L2.
-template <bool kSym>
-__device__ __forceinline__ int64_t tile_at(const ItemView& v, int64_t ti) {
+template <bool kSym, bool kList>
+__device__ __forceinline__ int64_t tile_at(const ItemView& v, int64_t ti, int lg) {
+  if (kList) return (int64_t(v.list[ti >> lg]) << lg) + (ti & ((int64_t(1) << lg) - 1));
   return (kSym && ti > 0) ? v.n_ktiles - ti : v.kt0 + ti;
 }
 
@@ -487,12 +512,14 @@ __device__ __forceinline__ bool epilogue_vote(int nthreads, bool ok) {
 
 }  // namespace
 
-template <int MODE, int STAGES, int GROUPS, bool kSmemHeap, bool kBatch, bool kPair = false, bool kSym = false>
+template <int MODE, int STAGES, int GROUPS, bool kSmemHeap, bool kBatch, bool kPair = false, bool kSym = false,
+          bool kList = false>
 __global__ void __launch_bounds__(64 + GROUPS * 128, 1)
 tc_scan_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const ScanParams p) {
   using namespace sm100;
   static_assert(!(kPair && kBatch), "CTA pairs run single requests");
   static_assert(!kSym || (MODE == kModeHalf && !kBatch && !kPair), "symmetric mode: 16-bit single requests");
+  static_assert(!kList || (!kSym && !kBatch && !kPair), "list mode: single requests");
   constexpr int SB = kPair ? PAIR_STAGE_BYTES : STAGE_BYTES;  // bytes of one stage in this CTA
   extern __shared__ uint8_t smem_dyn[];
   const uint32_t pad = (1024u - (smem_addr(smem_dyn) & 1023u)) & 1023u;
@@ -564,13 +591,16 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       uint32_t it = 0;
       bool ok = true;
       for (int64_t itm = item0; ok && itm < n_items; itm += item_step) {
-        const ItemView v = item_view<kBatch, kSym>(p, &tmA, &tmB, kPair ? 2 * itm + rank : itm);
+        const ItemView v = item_view<kBatch, kSym, kList>(p, &tmA, &tmB, kPair ? 2 * itm + rank : itm);
         if (kBatch) {
           tensormap_acquire(v.ma);
           tensormap_acquire(v.mb);
         }
+        int64_t next = tile_at<kSym, kList>(v, 0, p.lists.lg);
         for (int64_t ti = 0; ok && ti < v.n_ktiles - v.kt0; ti++) {
-          const int64_t kt = tile_at<kSym>(v, ti);
+          const int64_t kt = next;
+          // the next list entry is on its way while this tile's loads are issued
+          if (ti + 1 < v.n_ktiles - v.kt0) next = tile_at<kSym, kList>(v, ti + 1, p.lists.lg);
           for (int kc = 0; kc < v.n_kchunks; kc++) {
             const uint32_t s = it % STAGES, ph = (it / STAGES) & 1u;
             if (!mbar_wait(&empty[s], ph ^ 1u, abort, p.timeout_ns)) {
@@ -609,7 +639,7 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       uint32_t it = 0, tile = 0;
       bool ok = true;
       for (int64_t itm = item0; ok && itm < n_items; itm += item_step) {
-        const ItemView v = item_view<kBatch, kSym>(p, &tmA, &tmB, kPair ? 2 * itm : itm);
+        const ItemView v = item_view<kBatch, kSym, kList>(p, &tmA, &tmB, kPair ? 2 * itm : itm);
         for (int64_t ti = 0; ok && ti < v.n_ktiles - v.kt0; ti++, tile++) {
           const uint32_t a = tile & 1u, tph = (tile >> 1) & 1u;
           if (!mbar_wait(&tempty[a], tph ^ 1u, abort, p.timeout_ns)) {
@@ -694,13 +724,14 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     uint32_t tile = 0;
     bool ok = true;
     for (int64_t itm = item0; ok && itm < n_items; itm += item_step) {
-      const ItemView v = item_view<kBatch, kSym>(p, &tmA, &tmB, kPair ? 2 * itm + rank : itm);
+      const ItemView v = item_view<kBatch, kSym, kList>(p, &tmA, &tmB, kPair ? 2 * itm + rank : itm);
       const int64_t q = v.qb * BM + row_local;  // output row
       const bool valid = q < v.n_q;
       // row of the data set (its key index for the self rule)
       const int64_t qg = v.q_self ? (valid ? v.q_self_base + v.q_self[q] : -1) : v.q_row0 + q;
       // symmetric mode: qg is the scanned row, qd its row of the data set (keys and outputs)
-      const int32_t qd = kSym ? (valid ? p.sym_perm[q] : -1) : int32_t(qg);
+      const int32_t* const perm = kList ? p.lists.perm : p.sym_perm;
+      const int32_t qd = kSym || kList ? (valid ? perm[q] : -1) : int32_t(qg);
       // four groups: a binary heap, the other's registers would not fit
       std::conditional_t<GROUPS == 4, KeyHeap, KeySet> heap;
       heap.init(hstore, v.keep);
@@ -708,10 +739,14 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       const int32_t pa = (MODE == kModeJaccard && valid) ? v.pc[qg] : 0;
       // symmetric mode: the row's mailbox threshold also bounds its own side (a score
       // below it cannot be among the row's C best over all keys)
-      const float seed = kSym && valid ? p.sym_thr[q] : -__builtin_huge_valf();
-      uint32_t thr = seeded<MODE>(pass_threshold<MODE>(heap, pa), seed);
+      const uint32_t seed = kSym && valid ? __float_as_uint(p.sym_thr[q]) : open_threshold<MODE>();
+      const float seed_raw = kList && valid ? p.lists.seed[q] : kHeapInf;
+      const uint32_t row_seed = kList && seed_raw < kHeapInf ? raw_threshold<MODE>(seed_raw, pa) : seed;
+      uint32_t thr = seeded<MODE>(pass_threshold<MODE>(heap, pa), row_seed);
+      int64_t next = tile_at<kSym, kList>(v, 0, p.lists.lg);
       for (int64_t ti = 0; ti < v.n_ktiles - v.kt0; ti++, tile++) {
-        const int64_t kt = tile_at<kSym>(v, ti);
+        const int64_t kt = next;
+        if (ti + 1 < v.n_ktiles - v.kt0) next = tile_at<kSym, kList>(v, ti + 1, p.lists.lg);
         const uint32_t a = tile & 1u, tph = (tile >> 1) & 1u;
         int got = 1;
         if (lane == 0) got = mbar_wait(&tfull[a], tph, abort, p.timeout_ns) ? 1 : 0;
@@ -729,7 +764,7 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           // this tile's copy was issued with the tile before (the first of an item: now); the next tile's goes now
           if (ti == 0) fetch_thr(kt, 0);
           cp_async_commit();
-          if (ti + 1 < v.n_ktiles - v.kt0) fetch_thr(tile_at<kSym>(v, ti + 1), (ti + 1) & 1);
+          if (ti + 1 < v.n_ktiles - v.kt0) fetch_thr(next, (ti + 1) & 1);
           cp_async_commit();
           cp_async_wait<1>();
           __syncwarp();
@@ -746,11 +781,12 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             const int32_t* ids = reinterpret_cast<const int32_t*>(tth + kTileIds) + col_base + c * 32;
             if (valid && (int32_t(thr) > 0 ? mx >= int32_t(thr) : chunk_any<MODE>(vv, thr)))
               offer_chunk<MODE>(vv, chunk_mask<MODE>(vv, thr), col, v.n_k, v.self_mode, qg, heap, thr, pa, v.pc,
-                                ids, seed);
+                                ids, row_seed);
             if (col >= (v.qb + 1) * BM)
               mirror_chunk(vv, mx, um, tth + (col_base + c * 32), ids, col, v.n_k, qd, valid, mst, lane, p);
           } else if (valid && chunk_any<MODE>(vv, thr)) {
-            offer_chunk<MODE>(vv, chunk_mask<MODE>(vv, thr), col, v.n_k, v.self_mode, qg, heap, thr, pa, v.pc);
+            offer_chunk<MODE>(vv, chunk_mask<MODE>(vv, thr), col, v.n_k, v.self_mode, qg, heap, thr, pa, v.pc,
+                              kList ? perm + col : nullptr, row_seed, seed_raw);
           }
         };
         // One group: a chunk is processed while the next is read.  Several
@@ -807,7 +843,8 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         // mailbox merge's input, is sorted (60 keys took ~45k cycles a block).
         const uint64_t worst = heap.threshold();
         const int got = v.final_mode || kSym ? heap.finish() : heap.size;
-        const int64_t orow = (kSym ? int64_t(qd) : q) * v.keep;  // symmetric mode: rows of the data set
+        // symmetric and list mode: rows of the data set
+        const int64_t orow = (kSym || kList ? int64_t(qd) : q) * v.keep;
         for (int j = 0; j < v.keep; j++) {
           float raw = kHeapInf;
           int32_t idx = -1;
@@ -817,13 +854,16 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             // Keys fold -0.0 onto +0.0; restore the reference's sign: an int8
             // zero dot is -0.0; a Jaccard zero is +0.0 only for two empty rows.
             if (MODE == kModeInt8) raw = int8_raw_from_key(raw);
-            if (MODE == kModeJaccard && raw == 0.0f) raw = (pa + v.pc[idx] == 0) ? 0.0f : -0.0f;
+            if (MODE == kModeJaccard && raw == 0.0f)
+              raw = (pa + (kList ? p.lists.pc_rows : v.pc)[idx] == 0) ? 0.0f : -0.0f;
           }
           v.out_idx[orow + j] = idx;
           if (v.out_raw) v.out_raw[orow + j] = raw;
           if (v.final_mode && v.out_dist) v.out_dist[orow + j] = transform_raw(v.dtype, raw);
         }
-        if (v.out_bound) v.out_bound[q] = got == v.keep ? from_orderable(uint32_t(worst >> 32)) : kHeapInf;
+        if (v.out_bound)
+          v.out_bound[kList ? int64_t(qd) : q] =
+              got == v.keep ? from_orderable(uint32_t(worst >> 32)) : kHeapInf;
       }
       if (GROUPS > 1) epilogue_sync(GROUPS * 128);  // heaps are reused by the next block
     }
@@ -862,9 +902,11 @@ PFN_cuTensorMapEncodeTiled_v12000 get_encode() {
   return fn;
 }
 
+}  // namespace
+
 // 2-D map over `rows` rows of `row_bytes` (a multiple of 128); box = 128 bytes x box_rows.
-bool make_map(CUtensorMap* m, const void* base, int64_t rows, int64_t row_bytes, int elem_bytes, int box_rows,
-              int half_type = kHalfF16) {
+bool encode_row_map(CUtensorMap* m, const void* base, int64_t rows, int64_t row_bytes, int elem_bytes, int box_rows,
+                    int half_type) {
   auto enc = get_encode();
   if (!enc) return false;
   const cuuint64_t dims[2] = {cuuint64_t(row_bytes / elem_bytes), cuuint64_t(rows)};
@@ -879,8 +921,6 @@ bool make_map(CUtensorMap* m, const void* base, int64_t rows, int64_t row_bytes,
                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
 }
-
-}  // namespace
 
 size_t tc_scan_smem_bytes() { return smem_bytes(4, 1, 0); }
 
@@ -1038,8 +1078,8 @@ cudaError_t launch_tc_scan(int mode, const void* Q, int64_t q_rows, int64_t q_ro
   // variant launch_mode takes, a forced one when it is feasible).
   const bool pair = variant >= 0 && variant_feasible(variant, keep, scratch != nullptr) && kVariantCfg[variant][3];
   alignas(64) CUtensorMap ma, mb;
-  if (!make_map(&ma, Q, q_rows, row_bytes, eb, BM, half_type) ||
-      !make_map(&mb, K, k_rows, row_bytes, eb, pair ? BM : BN, half_type))
+  if (!encode_row_map(&ma, Q, q_rows, row_bytes, eb, BM, half_type) ||
+      !encode_row_map(&mb, K, k_rows, row_bytes, eb, pair ? BM : BN, half_type))
     return cudaErrorInvalidValue;
   ScanParams p{};
   p.n_q = n_q;
@@ -1100,7 +1140,7 @@ cudaError_t launch_tc_scan_sym(const void* X, int64_t rows, int64_t n, int64_t r
   if (!tc_scan_sym_feasible(keep)) return cudaErrorInvalidValue;
   // the same rows as queries (128-row boxes) and keys (256-row boxes)
   alignas(64) CUtensorMap ma, mb;
-  if (!make_map(&ma, X, rows, row_bytes, 2, BM, half_type) || !make_map(&mb, X, rows, row_bytes, 2, BN, half_type))
+  if (!encode_row_map(&ma, X, rows, row_bytes, 2, BM, half_type) || !encode_row_map(&mb, X, rows, row_bytes, 2, BN, half_type))
     return cudaErrorInvalidValue;
   ScanParams p{};
   p.n_q = n;
@@ -1128,6 +1168,78 @@ cudaError_t launch_tc_scan_sym(const void* X, int64_t rows, int64_t n, int64_t r
   if (sym_smem_bytes(4, 1, odd) <= SMEM_LIMIT) return launch_sym_variant<4, 1>(ma, mb, p, grid, stream);
   if (sym_smem_bytes(3, 1, odd) <= SMEM_LIMIT) return launch_sym_variant<3, 1>(ma, mb, p, grid, stream);
   return launch_sym_variant<2, 1>(ma, mb, p, grid, stream);
+}
+
+namespace {
+template <int MODE, int STAGES, int GROUPS>
+cudaError_t launch_list_variant(const CUtensorMap& ma, const CUtensorMap& mb, const ScanParams& p, int grid,
+                                cudaStream_t stream) {
+  auto kern = tc_scan_kernel<MODE, STAGES, GROUPS, true, false, false, false, true>;
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SMEM_LIMIT));
+  if (e != cudaSuccess) return e;
+  kern<<<grid, 64 + GROUPS * 128, smem_bytes(STAGES, GROUPS, p.heap_stride), stream>>>(ma, mb, p);
+  return cudaGetLastError();
+}
+
+// The first variant of the automatic order whose heaps fit shared memory
+// (without the four-group one: its list form would spill registers that TMEM
+// loads are still writing).
+template <int MODE>
+cudaError_t launch_list_mode(const CUtensorMap& ma, const CUtensorMap& mb, const ScanParams& p, int grid,
+                             cudaStream_t stream) {
+  switch (tc_scan_automatic_variant(kModeHalf, p.keep)) {
+    case 0: return launch_list_variant<MODE, 4, 2>(ma, mb, p, grid, stream);
+    case 1: return launch_list_variant<MODE, 3, 2>(ma, mb, p, grid, stream);
+    case 2: return launch_list_variant<MODE, 4, 1>(ma, mb, p, grid, stream);
+    case 3: return launch_list_variant<MODE, 3, 1>(ma, mb, p, grid, stream);
+    case 14: return launch_list_variant<MODE, 2, 1>(ma, mb, p, grid, stream);
+    default: return cudaErrorInvalidValue;
+  }
+}
+}  // namespace
+
+bool tc_scan_list_feasible(int keep) { return tc_scan_automatic_variant(kModeHalf, keep) != 4; }
+
+cudaError_t launch_tc_scan_list(int mode, const void* X, int64_t rows, int64_t n, int64_t row_bytes, int keep,
+                                int grid, int final_mode, int dtype, int32_t* out_idx, float* out_raw,
+                                float* out_dist, float* out_bound, int* status, uint64_t timeout_ns,
+                                const int32_t* pc, cudaStream_t stream, int half_type, const ScanLists& lists,
+                                uint64_t delay_ns) {
+  if (row_bytes % KCB != 0 || n <= 0 || keep < 1 || rows < n || rows % BN != 0) return cudaErrorInvalidValue;
+  if ((reinterpret_cast<uintptr_t>(X) & 15) || !lists.perm || !lists.list || !lists.len || !lists.block_order ||
+      !lists.seed || !out_idx)
+    return cudaErrorInvalidValue;
+  if (mode < kModeHalf || mode > kModeJaccard || (mode == kModeJaccard && (!pc || !lists.pc_rows)))
+    return cudaErrorInvalidValue;
+  if (half_type != kHalfF16 && half_type != kHalfBf16) return cudaErrorInvalidValue;
+  const int eb = mode == kModeHalf ? 2 : 1;
+  alignas(64) CUtensorMap ma, mb;
+  if (!encode_row_map(&ma, X, rows, row_bytes, eb, BM, half_type) ||
+      !encode_row_map(&mb, X, rows, row_bytes, eb, BN, half_type))
+    return cudaErrorInvalidValue;
+  ScanParams p{};
+  p.n_q = n;
+  p.n_k = n;
+  p.n_kchunks = int(row_bytes / KCB);
+  p.keep = keep;
+  p.heap_stride = keep | 1;
+  p.self_mode = 1;
+  p.final_mode = final_mode;
+  p.dtype = dtype;
+  p.out_idx = out_idx;
+  p.out_raw = out_raw;
+  p.out_dist = out_dist;
+  p.out_bound = out_bound;
+  p.status = status;
+  p.timeout_ns = timeout_ns;
+  p.drain_ns = timeout_ns > kDrainNs ? timeout_ns : kDrainNs;
+  p.delay_ns = delay_ns;
+  p.pc = pc;
+  p.half_type = half_type;
+  p.lists = lists;
+  if (mode == kModeInt8) return launch_list_mode<kModeInt8>(ma, mb, p, grid, stream);
+  if (mode == kModeJaccard) return launch_list_mode<kModeJaccard>(ma, mb, p, grid, stream);
+  return launch_list_mode<kModeHalf>(ma, mb, p, grid, stream);
 }
 
 bool tc_scan_variant_feasible(int variant, int keep, bool has_scratch) {
@@ -1179,8 +1291,8 @@ bool encode_scan_job(ScanJob* sj, int mode, const void* rows, int64_t rows_mem, 
   if (row_bytes % KCB != 0 || n <= 0 || keep < 1 || rows_mem < n || rows_mem % BN != 0) return false;
   if (reinterpret_cast<uintptr_t>(rows) & 15) return false;
   const int eb = mode == kModeHalf ? 2 : 1;
-  if (!make_map(&sj->ma, rows, rows_mem, row_bytes, eb, BM, half_type) ||
-      !make_map(&sj->mb, rows, rows_mem, row_bytes, eb, BN, half_type))
+  if (!encode_row_map(&sj->ma, rows, rows_mem, row_bytes, eb, BM, half_type) ||
+      !encode_row_map(&sj->mb, rows, rows_mem, row_bytes, eb, BN, half_type))
     return false;
   sj->n_q = n;
   sj->n_k = n;
