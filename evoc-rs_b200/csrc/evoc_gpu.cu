@@ -216,9 +216,10 @@ int prune_lg(int64_t n) {
 }
 
 struct PruneLayout {
-  size_t rows, centres, u, g, list, len, blocks, stats, seed, sq, rank, cells, second, total;
+  size_t rows, centres, u, g, list, len, blocks, stats, seed, sq, rank, attach, cells, second, raw2, cuts, start,
+      first, group_of, total;
   int lg;
-  int64_t groups, ld, group_rows;
+  int64_t groups, segments, ld, group_rows;  // segments: at most
 };
 
 // row_bytes: of the operand rows; xs_bytes: of the rows copied into scanned
@@ -229,7 +230,8 @@ PruneLayout prune_layout(int64_t n, int64_t row_bytes, int64_t xs_bytes) {
   L.lg = prune_lg(n);
   L.group_rows = int64_t(256) << L.lg;
   L.groups = (n + L.group_rows - 1) / L.group_rows;
-  L.ld = round_up(std::max(L.groups, piv), 256);
+  L.segments = std::min<int64_t>(L.groups + piv, evoc::kPruneSegments);
+  L.ld = round_up(std::max(L.segments, piv), 256);
   size_t off = 0;
   auto take = [&](size_t bytes) {
     const size_t at = off;
@@ -237,18 +239,24 @@ PruneLayout prune_layout(int64_t n, int64_t row_bytes, int64_t xs_bytes) {
     return at;
   };
   L.rows = take(size_t(evoc::padded_rows(n) * xs_bytes));
-  L.centres = take(size_t(round_up(L.groups, 256) * row_bytes));
-  L.u = take(size_t(L.groups * L.ld) * 4);
-  L.g = take(size_t(std::max(L.groups, piv) * L.ld) * 4);  // the pivots' similarities first
+  L.centres = take(size_t(round_up(L.segments, 256) * row_bytes));
+  L.u = take(size_t(L.segments * L.ld) * 4);
+  L.g = take(size_t(std::max(L.segments, piv) * L.ld) * 4);  // the pivots' similarities first
   L.list = take(size_t(L.groups * L.groups) * 4);
   L.len = take(size_t(L.groups) * 4);
   L.blocks = take(size_t((n + 127) / 128) * 4);
-  L.stats = take(size_t(4 * L.groups) * 4 + 256);
+  L.stats = take(size_t(4 * L.segments) * 4 + 256);
   L.seed = take(size_t(n) * 4);    // the pivot scan's dissimilarities first
   L.sq = take(size_t(n) * 4);      // int8: squared norms; binary: popcounts in scanned order
   L.rank = take(size_t(piv) * 4);
-  L.cells = take(size_t(2 * piv) * 4 + 256);
-  L.second = take(size_t(n) * 4);  // the strays' second labels
+  L.attach = take(size_t(piv) * 4);
+  L.cells = take(size_t(6 * piv) * 4 + 256);
+  L.second = take(size_t(n) * 4);  // the strays' second labels, and their dissimilarities
+  L.raw2 = take(size_t(n) * 4);
+  L.cuts = take(size_t(piv) * 4);
+  L.start = take(size_t(L.segments + 1) * 4);
+  L.first = take(size_t(L.groups + 1) * 4);
+  L.group_of = take(size_t(L.segments + 1) * 4);
   L.total = off;
   return L;
 }
@@ -291,6 +299,8 @@ int list_scan(evoc_gpu_ctx* ctx, const Job& j, int mode, const void* rows, int64
   const int gemm = mode == evoc::kScanHalf ? evoc::kScanHalf : evoc::kScanInt8;
   const int64_t piv1 = list_pivots(n);
   int64_t piv2 = 0;
+  int32_t segments = 0;
+  const evoc::Segments seg{i32(L.start), i32(L.first), L.group_rows};
   {
     Stage st(ctx, "scan_order");
     const bool int8 = gemm == evoc::kScanInt8;
@@ -304,7 +314,13 @@ int list_scan(evoc_gpu_ctx* ctx, const Job& j, int mode, const void* rows, int64
     } else if (binary) {
       sq = ctx->popc.as<int32_t>();
     }
-    EVOC_TRY(cudaMemsetAsync(b + L.cells, 0, size_t(2 * piv1 + 2) * 4, ctx->stream), "clear cells");
+    // counters, then the first pivots' cells (all rows, the closer ones), then every pivot's rows
+    // without the strays
+    const int64_t piv_max = piv1 + kStrayPivots;
+    int32_t* counters = i32(L.cells);  // close sample rows, strays, segments
+    float *sum = f(L.cells) + 4, *top_sum = sum + 2 * piv1, *own_sum = sum + 4 * piv1;
+    int32_t *cnt = i32(L.cells) + 4 + piv1, *top_cnt = cnt + 2 * piv1, *own_cnt = cnt + 3 * piv1 + piv_max;
+    EVOC_TRY(cudaMemsetAsync(b + L.cells, 0, size_t(4 + 4 * piv1 + 2 * piv_max) * 4, ctx->stream), "clear cells");
     EVOC_TRY(ctx->labels.ensure(size_t(n) * 4), "alloc labels");
     int32_t* label = ctx->labels.as<int32_t>();
     // the sample's rows pass through the place of the scanned rows
@@ -316,10 +332,10 @@ int list_scan(evoc_gpu_ctx* ctx, const Job& j, int mode, const void* rows, int64
                         f(L.seed), j.status);
     if (rc) return rc;
     EVOC_TRY(evoc::launch_sample_fit(label, f(L.seed), int(kFitSample), stride, n, int(piv1), sq,
-                                     binary ? kFitCosineBits : kFitCosine, i32(L.cells), ctx->stream),
+                                     binary ? kFitCosineBits : kFitCosine, counters, ctx->stream),
              "sample fit");
     ctx->launches += 2;
-    const int32_t close = read_count(ctx, i32(L.cells), &rc);
+    const int32_t close = read_count(ctx, counters, &rc);
     if (rc || close < kFitSample / 4) return rc;
     *taken = true;
     rc = nearest_pivots(ctx, rows, rows_mem, 0, n, row_bytes, int8, half, ctx->pivots.p, piv1, label, f(L.seed),
@@ -327,10 +343,17 @@ int list_scan(evoc_gpu_ctx* ctx, const Job& j, int mode, const void* rows, int64
     if (rc) return rc;
     EVOC_TRY(ctx->order.ensure(size_t(n) * 4), "alloc order");
     int32_t* strays = ctx->order.as<int32_t>();  // until the order is known
-    const evoc::CellFit fit{f(L.cells) + 2, i32(L.cells) + 2 + piv1, i32(L.cells) + 1};
-    EVOC_TRY(evoc::launch_cell_fit(label, f(L.seed), n, int(piv1), sq, fit, strays, ctx->sms, ctx->stream), "cell fit");
-    ctx->launches += 2;
-    const int32_t n_strays = read_count(ctx, i32(L.cells) + 1, &rc);
+    EVOC_TRY(evoc::launch_cell_fit(label, f(L.seed), n, int(piv1), sq, nullptr, nullptr, nullptr, sum, cnt, ctx->sms,
+                                   ctx->stream),
+             "cell fit");
+    EVOC_TRY(evoc::launch_cell_fit(label, f(L.seed), n, int(piv1), sq, nullptr, sum, cnt, top_sum, top_cnt, ctx->sms,
+                                   ctx->stream),
+             "cell fit");
+    EVOC_TRY(evoc::launch_strays(label, f(L.seed), n, int(piv1), sq, top_sum, top_cnt, own_sum, own_cnt, strays,
+                                 counters + 1, ctx->sms, ctx->stream),
+             "strays");
+    ctx->launches += 3;
+    const int32_t n_strays = read_count(ctx, counters + 1, &rc);
     if (rc) return rc;
     // their operand rows are gathered in the arena's place for the scanned rows (binary data: packed
     // rows' place, which holds an eighth of the 0/1 rows; strays past that keep their first cell)
@@ -345,12 +368,16 @@ int list_scan(evoc_gpu_ctx* ctx, const Job& j, int mode, const void* rows, int64
                "stray rows");
       EVOC_TRY(cudaMemsetAsync(p2, 0, size_t(evoc::padded_rows(piv2) * row_bytes), ctx->stream), "clear pivots");
       EVOC_TRY(evoc::launch_gather_pivots(q, row_bytes, count, piv2, p2, ctx->sms, ctx->stream), "gather pivots");
-      rc = nearest_pivots(ctx, q, crows, 0, count, row_bytes, int8, half, p2, piv2, i32(L.second), nullptr, j.status);
+      rc = nearest_pivots(ctx, q, crows, 0, count, row_bytes, int8, half, p2, piv2, i32(L.second), f(L.raw2),
+                          j.status);
       if (rc) return rc;
+      EVOC_TRY(evoc::launch_cell_fit(i32(L.second), f(L.raw2), count, int(piv2), sq, strays, nullptr, nullptr,
+                                     own_sum + piv1, own_cnt + piv1, ctx->sms, ctx->stream),
+               "stray fit");
       EVOC_TRY(evoc::launch_stray_labels(strays, i32(L.second), count, int(piv1), int(piv2), label, ctx->sms,
                                          ctx->stream),
                "stray labels");
-      ctx->launches += 3;
+      ctx->launches += 4;
     }
     const int64_t piv = piv1 + piv2, piv_mem = evoc::padded_rows(piv);
     if (piv2 > 0 || piv_mem > evoc::padded_rows(piv1)) {
@@ -361,16 +388,21 @@ int list_scan(evoc_gpu_ctx* ctx, const Job& j, int mode, const void* rows, int64
                  "clear pivots");
     }
     EVOC_TRY(evoc::launch_centre_products(gemm, ctx->pivots.p, piv_mem, piv, ctx->pivots.p, piv_mem, row_bytes, half,
-                                          true, 256, f(L.g), L.ld, j.status, ctx->timeout_ns, ctx->sms, ctx->stream),
+                                          nullptr, f(L.g), L.ld, j.status, ctx->timeout_ns, ctx->sms, ctx->stream),
              "pivot similarities");
-    EVOC_TRY(evoc::launch_prim_order(f(L.g), L.ld, int(piv), i32(L.rank), label, n, ctx->sms, ctx->stream),
+    EVOC_TRY(evoc::launch_prim_order(f(L.g), L.ld, int(piv), i32(L.rank), f(L.attach), label, n, ctx->sms,
+                                     ctx->stream),
              "pivot order");
     rc = order_by_pivot(ctx, j, piv, false);
     if (rc) return rc;
+    EVOC_TRY(evoc::launch_segments(i32(L.rank), f(L.attach), own_sum, own_cnt, int(piv), ctx->cursor.as<int32_t>(),
+                                   ctx->hist.as<int32_t>(), n, L.group_rows, int(L.groups), int(L.segments),
+                                   i32(L.cuts), seg, counters + 2, i32(L.group_of), ctx->stream),
+             "segments");
     EVOC_TRY(evoc::launch_gather_rows_list(binary ? packed : rows, binary ? ldp : row_bytes, 0,
                                            ctx->order.as<int32_t>(), n, rows_mem, b + L.rows, ctx->sms, ctx->stream),
              "rows in scanned order");
-    ctx->launches += 4;
+    ctx->launches += 5;
     if (binary) {
       EVOC_TRY(evoc::launch_popcount_rows(b + L.rows, n, int(ldp / 4), i32(L.sq), ctx->sms, ctx->stream), "popcounts");
       EVOC_TRY(evoc::launch_expand_bits(b + L.rows, n, ldp, nbytes, ctx->xb.p, rows_mem, row_bytes, ctx->sms,
@@ -378,32 +410,34 @@ int list_scan(evoc_gpu_ctx* ctx, const Job& j, int mode, const void* rows, int64
                "expand bits");
       ctx->launches += 2;
     }
+    segments = read_count(ctx, counters + 2, &rc);
+    if (rc) return rc;
+    if (segments < L.groups || segments > L.segments)
+      return fail(ctx, EVOC_ERR_CUDA, "device self-check failed (segments)");
   }
   const void* xs = binary ? ctx->xb.p : b + L.rows;
   const int32_t* pc = binary ? i32(L.sq) : nullptr;
-  const evoc::PruneStats ps{f(L.stats), f(L.stats) + L.groups, f(L.stats) + 2 * L.groups, f(L.stats) + 3 * L.groups,
-                            reinterpret_cast<unsigned int*>(f(L.stats) + 4 * L.groups)};
+  const evoc::PruneStats ps{f(L.stats), f(L.stats) + L.segments, f(L.stats) + 2 * L.segments,
+                            f(L.stats) + 3 * L.segments, reinterpret_cast<unsigned int*>(f(L.stats) + 4 * L.segments)};
   {
     Stage st(ctx, "tile_lists");
-    const int64_t crows = round_up(L.groups, 256);
+    const int64_t crows = round_up(segments, 256);
     EVOC_TRY(cudaMemsetAsync(b + L.centres, 0, size_t(crows * row_bytes), ctx->stream), "clear centres");
-    EVOC_TRY(evoc::launch_group_stats(gemm, xs, row_bytes, n, L.group_rows, int(L.groups), half, b + L.centres, ps,
-                                      ctx->stream),
-             "group statistics");
-    EVOC_TRY(cudaMemsetAsync(b + L.u, 0, size_t(L.groups * L.ld) * 4, ctx->stream), "clear maxima");
-    EVOC_TRY(evoc::launch_centre_products(gemm, xs, rows_mem, n, b + L.centres, crows, row_bytes, half, false,
-                                          L.group_rows, i32(L.u), L.ld, j.status, ctx->timeout_ns, ctx->sms,
-                                          ctx->stream),
-             "group maxima");
-    EVOC_TRY(evoc::launch_centre_products(gemm, b + L.centres, crows, L.groups, b + L.centres, crows, row_bytes, half,
-                                          true, L.group_rows, f(L.g), L.ld, j.status, ctx->timeout_ns, ctx->sms,
-                                          ctx->stream),
+    EVOC_TRY(evoc::launch_segment_stats(gemm, xs, row_bytes, seg, segments, half, b + L.centres, ps, ctx->stream),
+             "segment statistics");
+    EVOC_TRY(cudaMemsetAsync(b + L.u, 0, size_t(segments * L.ld) * 4, ctx->stream), "clear maxima");
+    EVOC_TRY(evoc::launch_centre_products(gemm, xs, rows_mem, n, b + L.centres, crows, row_bytes, half, &seg,
+                                          i32(L.u), L.ld, j.status, ctx->timeout_ns, ctx->sms, ctx->stream),
+             "segment maxima");
+    EVOC_TRY(evoc::launch_centre_products(gemm, b + L.centres, crows, segments, b + L.centres, crows, row_bytes, half,
+                                          nullptr, f(L.g), L.ld, j.status, ctx->timeout_ns, ctx->sms, ctx->stream),
              "centre products");
     EVOC_TRY(evoc::launch_seeds(mode, xs, rows_mem, n, row_bytes, keep, half, ps.top, pc, f(L.seed), j.status,
                                 ctx->timeout_ns, scan_grid(ctx, n), ctx->stream),
              "seeds");
-    EVOC_TRY(evoc::launch_prune_lists(mode, n, L.group_rows, int(L.groups), L.ld, i32(L.u), f(L.g), ps, f(L.seed),
-                                      int(row_bytes / 2), i32(L.list), i32(L.len), i32(L.blocks), ctx->stream),
+    EVOC_TRY(evoc::launch_prune_lists(mode, n, L.group_rows, int(L.groups), seg, i32(L.group_of), segments, L.ld,
+                                      i32(L.u), f(L.g), ps, f(L.seed), int(row_bytes / 2), i32(L.list), i32(L.len),
+                                      i32(L.blocks), ctx->stream),
              "tile lists");
     ctx->launches += 6;
   }

@@ -120,18 +120,25 @@ cudaError_t launch_tc_scan_list(int mode, const void* X, int64_t rows, int64_t n
                                 const int32_t* pc, cudaStream_t stream, int half_type, const ScanLists& lists,
                                 uint64_t delay_ns = 0);
 
-// prune.cu: the lists.  Groups of group_rows rows (a multiple of 256), at most kPruneGroups of them.
+// prune.cu: the lists.  Groups of group_rows rows (a multiple of 256), at most kPruneGroups of them, cut
+// into segments of like rows, at most kPruneSegments.
 constexpr int kPruneGroups = 4096;
-struct PruneStats {
-  float *a0, *a1, *rho, *sq0;  // per group: smallest / largest a_x, largest |x'|, smallest |x|^2
-  unsigned int* top;                 // largest |x|^2 of all rows (f32 bits)
+constexpr int kPruneSegments = 6144;
+struct Segments {
+  int32_t* start;  // first row of each segment, and n
+  int32_t* first;  // first segment of each group, and their number
+  int64_t group_rows;
 };
-// Products of the first `rows` rows of A with all rows of C (a multiple of 256): f32 out[row][ld], or
-// per group the column maxima with 0 (f32 / s32 patterns, out cleared by the caller).
+struct PruneStats {
+  float *a0, *a1, *rho, *sq0;  // per segment: smallest / largest a_x, largest |x'|, smallest |x|^2
+  unsigned int* top;           // largest |x|^2 of all rows (f32 bits)
+};
+// Products of the first `rows` rows of A with all rows of C (a multiple of 256): f32 out[row][ld]; with
+// seg, per segment of A's rows the column maxima with 0 (f32 / s32 patterns, out cleared by the caller).
 cudaError_t launch_centre_products(int mode, const void* A, int64_t a_rows_mem, int64_t rows, const void* C,
-                                   int64_t c_rows_mem, int64_t row_bytes, int half_type, bool store,
-                                   int64_t group_rows, void* out, int64_t ld, int* status, uint64_t timeout_ns,
-                                   int sms, cudaStream_t stream);
+                                   int64_t c_rows_mem, int64_t row_bytes, int half_type, const Segments* seg,
+                                   void* out, int64_t ld, int* status, uint64_t timeout_ns, int sms,
+                                   cudaStream_t stream);
 // A seed per row (scanned order): a dissimilarity that keep other rows near it do not exceed.  top: the
 // largest |x|^2.
 cudaError_t launch_seeds(int mode, const void* X, int64_t rows_mem, int64_t n, int64_t row_bytes, int keep,
@@ -141,27 +148,35 @@ cudaError_t launch_int8_sq(const void* rows, int64_t row_bytes, int64_t n, int32
 // *close += the sampled rows (sample i is row i * stride) whose cosine with their pivot reaches `least`.
 cudaError_t launch_sample_fit(const int32_t* label, const float* raw, int m, int64_t stride, int64_t n, int n_piv,
                               const int32_t* sq, float least, int32_t* close, cudaStream_t stream);
-// How well the rows fit their pivots: per cell sum and count of the cosines, the rows that stray (listed in
-// any order).  All cleared by the caller.  raw: the pivot scan's dissimilarities; sq: squared norms of the
-// rows (null: unit rows).
-struct CellFit {
-  float* sum;
-  int32_t* count;
-  int32_t* strays;
-};
+// How well rows fit their pivots: per cell sum and count (cleared by the caller) of the cosines.  raw: the
+// pivot scan's dissimilarities; sq: squared norms (null: unit rows), of row map[i] for row i where given;
+// all_sum / all_count (an earlier call's; or null): only rows above their cell's mean.
 cudaError_t launch_cell_fit(const int32_t* label, const float* raw, int64_t n, int n_piv, const int32_t* sq,
-                            const CellFit& f, int32_t* list, int sms, cudaStream_t stream);
+                            const int32_t* map, const float* all_sum, const int32_t* all_count, float* sum,
+                            int32_t* count, int sms, cudaStream_t stream);
+// The rows that stray from their cell (listed in any order), and the other rows' sums and counts.
+cudaError_t launch_strays(const int32_t* label, const float* raw, int64_t n, int n_piv, const int32_t* sq,
+                          const float* sum, const int32_t* count, float* own_sum, int32_t* own_count, int32_t* list,
+                          int32_t* strays, int sms, cudaStream_t stream);
 // label[list[i]] = first + second[i].
 cudaError_t launch_stray_labels(const int32_t* list, const int32_t* second, int64_t count, int first, int n_second,
                                 int32_t* label, int sms, cudaStream_t stream);
-// rank[p] = the pivot's place in the order; label[i] = rank[label[i]].
-cudaError_t launch_prim_order(const float* sim, int64_t ld, int n, int32_t* rank, int32_t* label, int64_t n_rows,
-                              int sms, cudaStream_t stream);
-cudaError_t launch_group_stats(int mode, const void* rows, int64_t row_bytes, int64_t n, int64_t group_rows,
-                               int groups, int half_type, void* centres, const PruneStats& st, cudaStream_t stream);
-cudaError_t launch_prune_lists(int mode, int64_t n, int64_t group_rows, int groups, int64_t ld, const int32_t* U,
-                               const float* G, const PruneStats& st, const float* T, int half_len, int32_t* list,
-                               int32_t* len, int32_t* block_order, cudaStream_t stream);
+// rank[p] = the pivot's place in the order, attach[place] the similarity it was added at;
+// label[i] = rank[label[i]].
+cudaError_t launch_prim_order(const float* sim, int64_t ld, int n, int32_t* rank, float* attach, int32_t* label,
+                              int64_t n_rows, int sms, cudaStream_t stream);
+// Segments from the cells' places (end, size: in rank order) and fits (by pivot); cuts: scratch of n_piv
+// words; group_of[segment].
+cudaError_t launch_segments(const int32_t* rank, const float* attach, const float* own_sum, const int32_t* own_count,
+                            int n_piv, const int32_t* end, const int32_t* size, int64_t n, int64_t group_rows,
+                            int groups, int room, int32_t* cuts, const Segments& seg, int32_t* n_seg,
+                            int32_t* group_of, cudaStream_t stream);
+cudaError_t launch_segment_stats(int mode, const void* rows, int64_t row_bytes, const Segments& seg, int segments,
+                                 int half_type, void* centres, const PruneStats& st, cudaStream_t stream);
+cudaError_t launch_prune_lists(int mode, int64_t n, int64_t group_rows, int groups, const Segments& seg,
+                               const int32_t* group_of, int segments, int64_t ld, const int32_t* U, const float* G,
+                               const PruneStats& st, const float* T, int half_len, int32_t* list, int32_t* len,
+                               int32_t* block_order, cudaStream_t stream);
 
 // sym.cu.  Row j of dst = row j * stride of src for j < m, zero rows up to m_pad.
 cudaError_t launch_gather_strided_rows(const void* src, int64_t row_bytes, int64_t stride, int64_t m, int64_t m_pad,

@@ -5,21 +5,24 @@
 // row goes to its nearest pivot (n/512 evenly spaced rows), and the pivots are
 // visited as Prim's algorithm adds them to a maximum spanning tree of their
 // similarities, so whatever clusters the data has at whatever scale lie in
-// one run each.  Rows far less similar to their pivot than the other rows of
-// its cell are strays, members of clusters too small to have drawn a pivot;
+// one run each.  Rows far less similar to their pivot than the closer rows of
+// its cell (those above the cell's mean) are strays, members of clusters too small to have drawn a pivot;
 // one stray opens its whole tile, so the strays get pivots of their own
 // (every 64th) in a second round.  A group is `g` consecutive tiles (g = 1 up
-// to 2^20 rows) with a centre m, the mean of its rows rounded to the operand
-// type.
+// to 2^20 rows).  Where the order passes from one cluster to the next inside
+// a group (a pivot is added at a similarity under 0.75 of its cell's own), the
+// group is cut there: a segment is what lies between two cuts or group ends,
+// with a centre m, the mean of its rows rounded to the operand type.
 //
-// Bound.  With x = a_x m_A + x' for a row x of group A (a_x = x.m_A / |m_A|^2,
+// Bound.  With x = a_x m_A + x' for a row x of segment A (a_x = x.m_A / |m_A|^2,
 // x' orthogonal to m_A), for q in A and k in B
 //   q.k = a_q (k.m_A) + a_k (q.m_B - a_q m_A.m_B) + q'.k'
-// and q'.k' <= |q'| |k'|.  Per group the smallest and largest a and the
-// largest |x'| are known, per pair of groups the largest x.m_B over x in A
+// and q'.k' <= |q'| |k'|.  Per segment the smallest and largest a and the
+// largest |x'| are known, per pair of segments the largest x.m_B over x in A
 // (one product of the rows with the centres, the column maxima taken in its
 // epilogue) and m_A.m_B.  A pair is skipped when the bound stays below the
-// smallest of its query rows' thresholds: a score that keep other rows among
+// smallest of its query rows' thresholds; groups multiply when any pair of
+// their segments does.  A row's threshold is a score that keep other rows among
 // the 512 around the row's block reach (seed_kernel).  A skipped key
 // then scores strictly below keep keys of the row, so the kept sets are those
 // of the full scan, ties included.
@@ -32,7 +35,7 @@
 // operands of length L, exact for integers.  The bound adds up five such
 // terms of size at most N^2 (N the largest row norm); it is given 16 e N^2 and
 // 1e-5 N^2 more for the f32 arithmetic here.  For binary rows the bound on
-// the intersection becomes one on J through the groups' smallest popcounts.
+// the intersection becomes one on J through the segments' smallest popcounts.
 //
 // Replaces nothing in the reference, which prunes by its RP forest and
 // NN-descent (src/nndescent/float.rs:775-879) without a guarantee.
@@ -59,8 +62,8 @@ constexpr size_t kSmem = size_t(STAGES) * STAGE_BYTES + 1024 + 256;
 struct ProductParams {
   int64_t rows, n_ctiles;  // rows of A; tiles of 256 centres
   int n_kchunks, half_type;
-  int64_t group_rows;      // rows per group (column maxima)
-  void* out;               // kStore: f32 [rows][ld]; else int32 [groups][ld], maxima with 0
+  Segments seg;            // column maxima are per segment
+  void* out;               // kStore: f32 [rows][ld]; else int32 [segments][ld], maxima with 0
   int64_t ld;
   int* status;
   uint64_t timeout_ns, drain_ns;
@@ -69,7 +72,7 @@ struct ProductParams {
 
 // Rows x centres on the tensor cores (the scan's pipeline: TMA producer warp,
 // MMA warp, four epilogue warps, two accumulators).  kStore writes the
-// products; otherwise each column's maximum over the group's rows, as the
+// products; otherwise each column's maximum over a segment's rows, as the
 // signed pattern of a non-negative f32 or s32.  At 1M x 768 against 3,907
 // centres: 6 TFLOP.
 template <bool kInt8, bool kStore>
@@ -171,8 +174,16 @@ centre_product_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   } else {
     const int quad = warp & 3;
     uint32_t tile = 0;
+    int64_t last = -1;
+    int32_t seg = 0;
     for (int64_t i = blockIdx.x; i < items; i += gridDim.x, tile++) {
       const uint32_t a = tile & 1u;
+      if (!kStore && i / p.n_ctiles != last) {  // the lane's row's segment
+        last = i / p.n_ctiles;
+        const int64_t r = min(last * BM + quad * 32 + lane, p.rows - 1);  // rows past the data are zero
+        seg = p.seg.first[r / p.seg.group_rows];
+        while (p.seg.start[seg + 1] <= r) seg++;
+      }
       int got = 1;
       if (lane == 0) got = mbar_wait(&tfull[a], (tile >> 1) & 1u, abort, p.timeout_ns) ? 1 : 0;
       if (!__shfl_sync(0xffffffffu, got, 0)) {
@@ -200,15 +211,19 @@ centre_product_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
             }
           }
         } else {
-          int32_t mine = 0;  // lane j: column j's maximum (rows past the data are zero)
+          // the warp's rows mostly share a segment: one round
+          uint32_t todo = 0xffffffffu;
+          while (todo) {
+            const int32_t sg = __shfl_sync(0xffffffffu, seg, __ffs(todo) - 1);
+            todo &= ~__ballot_sync(0xffffffffu, seg == sg);
+            int32_t mine = 0;  // lane j: column j's maximum
 #pragma unroll
-          for (int j = 0; j < 32; j++) {
-            const int32_t m = __reduce_max_sync(0xffffffffu, int32_t(v[j]));
-            if (lane == j) mine = m;
+            for (int j = 0; j < 32; j++) {
+              const int32_t m = __reduce_max_sync(0xffffffffu, seg == sg ? int32_t(v[j]) : 0);
+              if (lane == j) mine = m;
+            }
+            if (mine > 0) atomicMax(static_cast<int32_t*>(p.out) + int64_t(sg) * p.ld + col0 + c + lane, mine);
           }
-          if (mine > 0)
-            atomicMax(static_cast<int32_t*>(p.out) + i / p.n_ctiles * BM / p.group_rows * p.ld + col0 + c + lane,
-                      mine);
         }
       }
       tc_fence_before();
@@ -416,44 +431,60 @@ namespace {
 
 // Visits the pivots as Prim's algorithm does, each time the one most similar
 // to any visited so far: a cluster of pivots at any similarity is one run.
-// One block; a step is one row of the similarities (from L2) and a block
-// maximum with a single barrier (two sets of warp results alternate).
+// One block, four pivots a thread; a step is one row of the similarities
+// (shared memory where the matrix fits it, else L2) and one block maximum.
+// Similarity and pivot share a word (20 and 12 bits: the order need not be
+// exact), so a maximum is one reduction a warp and one more over the warps,
+// with a single barrier between (two sets of warp results alternate).
+// Bound by that chain: ~0.35 us a step from shared memory, ~0.6 from L2.
 constexpr int kPrimThreads = 1024;
 constexpr int kPrimMax = 4096;
+constexpr int kPrimShared = 224;  // largest matrix kept in shared memory
 
+template <bool kShared>
 __global__ void __launch_bounds__(kPrimThreads)
-prim_order_kernel(const float* __restrict__ sim, int64_t ld, int n, int32_t* __restrict__ rank) {
-  __shared__ unsigned long long part[2][kPrimThreads / 32];
-  constexpr int PER = kPrimMax / kPrimThreads;
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  uint32_t best[PER];  // orderable similarity to the visited ones; 0: visited or past the end
-#pragma unroll
-  for (int u = 0; u < PER; u++) best[u] = t + u * kPrimThreads < n ? 1u : 0u;
-  int cur = 0;
-  for (int step = 0; step < n; step++) {
-    if (t == 0) rank[cur] = step;
-    uint32_t top = 0;
-    int at = 0;
-    float v[PER];  // all loads before the first use: a step is one L2 round trip
-#pragma unroll
-    for (int u = 0; u < PER; u++) v[u] = sim[int64_t(cur) * ld + min(t + u * kPrimThreads, n - 1)];
-#pragma unroll
-    for (int u = 0; u < PER; u++) {
-      const int j = t + u * kPrimThreads;
-      if (best[u] != 0u) best[u] = j == cur ? 0u : max(best[u], max(orderable(v[u]), 1u));
-      if (best[u] > top) {
-        top = best[u];
-        at = j;
-      }
-    }
-    const uint32_t wtop = __reduce_max_sync(0xffffffffu, top);
-    const uint32_t wat = __reduce_min_sync(0xffffffffu, top == wtop ? uint32_t(at) : 0xffffffffu);
-    if (lane == 0) part[step & 1][warp] = (static_cast<unsigned long long>(wtop) << 32) | wat;
+prim_order_kernel(const float* __restrict__ sim, int64_t ld, int n, int active, int32_t* __restrict__ rank,
+                  float* __restrict__ attach) {
+  extern __shared__ float matrix[];
+  __shared__ uint32_t part[2][32];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, warps = active >> 5;
+  if (kShared) {  // all threads load, `active` of them go on
+    for (int r = warp; r < n; r += int(blockDim.x) >> 5)
+#pragma unroll 4
+      for (int c = lane; c < n; c += 32) matrix[r * n + c] = sim[int64_t(r) * ld + c];
     __syncthreads();
-    const unsigned long long w = part[step & 1][lane];
-    const uint32_t btop = __reduce_max_sync(0xffffffffu, uint32_t(w >> 32));
-    cur = int(__reduce_min_sync(0xffffffffu, uint32_t(w >> 32) == btop ? uint32_t(w) : 0xffffffffu));
-    if (btop == 0u) break;  // all visited
+    if (t >= active) return;
+  }
+  uint32_t best[4];  // orderable similarity to the visited ones; 0: visited or past the end
+#pragma unroll
+  for (int u = 0; u < 4; u++) best[u] = t + u * active < n ? 1u << 12 : 0u;
+  int cur = 0;
+  float with = 0.0f;  // the similarity the current pivot was added at
+  for (int step = 0; step < n; step++) {
+    if (t == 0) {
+      rank[cur] = step;
+      attach[step] = with;
+    }
+    const float* row = kShared ? matrix + cur * n : sim + int64_t(cur) * ld;
+    float v[4];  // all loads before the first use
+#pragma unroll
+    for (int u = 0; u < 4; u++) v[u] = row[min(t + u * active, n - 1)];
+    uint32_t top = 0;
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const int j = t + u * active;
+      if (best[u] != 0u) best[u] = j == cur ? 0u : max(best[u], orderable(v[u]));
+      if (best[u] != 0u) top = max(top, (best[u] & ~0xfffu) | uint32_t(kPrimMax - 1 - j));
+    }
+    top = __reduce_max_sync(0xffffffffu, top);
+    if (warps > 1) {
+      if (lane == 0) part[step & 1][warp] = top;
+      asm volatile("bar.sync 1, %0;" ::"r"(active) : "memory");
+      top = __reduce_max_sync(0xffffffffu, lane < warps ? part[step & 1][lane] : 0u);
+    }
+    if (top == 0u) break;  // all visited
+    cur = kPrimMax - 1 - int(top & 0xfffu);
+    with = from_orderable(top & ~0xfffu);
   }
 }
 
@@ -476,11 +507,14 @@ __global__ void int8_sq_kernel(const uint8_t* __restrict__ rows, int64_t row_byt
   }
 }
 
+// Cosine of row i with its pivot.  Pivot p is row floor(p n / n_piv); map
+// (optional) leads from both to the rows sq is about.
 __device__ __forceinline__ float pivot_cosine(int64_t i, int32_t label, int n_piv, int64_t n, const float* raw,
-                                              const int32_t* sq) {
+                                              const int32_t* sq, const int32_t* map) {
   const float s = fmaxf(-raw[i], 0.0f);
   if (!sq) return s;  // unit rows
-  const float w = float(sq[i]) * float(sq[int64_t(label) * n / n_piv]);  // pivot p is row floor(p n / n_piv)
+  const int64_t p = int64_t(label) * n / n_piv;
+  const float w = float(sq[map ? map[i] : i]) * float(sq[map ? map[p] : p]);
   return w > 0.0f ? s * rsqrtf(w) : 0.0f;
 }
 
@@ -500,23 +534,36 @@ __global__ void sample_fit_kernel(const int32_t* __restrict__ label, const float
   if ((threadIdx.x & 31) == 0) atomicAdd(close, c);
 }
 
-// Per cell the sum of its rows' cosines with the pivot and their number.
+// Per cell the sum of its rows' cosines with the pivot and their number; with
+// all_sum / all_count (an earlier call's), of the rows above the cell's mean.
 __global__ void cell_fit_kernel(const int32_t* __restrict__ label, const float* __restrict__ raw, int64_t n, int n_piv,
-                                const int32_t* __restrict__ sq, CellFit f) {
+                                const int32_t* __restrict__ sq, const int32_t* __restrict__ map,
+                                const float* __restrict__ all_sum, const int32_t* __restrict__ all_count,
+                                float* __restrict__ sum, int32_t* __restrict__ count) {
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
     const int32_t b = min(max(label[i], 0), n_piv - 1);
-    atomicAdd(&f.sum[b], pivot_cosine(i, b, n_piv, n, raw, sq));
-    atomicAdd(&f.count[b], 1);
+    const float c = pivot_cosine(i, b, n_piv, n, raw, sq, map);
+    if (all_sum && c < all_sum[b] / float(max(all_count[b], 1))) continue;
+    atomicAdd(&sum[b], c);
+    atomicAdd(&count[b], 1);
   }
 }
 
-// Rows whose cosine is under 0.6 of their cell's mean.
+// Rows whose cosine is under 0.6 of the given mean; the other rows' sums.
 __global__ void strays_kernel(const int32_t* __restrict__ label, const float* __restrict__ raw, int64_t n, int n_piv,
-                              const int32_t* __restrict__ sq, CellFit f, int32_t* __restrict__ list) {
+                              const int32_t* __restrict__ sq, const float* __restrict__ sum,
+                              const int32_t* __restrict__ count, float* __restrict__ own_sum,
+                              int32_t* __restrict__ own_count, int32_t* __restrict__ list,
+                              int32_t* __restrict__ strays) {
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
     const int32_t b = min(max(label[i], 0), n_piv - 1);
-    if (pivot_cosine(i, b, n_piv, n, raw, sq) < 0.6f * f.sum[b] / float(max(f.count[b], 1)))
-      list[atomicAdd(f.strays, 1)] = int32_t(i);
+    const float c = pivot_cosine(i, b, n_piv, n, raw, sq, nullptr);
+    if (c < 0.6f * sum[b] / float(max(count[b], 1))) {
+      list[atomicAdd(strays, 1)] = int32_t(i);
+    } else {
+      atomicAdd(&own_sum[b], c);
+      atomicAdd(&own_count[b], 1);
+    }
   }
 }
 
@@ -533,42 +580,131 @@ __global__ void relabel_kernel(int32_t* __restrict__ label, int64_t n, const int
   }
 }
 
-__device__ __forceinline__ float half_at(const uint8_t* row, int c, int half_type) {
-  const uint16_t b = reinterpret_cast<const uint16_t*>(row)[c];
-  return half_type == kHalfBf16 ? __bfloat162float(__ushort_as_bfloat16(b)) : __half2float(__ushort_as_half(b));
+// The segments: group starts and, merged in, the starts of cells that begin a
+// cluster.  One block.  cell c (in rank order) holds rows [end[c] - size[c],
+// end[c]); room: segments the arrays hold.
+__global__ void __launch_bounds__(1024)
+segments_kernel(const int32_t* __restrict__ rank, const float* __restrict__ attach, const float* __restrict__ own_sum,
+                const int32_t* __restrict__ own_count, int n_piv, const int32_t* __restrict__ end,
+                const int32_t* __restrict__ size, int64_t n, int64_t group_rows, int groups, int room,
+                int32_t* __restrict__ cuts, Segments seg, int32_t* __restrict__ n_seg, int32_t* __restrict__ group_of) {
+  __shared__ uint8_t begins[kPrimMax];
+  __shared__ int32_t part[1024];
+  const int t = threadIdx.x;
+  for (int c = t; c < n_piv; c += 1024) {
+    const int r = rank[c];
+    const float own = own_sum[c] / float(max(own_count[c], 1));
+    begins[r] = r > 0 && own_count[c] > 0 && attach[r] < 0.75f * own ? 1 : 0;
+  }
+  __syncthreads();
+  const int per = (n_piv + 1023) / 1024;
+  int mine = 0;
+  for (int i = 0; i < per; i++) {
+    const int c = t * per + i;
+    if (c >= n_piv) break;
+    const int64_t at = int64_t(end[c]) - size[c];
+    if (size[c] == 0 || at <= 0 || at >= n || at % group_rows == 0) begins[c] = 0;
+    mine += begins[c];
+  }
+  part[t] = mine;
+  __syncthreads();
+  for (int off = 1; off < 1024; off <<= 1) {
+    const int32_t v = t >= off ? part[t - off] : 0;
+    __syncthreads();
+    part[t] += v;
+    __syncthreads();
+  }
+  const int n_cuts = min(part[1023], room - groups);
+  int at = part[t] - mine;
+  for (int i = 0; i < per; i++) {
+    const int c = t * per + i;
+    if (c >= n_piv) break;
+    if (begins[c]) {
+      if (at < n_cuts) cuts[at] = end[c] - size[c];  // cells are in row order, so the cuts ascend
+      at++;
+    }
+  }
+  __syncthreads();
+  // merge: a group start's place is its index plus the cuts before it, and the other way round
+  for (int g = t; g <= groups; g += 1024) {
+    const int64_t s = g < groups ? int64_t(g) * group_rows : n;
+    int lo = 0, hi = n_cuts;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (cuts[mid] < s) lo = mid + 1;
+      else hi = mid;
+    }
+    seg.start[g + lo] = int32_t(s);
+    if (g < groups) {
+      seg.first[g] = g + lo;
+      group_of[g + lo] = g;
+    } else {
+      seg.first[groups] = g + lo;
+      *n_seg = groups + n_cuts;
+    }
+  }
+  for (int i = t; i < n_cuts; i += 1024) {
+    const int g = int(cuts[i] / group_rows);  // its group's start lies before it
+    seg.start[i + g + 1] = cuts[i];
+    group_of[i + g + 1] = g;
+  }
 }
 
+// The 16 bytes at word w of a row: 8 16-bit or 16 int8 values.
 template <bool kInt8>
-__device__ __forceinline__ float elem(const uint8_t* row, int c, int half_type) {
-  return kInt8 ? float(reinterpret_cast<const int8_t*>(row)[c]) : half_at(row, c, half_type);
-}
+struct Lane16 {
+  static constexpr int N = kInt8 ? 16 : 8;
+  float v[N];
+  __device__ __forceinline__ Lane16(const uint8_t* row, int w, int half_type) {
+    const uint4 q = reinterpret_cast<const uint4*>(row)[w];
+    const uint32_t r[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+      if (kInt8) {
+        v[i] = float(int8_t(r[i >> 2] >> (8 * (i & 3))));
+      } else {
+        const uint16_t h = uint16_t(r[i >> 1] >> (16 * (i & 1)));
+        v[i] = half_type == kHalfBf16 ? __bfloat162float(__ushort_as_bfloat16(h)) : __half2float(__ushort_as_half(h));
+      }
+    }
+  }
+};
 
-// One block per group: its centre (16-bit: the mean scaled to unit length;
+// One block per segment: its centre (16-bit: the mean scaled to unit length;
 // int8: scaled to a largest entry of 127), then per row a_x and |x'|.
-// Two passes over the group's rows, the second from L2.
-constexpr int kStatThreads = 256;
+// Two passes over the segment's rows, the second from L2.
+constexpr int kStatThreads = 512;
 
 template <bool kInt8>
 __global__ void __launch_bounds__(kStatThreads)
-group_stats_kernel(const uint8_t* __restrict__ rows, int64_t row_bytes, int64_t n, int64_t group_rows, int half_type,
-                   uint8_t* __restrict__ centres, PruneStats st) {
+segment_stats_kernel(const uint8_t* __restrict__ rows, int64_t row_bytes, Segments seg, int half_type,
+                     uint8_t* __restrict__ centres, PruneStats st) {
   extern __shared__ float mean[];  // one value per element of a row, then the centre's values
   __shared__ float red[kStatThreads / 32][4];
   const int len = int(kInt8 ? row_bytes : row_bytes / 2);
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  const int64_t A = blockIdx.x, r0 = A * group_rows, r1 = min(n, r0 + group_rows);
+  const int64_t A = blockIdx.x, r0 = seg.start[A], r1 = seg.start[A + 1];
+  using Vec = Lane16<kInt8>;
+  for (int c = t; c < len; c += kStatThreads) mean[c] = 0.0f;
+  __syncthreads();
+  for (int w = lane; w < row_bytes / 16; w += 32) {  // each warp its rows, 16 bytes of a row a lane
+    float s[Vec::N];
+#pragma unroll
+    for (int i = 0; i < Vec::N; i++) s[i] = 0.0f;
+#pragma unroll 4
+    for (int64_t r = r0 + warp; r < r1; r += kStatThreads / 32) {
+      const Vec x(rows + r * row_bytes, w, half_type);
+#pragma unroll
+      for (int i = 0; i < Vec::N; i++) s[i] += x.v[i];
+    }
+#pragma unroll
+    for (int i = 0; i < Vec::N; i++) atomicAdd(&mean[w * Vec::N + i], s[i]);
+  }
+  __syncthreads();
   float acc_max = 0.0f, acc_sq = 0.0f;
   for (int c = t; c < len; c += kStatThreads) {
-    float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    int64_t r = r0;
-    for (; r + 4 <= r1; r += 4)
-#pragma unroll
-      for (int u = 0; u < 4; u++) s[u] += elem<kInt8>(rows + (r + u) * row_bytes, c, half_type);
-    for (; r < r1; r++) s[0] += elem<kInt8>(rows + r * row_bytes, c, half_type);
-    const float m = (s[0] + s[1]) + (s[2] + s[3]);
-    mean[c] = m;
-    acc_max = fmaxf(acc_max, fabsf(m));
-    acc_sq += m * m;
+    acc_max = fmaxf(acc_max, fabsf(mean[c]));
+    acc_sq += mean[c] * mean[c];
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -614,10 +750,14 @@ group_stats_kernel(const uint8_t* __restrict__ rows, int64_t row_bytes, int64_t 
   for (int64_t r = r0 + warp; r < r1; r += kStatThreads / 32) {
     const uint8_t* row = rows + r * row_bytes;
     float dot = 0.0f, sq = 0.0f;
-    for (int c = lane; c < len; c += 32) {
-      const float x = elem<kInt8>(row, c, half_type);
-      dot = fmaf(x, mean[c], dot);
-      sq = fmaf(x, x, sq);
+#pragma unroll 2
+    for (int w = lane; w < row_bytes / 16; w += 32) {
+      const Vec x(row, w, half_type);
+#pragma unroll
+      for (int i = 0; i < Vec::N; i++) {
+        dot = fmaf(x.v[i], mean[w * Vec::N + i], dot);
+        sq = fmaf(x.v[i], x.v[i], sq);
+      }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -660,63 +800,74 @@ group_stats_kernel(const uint8_t* __restrict__ rows, int64_t row_bytes, int64_t 
   }
 }
 
-// One block per group A: the ascending list of groups B it has to multiply.
+// One block per group: the ascending list of groups it has to multiply.
 constexpr int kDecideThreads = 256;
 
 __global__ void __launch_bounds__(kDecideThreads)
-decide_kernel(int mode, int64_t n, int64_t group_rows, int groups, int64_t ld, const int32_t* __restrict__ U,
-              const float* __restrict__ G, PruneStats st, const float* __restrict__ T, int half_len,
-              int32_t* __restrict__ list, int32_t* __restrict__ len) {
+decide_kernel(int mode, Segments seg, const int32_t* __restrict__ group_of, int segments, int groups, int64_t ld,
+              const int32_t* __restrict__ U, const float* __restrict__ G, PruneStats st, const float* __restrict__ T,
+              int half_len, int32_t* __restrict__ list, int32_t* __restrict__ len) {
   __shared__ float red[kDecideThreads / 32];
   __shared__ int base, counts[kDecideThreads / 32];
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, A = blockIdx.x;
-  // the smallest of the rows' thresholds, as a score (-FLT_MAX: no bound)
-  float thr = FLT_MAX;
-  for (int64_t r = A * group_rows + t; r < min(n, (A + 1) * group_rows); r += kDecideThreads) {
-    const float raw = T[r];
-    const bool none = raw == kHeapInf || (mode != kScanInt8 && raw >= 0.0f);
-    thr = fminf(thr, none ? -FLT_MAX : -raw);
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) thr = fminf(thr, __shfl_xor_sync(0xffffffffu, thr, o));
-  if (lane == 0) red[warp] = thr;
-  if (t == 0) base = 0;
-  __syncthreads();
-  for (int w = 0; w < kDecideThreads / 32; w++) thr = fminf(thr, red[w]);
+  __shared__ uint32_t hit[kPruneGroups / 32];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, g = blockIdx.x;
+  for (int i = t; i < kPruneGroups / 32; i += kDecideThreads) hit[i] = 0u;
   const float nn = __uint_as_float(*st.top);
   const float e = mode == kScanHalf ? (float(half_len) / 4.0f + 2.0f) * 0x1p-21f * 16.0f : 0.0f;
   const float slack = (e + 1e-5f) * nn;
-  const float a0 = st.a0[A], a1 = st.a1[A], rho = st.rho[A], sqa = st.sq0[A];
   auto value = [&](int32_t u) { return mode == kScanHalf ? __int_as_float(u) : float(u); };
-  for (int b0 = 0; b0 < groups; b0 += kDecideThreads) {
-    const int B = b0 + t;
-    bool in = false;
-    if (B < groups) {
-      const float uab = value(U[A * ld + B]), uba = value(U[B * ld + A]), g = G[A * ld + B];
+  __syncthreads();
+  for (int A = seg.first[g]; A < seg.first[g + 1]; A++) {
+    // the smallest of the rows' thresholds, as a score (-FLT_MAX: no bound)
+    float thr = FLT_MAX;
+    for (int r = seg.start[A] + t; r < seg.start[A + 1]; r += kDecideThreads) {
+      const float raw = T[r];
+      const bool none = raw == kHeapInf || (mode != kScanInt8 && raw >= 0.0f);
+      thr = fminf(thr, none ? -FLT_MAX : -raw);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) thr = fminf(thr, __shfl_xor_sync(0xffffffffu, thr, o));
+    __syncthreads();
+    if (lane == 0) red[warp] = thr;
+    __syncthreads();
+    for (int w = 0; w < kDecideThreads / 32; w++) thr = fminf(thr, red[w]);
+    const float a0 = st.a0[A], a1 = st.a1[A], rho = st.rho[A], sqa = st.sq0[A];
+    for (int B = t; B < segments; B += kDecideThreads) {
+      const float uab = value(U[A * ld + B]), uba = value(U[B * ld + A]), gab = G[A * ld + B];
       const float c0 = st.a0[B], c1 = st.a1[B];
-      const float w = uab - fminf(a0 * g, a1 * g);
+      const float w = uab - fminf(a0 * gab, a1 * gab);
       const float top = a1 * uba + fmaxf(c0 * w, c1 * w) + rho * st.rho[B] + slack;
-      // a row against its centre (never seen) leaves the bound's sign cases: keep the pair
-      in = A == B || a0 < 0.0f || c0 < 0.0f || !(thr > -FLT_MAX);
+      // a row turned against its centre leaves the bound's sign cases: keep the pair
+      bool in = A == B || a0 < 0.0f || c0 < 0.0f || !(thr > -FLT_MAX);
       if (!in && mode == kScanJaccard) {
         const float size = sqa + st.sq0[B] - top;  // J <= i / (|a| + |b| - i), increasing in i
         in = !(size > 0.0f) || top >= thr * size * (1.0f - 1e-5f);
       } else if (!in) {
         in = !(top < thr);
       }
+      if (in) {
+        const int h = group_of[B];
+        if (!(hit[h >> 5] >> (h & 31) & 1u)) atomicOr(&hit[h >> 5], 1u << (h & 31));
+      }
     }
+  }
+  if (t == 0) base = 0;
+  __syncthreads();
+  for (int b0 = 0; b0 < groups; b0 += kDecideThreads) {
+    const int b = b0 + t;
+    const bool in = b < groups && (hit[b >> 5] >> (b & 31) & 1u);
     const uint32_t who = __ballot_sync(0xffffffffu, in);
     if (lane == 0) counts[warp] = __popc(who);
     __syncthreads();
     int at = base;
     for (int w = 0; w < warp; w++) at += counts[w];
-    if (in) list[int64_t(A) * groups + at + __popc(who & ((1u << lane) - 1u))] = B;
+    if (in) list[int64_t(g) * groups + at + __popc(who & ((1u << lane) - 1u))] = b;
     __syncthreads();
     if (t == 0)
       for (int w = 0; w < kDecideThreads / 32; w++) base += counts[w];
     __syncthreads();
   }
-  if (t == 0) len[A] = base;
+  if (t == 0) len[g] = base;
 }
 
 // The query blocks by descending list length (counting sort in one block):
@@ -758,12 +909,12 @@ block_order_kernel(const int32_t* __restrict__ len, int groups, int64_t n_blocks
 }  // namespace
 
 cudaError_t launch_centre_products(int mode, const void* A, int64_t a_rows_mem, int64_t rows, const void* C,
-                                   int64_t c_rows_mem, int64_t row_bytes, int half_type, bool store,
-                                   int64_t group_rows, void* out, int64_t ld, int* status, uint64_t timeout_ns,
-                                   int sms, cudaStream_t stream) {
-  if (row_bytes % KCB || rows < 1 || a_rows_mem < rows || c_rows_mem % BN || ld < c_rows_mem || ld % 4 ||
-      group_rows % BM)
+                                   int64_t c_rows_mem, int64_t row_bytes, int half_type, const Segments* seg,
+                                   void* out, int64_t ld, int* status, uint64_t timeout_ns, int sms,
+                                   cudaStream_t stream) {
+  if (row_bytes % KCB || rows < 1 || a_rows_mem < rows || c_rows_mem % BN || ld < c_rows_mem || ld % 4)
     return cudaErrorInvalidValue;
+  const bool store = seg == nullptr;
   const int eb = mode == kScanHalf ? 2 : 1;
   alignas(64) CUtensorMap ma, mb;
   if (!encode_row_map(&ma, A, a_rows_mem, row_bytes, eb, BM, half_type) ||
@@ -774,7 +925,7 @@ cudaError_t launch_centre_products(int mode, const void* A, int64_t a_rows_mem, 
   p.n_ctiles = c_rows_mem / BN;
   p.n_kchunks = int(row_bytes / KCB);
   p.half_type = half_type;
-  p.group_rows = group_rows;
+  if (seg) p.seg = *seg;
   p.out = out;
   p.ld = ld;
   p.status = status;
@@ -838,9 +989,26 @@ cudaError_t launch_sample_fit(const int32_t* label, const float* raw, int m, int
 }
 
 cudaError_t launch_cell_fit(const int32_t* label, const float* raw, int64_t n, int n_piv, const int32_t* sq,
-                            const CellFit& f, int32_t* list, int sms, cudaStream_t stream) {
-  cell_fit_kernel<<<sms * 4, 256, 0, stream>>>(label, raw, n, n_piv, sq, f);
-  strays_kernel<<<sms * 4, 256, 0, stream>>>(label, raw, n, n_piv, sq, f, list);
+                            const int32_t* map, const float* all_sum, const int32_t* all_count, float* sum,
+                            int32_t* count, int sms, cudaStream_t stream) {
+  cell_fit_kernel<<<sms * 4, 256, 0, stream>>>(label, raw, n, n_piv, sq, map, all_sum, all_count, sum, count);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_strays(const int32_t* label, const float* raw, int64_t n, int n_piv, const int32_t* sq,
+                          const float* sum, const int32_t* count, float* own_sum, int32_t* own_count, int32_t* list,
+                          int32_t* strays, int sms, cudaStream_t stream) {
+  strays_kernel<<<sms * 4, 256, 0, stream>>>(label, raw, n, n_piv, sq, sum, count, own_sum, own_count, list, strays);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_segments(const int32_t* rank, const float* attach, const float* own_sum, const int32_t* own_count,
+                            int n_piv, const int32_t* end, const int32_t* size, int64_t n, int64_t group_rows,
+                            int groups, int room, int32_t* cuts, const Segments& seg, int32_t* n_seg,
+                            int32_t* group_of, cudaStream_t stream) {
+  if (n_piv < 1 || n_piv > kPrimMax || room < groups) return cudaErrorInvalidValue;
+  segments_kernel<<<1, 1024, 0, stream>>>(rank, attach, own_sum, own_count, n_piv, end, size, n, group_rows, groups,
+                                          room, cuts, seg, n_seg, group_of);
   return cudaGetLastError();
 }
 
@@ -850,16 +1018,24 @@ cudaError_t launch_stray_labels(const int32_t* list, const int32_t* second, int6
   return cudaGetLastError();
 }
 
-cudaError_t launch_prim_order(const float* sim, int64_t ld, int n, int32_t* rank, int32_t* label, int64_t n_rows,
-                              int sms, cudaStream_t stream) {
+cudaError_t launch_prim_order(const float* sim, int64_t ld, int n, int32_t* rank, float* attach, int32_t* label,
+                              int64_t n_rows, int sms, cudaStream_t stream) {
   if (n < 1 || n > kPrimMax) return cudaErrorInvalidValue;
-  prim_order_kernel<<<1, kPrimThreads, 0, stream>>>(sim, ld, n, rank);
+  const int threads = ((n + 3) / 4 + 31) / 32 * 32;
+  if (n <= kPrimShared) {
+    const cudaError_t e = cudaFuncSetAttribute(prim_order_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               kPrimShared * kPrimShared * 4);
+    if (e != cudaSuccess) return e;
+    prim_order_kernel<true><<<1, kPrimThreads, size_t(n) * n * 4, stream>>>(sim, ld, n, threads, rank, attach);
+  } else {
+    prim_order_kernel<false><<<1, threads, 0, stream>>>(sim, ld, n, threads, rank, attach);
+  }
   relabel_kernel<<<sms * 4, 256, 0, stream>>>(label, n_rows, rank, n);
   return cudaGetLastError();
 }
 
-cudaError_t launch_group_stats(int mode, const void* rows, int64_t row_bytes, int64_t n, int64_t group_rows,
-                               int groups, int half_type, void* centres, const PruneStats& st, cudaStream_t stream) {
+cudaError_t launch_segment_stats(int mode, const void* rows, int64_t row_bytes, const Segments& seg, int segments,
+                                 int half_type, void* centres, const PruneStats& st, cudaStream_t stream) {
   const int len = int(mode == kScanHalf ? row_bytes / 2 : row_bytes);
   const size_t smem = size_t(len) * sizeof(float);
   if (smem > 200 * 1024) return cudaErrorInvalidValue;
@@ -868,19 +1044,20 @@ cudaError_t launch_group_stats(int mode, const void* rows, int64_t row_bytes, in
   auto go = [&](auto kern) {
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     if (e != cudaSuccess) return e;
-    kern<<<unsigned(groups), kStatThreads, smem, stream>>>(static_cast<const uint8_t*>(rows), row_bytes, n, group_rows,
-                                                           half_type, static_cast<uint8_t*>(centres), st);
+    kern<<<unsigned(segments), kStatThreads, smem, stream>>>(static_cast<const uint8_t*>(rows), row_bytes, seg,
+                                                             half_type, static_cast<uint8_t*>(centres), st);
     return cudaGetLastError();
   };
-  return mode == kScanHalf ? go(group_stats_kernel<false>) : go(group_stats_kernel<true>);
+  return mode == kScanHalf ? go(segment_stats_kernel<false>) : go(segment_stats_kernel<true>);
 }
 
-cudaError_t launch_prune_lists(int mode, int64_t n, int64_t group_rows, int groups, int64_t ld, const int32_t* U,
-                               const float* G, const PruneStats& st, const float* T, int half_len, int32_t* list,
-                               int32_t* len, int32_t* block_order, cudaStream_t stream) {
-  if (groups < 1 || groups > kPruneGroups) return cudaErrorInvalidValue;
-  decide_kernel<<<unsigned(groups), kDecideThreads, 0, stream>>>(mode, n, group_rows, groups, ld, U, G, st, T,
-                                                                 half_len, list, len);
+cudaError_t launch_prune_lists(int mode, int64_t n, int64_t group_rows, int groups, const Segments& seg,
+                               const int32_t* group_of, int segments, int64_t ld, const int32_t* U, const float* G,
+                               const PruneStats& st, const float* T, int half_len, int32_t* list, int32_t* len,
+                               int32_t* block_order, cudaStream_t stream) {
+  if (groups < 1 || groups > kPruneGroups || segments < groups) return cudaErrorInvalidValue;
+  decide_kernel<<<unsigned(groups), kDecideThreads, 0, stream>>>(mode, seg, group_of, segments, groups, ld, U, G, st,
+                                                                 T, half_len, list, len);
   block_order_kernel<<<1, 1024, size_t(groups + 1) * 4, stream>>>(len, groups, (n + BM - 1) / BM,
                                                                   int(group_rows / BM), block_order);
   return cudaGetLastError();

@@ -747,6 +747,8 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       for (int64_t ti = 0; ti < v.n_ktiles - v.kt0; ti++, tile++) {
         const int64_t kt = next;
         if (ti + 1 < v.n_ktiles - v.kt0) next = tile_at<kSym, kList>(v, ti + 1, p.lists.lg);
+        // list mode: the next tile's row indices (1 KB) on their way to L1, where a survivor reads its own
+        if (kList && lane < 8) prefetch_l1(perm + min(next * BN + lane * 32, v.n_k - 1));
         const uint32_t a = tile & 1u, tph = (tile >> 1) & 1u;
         int got = 1;
         if (lane == 0) got = mbar_wait(&tfull[a], tph, abort, p.timeout_ns) ? 1 : 0;
