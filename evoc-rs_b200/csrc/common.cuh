@@ -18,7 +18,8 @@ constexpr float kHeapInf = 3.40282347e+38f;      // f32::MAX, heap.rs:8
 constexpr uint64_t kKeyInf = ~0ull;
 
 // Codes of a request's device status word (0 = ok).  1..3: a pipeline wait of
-// the tensor-core scan ran out (producer, MMA issuer, epilogue); 16, 17: a
+// the tensor-core scan ran out (producer, MMA issuer, epilogue); 4: a copy of
+// the rerank did not arrive in time; 16, 17: a
 // self-check found a malformed row order or a candidate index out of range
 // and skipped it.
 constexpr int kStatusBadOrder = 16;

@@ -36,11 +36,13 @@
 // processed grouped by their nearest pivot (a deterministic sample of the
 // data found with the same tensor-core scan), so the warps in flight at any
 // moment work on nearby points whose candidates overlap.
+#include <algorithm>
 #include <cuda_bf16.h>
 
 #include "batch.h"
 #include "common.cuh"
 #include "kernels.h"
+#include "sm100.cuh"
 
 namespace evoc {
 
@@ -48,6 +50,7 @@ namespace {
 constexpr int RW = 8;          // warps per block
 constexpr int MAXC = 256;      // candidates per row handled in shared memory
 constexpr int GROUP = 4;       // candidates per pass over the query row
+constexpr int STEP = 4;        // column steps of 32 loaded ahead
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
@@ -112,45 +115,16 @@ __device__ __forceinline__ bool certify_row(const CertArgs& ct, const uint64_t* 
 }
 }  // namespace
 
-// One query row: FP32 dot products with its C candidates, a warp bitonic
-// sort of (raw, index) keys, FP64 at the k-th boundary, the sorted row
-// written to output row q.  kw: this warp's P key slots; dw: its 32 doubles.
-// With ct (and b_c, the scan's C-th kept raw value), returns whether the row
-// is certified (always true without).
-__device__ __forceinline__ bool rerank_row(const float* __restrict__ X, int ld, int d, int64_t n_keys, int64_t q,
-                                           int64_t qg, const int32_t* __restrict__ cq, int C, int P, int k,
-                                           int32_t* __restrict__ out_idx, float* __restrict__ out_raw,
-                                           float* __restrict__ out_dist, int* status, uint64_t* kw, double* dw,
-                                           int lane, const CertArgs* ct = nullptr, float b_c = 0.0f) {
+// From a query row's C keys (FP32) in kw: a warp bitonic sort of (raw, index)
+// keys, FP64 at the k-th boundary, the sorted row written to output row q.
+// kw: this warp's P key slots; dw: its 32 doubles.  With ct (and b_c, the
+// scan's C-th kept raw value), returns whether the row is certified (always
+// true without).
+__device__ __forceinline__ bool finish_row(const float* __restrict__ X, int ld, int d, int64_t n_keys, int64_t q,
+                                           int64_t qg, int C, int P, int k, int32_t* __restrict__ out_idx,
+                                           float* __restrict__ out_raw, float* __restrict__ out_dist, uint64_t* kw,
+                                           double* dw, int lane, const CertArgs* ct, float b_c) {
   const float* xq = X + qg * ld;
-  for (int j0 = 0; j0 < C; j0 += GROUP) {
-    int32_t id[GROUP];
-    float acc[GROUP];
-#pragma unroll
-    for (int u = 0; u < GROUP; u++) {
-      id[u] = (j0 + u < C) ? cq[j0 + u] : -1;
-      if (id[u] >= n_keys) {  // never written by a finished scan: record it, skip the candidate
-        if (status) atomicCAS(status, 0, kStatusBadCandidate);
-        id[u] = -1;
-      }
-      acc[u] = 0.0f;
-    }
-    for (int t = lane; t < d; t += 32) {
-      const float xv = xq[t];
-#pragma unroll
-      for (int u = 0; u < GROUP; u++)
-        if (id[u] >= 0) acc[u] = fmaf(xv, X[int64_t(id[u]) * ld + t], acc[u]);
-    }
-#pragma unroll
-    for (int u = 0; u < GROUP; u++) {
-      const float dot = warp_sum(acc[u]);
-      if (lane == u && j0 + u < C) {
-        uint64_t key = kKeyInf;
-        if (id[u] >= 0) key = make_key(id[u] == qg ? -1.0f : raw_cosine(dot), id[u]);
-        kw[j0 + u] = key;
-      }
-    }
-  }
   for (int j = C + lane; j < P; j += 32) kw[j] = kKeyInf;
   __syncwarp();
   warp_bitonic(kw, P, lane);
@@ -206,6 +180,69 @@ __device__ __forceinline__ bool rerank_row(const float* __restrict__ X, int ld, 
   return certified;
 }
 
+// One query row: FP32 dot products with its C candidates, then finish_row.
+__device__ __forceinline__ bool rerank_row(const float* __restrict__ X, int ld, int d, int64_t n_keys, int64_t q,
+                                           int64_t qg, const int32_t* __restrict__ cq, int C, int P, int k,
+                                           int32_t* __restrict__ out_idx, float* __restrict__ out_raw,
+                                           float* __restrict__ out_dist, int* status, uint64_t* kw, double* dw,
+                                           int lane, const CertArgs* ct = nullptr, float b_c = 0.0f) {
+  const float* xq = X + qg * ld;
+  // Bound by the L2's latency: what counts is loads in flight.  Candidate ids
+  // come 32 at a time (a lane each), and STEP x 32 columns of GROUP candidates
+  // are loaded before the first product.  (One column step at a time, every
+  // step waited for its own loads: 20,011 x 384 at 38 candidates took 0.23 ms,
+  // now 0.19.)
+  int32_t mine = -1, next = lane < C ? cq[lane] : -1;
+  for (int j0 = 0; j0 < C; j0 += GROUP) {
+    if (j0 % 32 == 0) {
+      mine = next;
+      next = j0 + 32 + lane < C ? cq[j0 + 32 + lane] : -1;
+      if (mine >= n_keys) {  // never written by a finished scan: record it, skip the candidate
+        if (status) atomicCAS(status, 0, kStatusBadCandidate);
+        mine = -1;
+      }
+    }
+    int32_t id[GROUP];
+    const float* y[GROUP];  // a missing candidate reads the query row; its product is not used
+    float acc[GROUP];
+#pragma unroll
+    for (int u = 0; u < GROUP; u++) {
+      id[u] = __shfl_sync(0xffffffffu, mine, (j0 + u) % 32);
+      y[u] = X + (id[u] >= 0 ? int64_t(id[u]) : qg) * ld;
+      acc[u] = 0.0f;
+    }
+    int t = lane;
+    for (; t - lane + 32 * STEP <= d; t += 32 * STEP) {
+      float xv[STEP], yv[GROUP][STEP];
+#pragma unroll
+      for (int i = 0; i < STEP; i++) {
+        xv[i] = xq[t + 32 * i];
+#pragma unroll
+        for (int u = 0; u < GROUP; u++) yv[u][i] = y[u][t + 32 * i];
+      }
+#pragma unroll
+      for (int i = 0; i < STEP; i++)
+#pragma unroll
+        for (int u = 0; u < GROUP; u++) acc[u] = fmaf(xv[i], yv[u][i], acc[u]);
+    }
+    for (; t < d; t += 32) {
+      const float xv = xq[t];
+#pragma unroll
+      for (int u = 0; u < GROUP; u++) acc[u] = fmaf(xv, y[u][t], acc[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < GROUP; u++) {
+      const float dot = warp_sum(acc[u]);
+      if (lane == u && j0 + u < C) {
+        uint64_t key = kKeyInf;
+        if (id[u] >= 0) key = make_key(id[u] == qg ? -1.0f : raw_cosine(dot), id[u]);
+        kw[j0 + u] = key;
+      }
+    }
+  }
+  return finish_row(X, ld, d, n_keys, q, qg, C, P, k, out_idx, out_raw, out_dist, kw, dw, lane, ct, b_c);
+}
+
 __global__ void __launch_bounds__(RW * 32)
 rerank_f32_kernel(const float* __restrict__ X, int ld, int d, int64_t n, int64_t n_keys, int64_t q_row0,
                   const int32_t* __restrict__ cand, int C, int k, const int32_t* __restrict__ order,
@@ -228,6 +265,127 @@ rerank_f32_kernel(const float* __restrict__ X, int ld, int d, int64_t n, int64_t
     const bool ok = rerank_row(X, ld, d, n_keys, q, q_row0 + q, cand + ci * C, C, P, k, out_idx, out_raw, out_dist,
                                status, keys[warp], d64[warp], lane, use_cert ? &cert : nullptr,
                                use_cert ? cert.bound[ci] : 0.0f);
+    if (!ok && lane == 0) {
+      const int slot = atomicAdd(cert.fail_count, 1);
+      if (slot < cert.fail_cap) cert.fail_list[slot] = int32_t(q);
+    }
+  }
+}
+
+// The same with the candidate rows brought into shared memory by bulk copies:
+// every warp keeps a ring of `slots` rows in flight, far more than registers
+// could hold, and takes its products from there in the same order (so the
+// results are the same bit for bit).  Bound by L2 bandwidth: 6.8 TB/s of
+// gathered rows.  1,000,000 x 768 with 60 candidates 27 ms (loads through
+// registers: 38), 200,000 x 768 with 75 the same 6.4; below 512 features the
+// copies are too short and the few warps show (20,011 x 384: 0.34 ms against
+// 0.19, 50,000 x 200: 0.77 against 0.34), above 1,600 two rows a warp no
+// longer fit.
+constexpr int BW = 16;  // warps per block, one block per SM
+constexpr int kBulkMin = 512, kBulkMax = 1600;  // row lengths taken
+
+__global__ void __launch_bounds__(BW * 32, 1)
+rerank_bulk_kernel(const float* __restrict__ X, int ld, int d, int64_t n, int64_t n_keys, int64_t q_row0,
+                   const int32_t* __restrict__ cand, int C, int P, int k, int slots,
+                   const int32_t* __restrict__ order, int32_t* __restrict__ out_idx, float* __restrict__ out_raw,
+                   float* __restrict__ out_dist, int* status, const CertArgs cert, bool use_cert, bool by_item,
+                   int64_t n_out) {
+  using namespace sm100;
+  extern __shared__ __align__(128) uint8_t smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // per warp: the query row and `slots` candidate rows (ld floats each), P keys, 32 doubles, the slots' barriers
+  const size_t per_warp = size_t(slots + 1) * ld * 4 + size_t(P) * 8 + 32 * 8 + size_t(slots) * 8;
+  uint8_t* mine = smem + warp * per_warp;
+  float* query = reinterpret_cast<float*>(mine);
+  float* ring = query + ld;
+  uint64_t* kw = reinterpret_cast<uint64_t*>(ring + size_t(slots) * ld);
+  double* dw = reinterpret_cast<double*>(kw + P);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(dw + 32);
+  if (*reinterpret_cast<volatile int*>(status) != 0) return;  // block-uniform: the scan has finished
+  if (lane == 0) {
+    for (int s = 0; s < slots; s++) mbar_init(&bars[s], 1);
+    fence_barrier_init();
+  }
+  __syncwarp();
+  const uint32_t bytes = uint32_t(ld) * 4u;
+  uint32_t used = 0;  // copies waited for so far: copy i uses slot i % slots, in its phase i / slots
+  bool alive = true;
+  for (int64_t w = int64_t(blockIdx.x) * BW + warp; alive && w < n; w += int64_t(gridDim.x) * BW) {
+    const int64_t q = order ? order[w] : w;  // output row
+    if (q < 0 || q >= n_out) {               // a malformed order: record it, skip the row
+      if (lane == 0) atomicCAS(status, 0, kStatusBadOrder);
+      continue;
+    }
+    const int64_t ci = by_item ? w : q, qg = q_row0 + q;  // candidate row, row of X
+    const int32_t* cq = cand + ci * C;
+    // a candidate's row; a missing one reads the query row, its product is not used
+    auto candidate = [&](int32_t id) {
+      if (id >= n_keys) {  // never written by a finished scan: record it, skip the candidate
+        atomicCAS(status, 0, kStatusBadCandidate);
+        id = -1;
+      }
+      return id;
+    };
+    // lane 0 has the ids it copies by from the warp's 32-wide reads
+    int32_t ids = lane < C ? candidate(cq[lane]) : -1, ahead = 32 + lane < C ? candidate(cq[32 + lane]) : -1;
+    int32_t later = 64 + lane < C ? candidate(cq[64 + lane]) : -1;  // two reads ahead: a slot's copy needs at most 32 on
+    auto copy = [&](int j, int base) {  // candidate j, ids holding base .. base + 31
+      const int32_t a = __shfl_sync(0xffffffffu, ids, j & 31), b = __shfl_sync(0xffffffffu, ahead, j & 31);
+      const int32_t id = j < base + 32 ? a : b;
+      if (lane == 0) {
+        const uint32_t s = (used + uint32_t(j)) % uint32_t(slots);
+        mbar_arrive_expect_tx(&bars[s], bytes);
+        bulk_load(ring + size_t(s) * ld, X + (id >= 0 ? int64_t(id) : qg) * ld, bytes, &bars[s]);
+      }
+    };
+    int sent = 0;
+    for (; sent < slots && sent < C; sent++) copy(sent, 0);
+    for (int t = lane; t < ld; t += 32) query[t] = X[qg * ld + t];
+    __syncwarp();
+    for (int j0 = 0, base = 0; j0 < sent; j0 += 2) {  // sent stays ahead, up to C
+      if (j0 == base + 32) {
+        base = j0;
+        ids = ahead;
+        ahead = later;
+        later = base + 64 + lane < C ? candidate(cq[base + 64 + lane]) : -1;
+      }
+      const float* y[2];
+      int32_t id[2];
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        const int j = j0 + u < sent ? j0 + u : j0;
+        const uint32_t i = used + uint32_t(j), s = i % uint32_t(slots);
+        id[u] = __shfl_sync(0xffffffffu, ids, j & 31);
+        y[u] = ring + size_t(s) * ld;
+        int got = 1;
+        if (lane == 0) got = mbar_wait(&bars[s], (i / uint32_t(slots)) & 1u, nullptr, 4000000000ull) ? 1 : 0;
+        got = __shfl_sync(0xffffffffu, got, 0);
+        __syncwarp();
+        if (!got) {  // send no more; the copies already sent are still waited for
+          if (lane == 0) atomicCAS(status, 0, 4);
+          alive = false;
+        }
+      }
+      float acc[2] = {0.0f, 0.0f};
+#pragma unroll 4
+      for (int t = lane; t < d; t += 32) {
+        const float xv = query[t];
+        acc[0] = fmaf(xv, y[0][t], acc[0]);
+        acc[1] = fmaf(xv, y[1][t], acc[1]);
+      }
+      __syncwarp();  // the slots have been read
+      for (int u = 0; alive && u < 2 && sent < C; u++, sent++) copy(sent, base);
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        const float dot = warp_sum(acc[u]);
+        if (lane == u && j0 + u < C)
+          kw[j0 + u] = id[u] >= 0 ? make_key(id[u] == qg ? -1.0f : raw_cosine(dot), id[u]) : kKeyInf;
+      }
+    }
+    used += uint32_t(C);
+    if (!alive) break;
+    const bool ok = finish_row(X, ld, d, n_keys, q, qg, C, P, k, out_idx, out_raw, out_dist, kw, dw, lane,
+                               use_cert ? &cert : nullptr, use_cert ? cert.bound[ci] : 0.0f);
     if (!ok && lane == 0) {
       const int slot = atomicAdd(cert.fail_count, 1);
       if (slot < cert.fail_cap) cert.fail_list[slot] = int32_t(q);
@@ -283,10 +441,26 @@ cudaError_t launch_rerank_f32(const float* X, int ld, int d, int64_t n, int64_t 
   if (by_item && !order) return cudaErrorInvalidValue;
   if (cert && (!cert->bound || !cert->rnorm || !cert->hnorm || !cert->maxes || !cert->fail_list || !cert->fail_count))
     return cudaErrorInvalidValue;
-  int64_t blocks = (n + RW - 1) / RW;
-  if (blocks > int64_t(sms) * 16) blocks = int64_t(sms) * 16;
   CertArgs ct{};
   if (cert) ct = *cert;
+  int P = 1;
+  while (P < C || P < 2) P <<= 1;
+  const size_t limit = 227 * 1024 - 1024, fixed = size_t(ld) * 4 + size_t(P) * 8 + 32 * 8;
+  const int64_t slots = (int64_t(limit / BW) - int64_t(fixed)) / (int64_t(ld) * 4 + 8);
+  if (status && ld >= kBulkMin && ld <= kBulkMax && slots >= 2) {
+    const int s = int(std::min<int64_t>(slots & ~int64_t(1), 16));
+    const size_t smem = BW * (fixed + size_t(s) * (size_t(ld) * 4 + 8));
+    const cudaError_t e = cudaFuncSetAttribute(rerank_bulk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               227 * 1024);
+    if (e != cudaSuccess) return e;
+    const int64_t grid = std::min<int64_t>((n + BW - 1) / BW, sms);
+    rerank_bulk_kernel<<<unsigned(grid), BW * 32, smem, stream>>>(X, ld, d, n, n_keys, q_row0, cand, C, P, k, s, order,
+                                                                  out_idx, out_raw, out_dist, status, ct,
+                                                                  cert != nullptr, by_item, n_out < 0 ? n : n_out);
+    return cudaGetLastError();
+  }
+  int64_t blocks = (n + RW - 1) / RW;
+  if (blocks > int64_t(sms) * 16) blocks = int64_t(sms) * 16;
   rerank_f32_kernel<<<unsigned(blocks), RW * 32, 0, stream>>>(X, ld, d, n, n_keys, q_row0, cand, C, k, order,
                                                                out_idx, out_raw, out_dist, status, ct, cert != nullptr,
                                                                by_item, n_out < 0 ? n : n_out);
