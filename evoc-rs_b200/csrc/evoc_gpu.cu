@@ -903,6 +903,9 @@ int run_int8(evoc_gpu_ctx* ctx, const Job& j, int64_t ldb) {
 // Bytes per row of the 0/1 int8 expansion of `nbytes` packed bytes.
 int64_t expanded_row_bytes(int64_t nbytes) { return round_up(nbytes * 8, 128); }
 
+// Popcounts of n rows, then the smallest of each 32.
+size_t popcount_words(int64_t n) { return size_t(n + (n + 31) / 32); }
+
 // Binary rows on the tensor cores: popcounts and the 0/1 expansion, then the
 // int8 scan in Jaccard mode.  ldb: bytes between staged packed rows.
 int run_jaccard_tc(evoc_gpu_ctx* ctx, const Job& j, int64_t ldb, int64_t nbytes) {
@@ -910,7 +913,7 @@ int run_jaccard_tc(evoc_gpu_ctx* ctx, const Job& j, int64_t ldb, int64_t nbytes)
   const int64_t lde = expanded_row_bytes(nbytes);
   {
     Stage st(ctx, "expand_bits");
-    EVOC_TRY(ctx->popc.ensure(size_t(j.n) * 4), "alloc popcounts");
+    EVOC_TRY(ctx->popc.ensure(popcount_words(j.n) * 4), "alloc popcounts");
     EVOC_TRY(evoc::launch_popcount_rows(ctx->x.p, j.n, int(ldb / 4), ctx->popc.as<int32_t>(), ctx->sms, ctx->stream),
              "popcounts");
     EVOC_TRY(ctx->xb.ensure(size_t(rows * lde)), "alloc expanded rows");
@@ -927,12 +930,15 @@ int run_jaccard_tc(evoc_gpu_ctx* ctx, const Job& j, int64_t ldb, int64_t nbytes)
   Stage st(ctx, "jaccard_scan");
   const int grid = scan_grid(ctx, j.nq);
   EVOC_TRY(ctx->scratch.ensure(size_t(grid) * 256 * size_t(j.keff) * 8), "alloc scratch");
+  int32_t* least = ctx->popc.as<int32_t>() + j.n;
+  EVOC_TRY(evoc::launch_least_popcounts(ctx->popc.as<int32_t>(), j.n, least, ctx->sms, ctx->stream), "popcounts");
   EVOC_TRY(evoc::launch_tc_scan(evoc::kScanJaccard, ctx->xb.p, rows, j.r0, j.nq, ctx->xb.p, rows, j.n, lde, j.keff,
                                 ctx->scratch.as<uint64_t>(), grid, 1, 1, EVOC_DTYPE_U8, j.idx, j.raw, j.dist, j.status,
                                 ctx->timeout_ns, ctx->popc.as<int32_t>(), ctx->stream,
-                                tuned_variant(ctx, evoc::kScanJaccard, j.keff, lde, j.n)),
+                                tuned_variant(ctx, evoc::kScanJaccard, j.keff, lde, j.n), evoc::kHalfF16, nullptr,
+                                nullptr, 0, 0, least),
            "jaccard scan");
-  ctx->launches += 1;
+  ctx->launches += 2;
   return EVOC_OK;
 }
 
@@ -2133,7 +2139,7 @@ void knn_buffer_needs(const evoc_gpu_ctx* ctx, const evoc_gpu_opts& opts, int32_
   } else {
     b[kBufX] = size_t(rows * round_up(dim, 64));
     if (form == EVOC_FORM_EXACT_INT) {
-      b[kBufPopc] = size_t(n) * 4;
+      b[kBufPopc] = popcount_words(n) * 4;
       b[kBufXb] = size_t(rows * expanded_row_bytes(dim));
       b[kBufScratch] = size_t(grid) * 256 * size_t(keff) * 8;
       list_plan(keff, expanded_row_bytes(dim), expanded_row_bytes(dim), round_up(dim, 64));

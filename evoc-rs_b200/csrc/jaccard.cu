@@ -202,6 +202,20 @@ __global__ void expand_bits_kernel(const uint8_t* __restrict__ X, int64_t n, int
   }
 }
 
+__global__ void least_popcounts_kernel(const int32_t* __restrict__ pc, int64_t n, int32_t* __restrict__ least) {
+  for (int64_t g = int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); g * 32 < n;
+       g += int64_t(gridDim.x) * (blockDim.x >> 5)) {
+    const int64_t i = g * 32 + (threadIdx.x & 31);
+    const uint32_t m = __reduce_min_sync(0xffffffffu, i < n ? uint32_t(pc[i]) : 0xffffffffu);
+    if ((threadIdx.x & 31) == 0) least[g] = int32_t(m);
+  }
+}
+
+cudaError_t launch_least_popcounts(const int32_t* pc, int64_t n, int32_t* least, int sms, cudaStream_t stream) {
+  least_popcounts_kernel<<<sms * 4, 256, 0, stream>>>(pc, n, least);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_expand_bits(const void* X, int64_t n, int64_t ld_in, int64_t nbytes, void* Y, int64_t rows,
                                int64_t ld_out, int sms, cudaStream_t stream) {
   if (ld_out % 16 != 0 || ld_out < 8 * nbytes || rows < n || (reinterpret_cast<uintptr_t>(Y) & 15))

@@ -73,7 +73,7 @@ cudaError_t launch_gather_rows_list(const void* src, int64_t row_bytes, int64_t 
 //   bits), Jaccard from the intersection counts and the row popcounts `pc` (self_mode, Q == K).
 //   q_self (optional): key index of query i for the self rule is q_self_base + q_self[i] (default
 //   q_row0 + i), for query rows gathered from elsewhere.  out_bound (optional): per query, the raw
-//   value of the keep-th kept key.
+//   value of the keep-th kept key.  pc_least (optional, mode 2): the smallest popcount of each 32 key rows.
 size_t tc_scan_smem_bytes();
 enum ScanMode { kScanHalf = 0, kScanInt8 = 1, kScanJaccard = 2 };
 cudaError_t launch_tc_scan(int mode, const void* Q, int64_t q_rows, int64_t q_row0, int64_t n_q, const void* K,
@@ -81,7 +81,8 @@ cudaError_t launch_tc_scan(int mode, const void* Q, int64_t q_rows, int64_t q_ro
                            int self_mode, int final_mode, int dtype, int32_t* out_idx, float* out_raw, float* out_dist,
                            int* status, uint64_t timeout_ns, const int32_t* pc, cudaStream_t stream,
                            int variant = -1, int half_type = kHalfF16, const int32_t* q_self = nullptr,
-                           float* out_bound = nullptr, int64_t q_self_base = 0, uint64_t delay_ns = 0);
+                           float* out_bound = nullptr, int64_t q_self_base = 0, uint64_t delay_ns = 0,
+                           const int32_t* pc_least = nullptr);
 // Symmetric scan of all n rows against themselves (16-bit operands, self
 // rule, candidates out).  X holds the rows in a permuted order: scanned row i
 // is data-set row perm[i].  Query block b multiplies only the key tiles from
@@ -296,6 +297,8 @@ namespace evoc {
 cudaError_t launch_scan_counts(const int32_t* cnt, int64_t n, int64_t* out, cudaStream_t stream);
 // jaccard.cu: per-row popcounts of rows of ldw 32-bit words.
 cudaError_t launch_popcount_rows(const void* X, int64_t n, int ldw, int32_t* pc, int sms, cudaStream_t stream);
+// jaccard.cu: the smallest of each 32 popcounts (the last group of what there is).
+cudaError_t launch_least_popcounts(const int32_t* pc, int64_t n, int32_t* least, int sms, cudaStream_t stream);
 // jaccard.cu: packed bit rows (ld_in bytes apart, nbytes used) -> 0/1 int8 rows of ld_out bytes
 // (ld_out >= 8 * nbytes, multiple of 16) for `rows` rows; rows past n and columns past 8*nbytes are 0.
 cudaError_t launch_expand_bits(const void* X, int64_t n, int64_t ld_in, int64_t nbytes, void* Y, int64_t rows,

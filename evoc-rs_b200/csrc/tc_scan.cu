@@ -100,6 +100,7 @@ struct ScanParams {
   uint64_t drain_ns;    // limit of the waits for loads and MMAs already issued (never shorter than 4 s)
   uint64_t delay_ns;    // tests of the timeout path: the producer starts this late (0 in normal use)
   const int32_t* pc; // Jaccard mode: popcount of every row (queries and keys)
+  const int32_t* pc_least;  // optional: the smallest popcount of each 32 key rows
   int half_type;     // 16-bit mode: kHalfF16 or kHalfBf16 operands
   const int32_t* q_self;  // optional: key index of query i is q_self_base + q_self[i] (gathered query rows)
   int64_t q_self_base;
@@ -143,7 +144,9 @@ constexpr int kModeJaccard = 2;  // 0/1 int8 rows: intersection counts, -(inter 
 // 16-bit float operands it is an f32.  For Jaccard it is a lower bound on the intersection:
 // J = inter / (pa + pb - inter) <= inter / pa, so a key reaching the heap's
 // similarity t needs inter >= t * pa (taken 1e-6 looser so f32 rounding of J
-// never rejects a key the exact compare would admit).  Passing scores are
+// never rejects a key the exact compare would admit); with the smallest
+// popcount of a chunk's keys, inter >= t / (1 + t) (pa + pb) is the closer one
+// (chunk_threshold).  Passing scores are
 // re-checked exactly by the key compare.
 // Integer scores are below 2^29 in magnitude (int8 dots for rows of fewer than
 // 33,000 bytes, intersection counts), so the "admit everything" threshold
@@ -169,6 +172,15 @@ __device__ __forceinline__ uint32_t raw_threshold(float raw, int32_t pa) {
     return uint32_t(int32_t(floorf(sim * float(pa) * (1.0f - 1e-6f))));
   }
   return raw < 0.0f ? __float_as_uint(-raw) : open_threshold<MODE>();  // raw = -score, or MIN_POSITIVE for scores <= 0
+}
+
+// Jaccard: the row's threshold for a chunk whose keys have at least `least`
+// bits.  Without it every row of the query's own cluster passes the bound that
+// only knows pa, and is divided and compared to no end: 250,000 x 1,024 bits,
+// whose clusters keep two thirds of their bits, scanned in 97 ms.
+__device__ __forceinline__ uint32_t chunk_threshold(uint32_t thr, float sim, int32_t pa, int32_t least) {
+  const float t = sim / (1.0f + sim) * float(pa + least) * (1.0f - 2e-6f);
+  return sim > 0.0f ? uint32_t(max(int32_t(thr), int32_t(floorf(t)))) : thr;
 }
 
 template <int MODE, class Keys>
@@ -259,11 +271,9 @@ __device__ __forceinline__ int32_t max32_s32(const uint32_t (&v)[32]) {
 
 // Whether any score of the chunk passes: a max tree (independent at each
 // level) and one compare.  Once a row's heap is full most chunks fail here
-// and skip the per-column mask.  Not for Jaccard: its intersection bound is
-// loose enough that the pre-check passes too often to pay for itself.
+// and skip the per-column mask.
 template <int MODE>
 __device__ __forceinline__ bool chunk_any(const uint32_t (&v)[32], uint32_t thr) {
-  if (MODE == kModeJaccard) return true;
   if (MODE != kModeHalf) return max32_s32(v) >= int32_t(thr);
   // 16-bit float scores: against a positive threshold the bit patterns as
   // signed integers order as the floats do (a negative score is a negative
@@ -749,6 +759,11 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         if (ti + 1 < v.n_ktiles - v.kt0) next = tile_at<kSym, kList>(v, ti + 1, p.lists.lg);
         // list mode: the next tile's row indices (1 KB) on their way to L1, where a survivor reads its own
         if (kList && lane < 8) prefetch_l1(perm + min(next * BN + lane * 32, v.n_k - 1));
+        // Jaccard: the smallest popcounts of the tile's chunks, a lane each
+        int32_t least = 0;
+        if (MODE == kModeJaccard && p.pc_least)
+          least = lane < NCH && kt * BN + col_base + lane * 32 < v.n_k
+                      ? p.pc_least[(kt * BN + col_base) / 32 + lane] : 0;
         const uint32_t a = tile & 1u, tph = (tile >> 1) & 1u;
         int got = 1;
         if (lane == 0) got = mbar_wait(&tfull[a], tph, abort, p.timeout_ns) ? 1 : 0;
@@ -786,8 +801,17 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                                 ids, row_seed);
             if (col >= (v.qb + 1) * BM)
               mirror_chunk(vv, mx, um, tth + (col_base + c * 32), ids, col, v.n_k, qd, valid, mst, lane, p);
-          } else if (valid && chunk_any<MODE>(vv, thr)) {
-            offer_chunk<MODE>(vv, chunk_mask<MODE>(vv, thr), col, v.n_k, v.self_mode, qg, heap, thr, pa, v.pc,
+            return;
+          }
+          uint32_t ct = thr;
+          if (MODE == kModeJaccard) {
+            const int32_t bits = __shfl_sync(0xffffffffu, least, c);
+            const uint64_t worst = heap.threshold();
+            const float sim = fmaxf(worst == kKeyInf ? 0.0f : -from_orderable(uint32_t(worst >> 32)), -seed_raw);
+            ct = chunk_threshold(thr, sim, pa, bits);
+          }
+          if (valid && chunk_any<MODE>(vv, ct)) {
+            offer_chunk<MODE>(vv, chunk_mask<MODE>(vv, ct), col, v.n_k, v.self_mode, qg, heap, thr, pa, v.pc,
                               kList ? perm + col : nullptr, row_seed, seed_raw);
           }
         };
@@ -1063,7 +1087,7 @@ cudaError_t launch_tc_scan(int mode, const void* Q, int64_t q_rows, int64_t q_ro
                            int self_mode, int final_mode, int dtype, int32_t* out_idx, float* out_raw, float* out_dist,
                            int* status, uint64_t timeout_ns, const int32_t* pc, cudaStream_t stream,
                            int variant, int half_type, const int32_t* q_self, float* out_bound,
-                           int64_t q_self_base, uint64_t delay_ns) {
+                           int64_t q_self_base, uint64_t delay_ns, const int32_t* pc_least) {
   // q_rows / k_rows: rows present in memory (multiples of the box heights);
   // n_q / n_k: rows that take part.  Rows past n are zero and never offered.
   if (row_bytes % KCB != 0 || n_q <= 0 || n_k <= 0 || keep < 1) return cudaErrorInvalidValue;
@@ -1101,6 +1125,7 @@ cudaError_t launch_tc_scan(int mode, const void* Q, int64_t q_rows, int64_t q_ro
   p.drain_ns = timeout_ns > kDrainNs ? timeout_ns : kDrainNs;
   p.delay_ns = delay_ns;
   p.pc = pc;
+  p.pc_least = pc_least;
   p.half_type = half_type;
   p.q_self = q_self;
   p.q_self_base = q_self_base;
