@@ -101,6 +101,13 @@ int main_scan_grid(const evoc_gpu_ctx* ctx, int64_t n_q, int keep, int variant) 
   return int(std::min<int64_t>((n_q + 127) / 128, int64_t(1) << 30));
 }
 
+// Whether a request's scan takes the small form (small.cu): few enough rows,
+// no tuned variant, no delayed producer (a test's).
+bool use_small(const evoc_gpu_ctx* ctx, int mode, int64_t n, int64_t keep, int variant) {
+  return variant < 0 && ctx->delay_ns == 0 &&
+         evoc::small_scan_feasible(mode, n, int(std::min<int64_t>(keep, 1 << 20)));
+}
+
 // One kNN request: all n rows are keys; query rows r0 .. r0+nq-1 are output rows 0 .. nq-1.
 struct Job {
   int64_t n, r0, nq;
@@ -825,6 +832,15 @@ int run_bf16_rerank(evoc_gpu_ctx* ctx, const evoc_gpu_opts& opts, const Job& j, 
   if (sym) {
     int rc = symmetric_scan(ctx, j, half, ldb, rows, C, cf(CL.bound), cf(CL.hnorm), maxes);
     if (rc) return rc;
+  } else if (!lists && use_small(ctx, evoc::kScanHalf, j.n, C, variant)) {
+    Stage st(ctx, "bf16_scan");
+    EVOC_TRY(ctx->scratch.ensure(evoc::small_scan_bytes(j.nq, j.n)), "alloc scratch");
+    EVOC_TRY(evoc::launch_small_scan(evoc::kScanHalf, ctx->xb.p, rows, j.n, j.r0, j.nq, ldb * 2, int(C), 0, 0,
+                                     ctx->scratch.p, ctx->cand.as<int32_t>(), nullptr, nullptr,
+                                     certify ? cf(CL.bound) : nullptr, j.status, ctx->timeout_ns, nullptr, half,
+                                     ctx->sms, ctx->stream),
+             "small scan");
+    ctx->launches += 2;
   } else if (!lists) {
     Stage st(ctx, "bf16_scan");
     EVOC_TRY(ctx->scratch.ensure(scan_scratch_bytes(ctx, j.nq, C)), "alloc scratch");
@@ -890,6 +906,15 @@ int run_int8(evoc_gpu_ctx* ctx, const Job& j, int64_t ldb) {
   const int variant = tuned_variant(ctx, evoc::kScanInt8, j.keff, ldb, j.n);
   const int grid = main_scan_grid(ctx, j.nq, j.keff, variant);
   const int64_t rows = evoc::padded_rows(j.n);
+  if (use_small(ctx, evoc::kScanInt8, j.n, j.keff, variant)) {
+    EVOC_TRY(ctx->scratch.ensure(evoc::small_scan_bytes(j.nq, j.n)), "alloc scratch");
+    EVOC_TRY(evoc::launch_small_scan(evoc::kScanInt8, ctx->x.p, rows, j.n, j.r0, j.nq, ldb, j.keff, 1, EVOC_DTYPE_I8,
+                                     ctx->scratch.p, j.idx, j.raw, j.dist, nullptr, j.status, ctx->timeout_ns, nullptr,
+                                     evoc::kHalfF16, ctx->sms, ctx->stream),
+             "small scan");
+    ctx->launches += 2;
+    return EVOC_OK;
+  }
   EVOC_TRY(ctx->scratch.ensure(size_t(scan_grid(ctx, j.nq)) * 256 * size_t(j.keff) * 8), "alloc scratch");
   EVOC_TRY(evoc::launch_tc_scan(evoc::kScanInt8, ctx->x.p, rows, j.r0, j.nq, ctx->x.p, rows, j.n, ldb, j.keff,
                                 ctx->scratch.as<uint64_t>(), grid, 1, 1, EVOC_DTYPE_I8, j.idx, j.raw, j.dist, j.status,
@@ -928,6 +953,16 @@ int run_jaccard_tc(evoc_gpu_ctx* ctx, const Job& j, int64_t ldb, int64_t nbytes)
     if (rc || taken) return rc;
   }
   Stage st(ctx, "jaccard_scan");
+  const int variant = tuned_variant(ctx, evoc::kScanJaccard, j.keff, lde, j.n);
+  if (use_small(ctx, evoc::kScanJaccard, j.n, j.keff, variant)) {
+    EVOC_TRY(ctx->scratch.ensure(evoc::small_scan_bytes(j.nq, j.n)), "alloc scratch");
+    EVOC_TRY(evoc::launch_small_scan(evoc::kScanJaccard, ctx->xb.p, rows, j.n, j.r0, j.nq, lde, j.keff, 1,
+                                     EVOC_DTYPE_U8, ctx->scratch.p, j.idx, j.raw, j.dist, nullptr, j.status,
+                                     ctx->timeout_ns, ctx->popc.as<int32_t>(), evoc::kHalfF16, ctx->sms, ctx->stream),
+             "small scan");
+    ctx->launches += 2;
+    return EVOC_OK;
+  }
   const int grid = scan_grid(ctx, j.nq);
   EVOC_TRY(ctx->scratch.ensure(size_t(grid) * 256 * size_t(j.keff) * 8), "alloc scratch");
   int32_t* least = ctx->popc.as<int32_t>() + j.n;
@@ -935,7 +970,7 @@ int run_jaccard_tc(evoc_gpu_ctx* ctx, const Job& j, int64_t ldb, int64_t nbytes)
   EVOC_TRY(evoc::launch_tc_scan(evoc::kScanJaccard, ctx->xb.p, rows, j.r0, j.nq, ctx->xb.p, rows, j.n, lde, j.keff,
                                 ctx->scratch.as<uint64_t>(), grid, 1, 1, EVOC_DTYPE_U8, j.idx, j.raw, j.dist, j.status,
                                 ctx->timeout_ns, ctx->popc.as<int32_t>(), ctx->stream,
-                                tuned_variant(ctx, evoc::kScanJaccard, j.keff, lde, j.n), evoc::kHalfF16, nullptr,
+                                variant, evoc::kHalfF16, nullptr,
                                 nullptr, 0, 0, least),
            "jaccard scan");
   ctx->launches += 2;
@@ -2077,6 +2112,10 @@ void knn_buffer_needs(const evoc_gpu_ctx* ctx, const evoc_gpu_opts& opts, int32_
     b[kBufHist] = size_t(n_piv) * 4;
     b[kBufCursor] = size_t(n_piv) * 4;
   };
+  auto scratch_plan = [&](int mode, int64_t keep) {  // the scan's heaps, or the small form's scores
+    b[kBufScratch] = size_t(grid) * 256 * size_t(keep) * 8;
+    if (use_small(ctx, mode, n, keep, -1)) b[kBufScratch] = std::max(b[kBufScratch], small_scan_bytes(n, n));
+  };
   auto list_plan = [&](int64_t keep, int64_t row_bytes, int64_t elems, int64_t xs_bytes) {
     if (!use_lists(n, 0, n, keep, elems)) return;
     const int64_t piv = list_pivots(n);
@@ -2106,7 +2145,7 @@ void knn_buffer_needs(const evoc_gpu_ctx* ctx, const evoc_gpu_opts& opts, int32_
       const int64_t C = bf16_candidates(opts, n, int(keff));
       b[kBufXb] = size_t(rows * ldb * 2);
       b[kBufCand] = size_t(n * C) * 4;
-      b[kBufScratch] = size_t(grid) * 256 * size_t(C) * 8;
+      scratch_plan(kScanHalf, C);
       if (n >= 65536) locality(ldb * 2);
       if (use_symmetric(ctx, opts.certify != 0, n, 0, n, C)) b[kBufSym] = sym_layout(n, C, ldb).total;
       else list_plan(C, ldb * 2, ldb, ldb * 2);
@@ -2130,7 +2169,7 @@ void knn_buffer_needs(const evoc_gpu_ctx* ctx, const evoc_gpu_opts& opts, int32_
     const int64_t ldb = round_up(dim, 128);
     b[kBufX] = size_t(rows * ldb);
     if (form == EVOC_FORM_EXACT_INT) {
-      b[kBufScratch] = size_t(grid) * 256 * size_t(keff) * 8;
+      scratch_plan(kScanInt8, keff);
       list_plan(keff, ldb, ldb, ldb);
     } else if (form == EVOC_FORM_NNDESCENT) {
       locality(ldb);
@@ -2141,7 +2180,7 @@ void knn_buffer_needs(const evoc_gpu_ctx* ctx, const evoc_gpu_opts& opts, int32_
     if (form == EVOC_FORM_EXACT_INT) {
       b[kBufPopc] = popcount_words(n) * 4;
       b[kBufXb] = size_t(rows * expanded_row_bytes(dim));
-      b[kBufScratch] = size_t(grid) * 256 * size_t(keff) * 8;
+      scratch_plan(kScanJaccard, keff);
       list_plan(keff, expanded_row_bytes(dim), expanded_row_bytes(dim), round_up(dim, 64));
     } else if (form == EVOC_FORM_POPCOUNT) {
       b[kBufPopc] = size_t(n) * 4;

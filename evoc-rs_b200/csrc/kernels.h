@@ -134,12 +134,13 @@ struct PruneStats {
   float *a0, *a1, *rho, *sq0;  // per segment: smallest / largest a_x, largest |x'|, smallest |x|^2
   unsigned int* top;           // largest |x|^2 of all rows (f32 bits)
 };
-// Products of the first `rows` rows of A with all rows of C (a multiple of 256): f32 out[row][ld]; with
+// Products of the first `rows` rows of A with all rows of C (a multiple of 256): f32 out[row][ld] (with
+// bits: int8 products as s32); with
 // seg, per segment of A's rows the column maxima with 0 (f32 / s32 patterns, out cleared by the caller).
 cudaError_t launch_centre_products(int mode, const void* A, int64_t a_rows_mem, int64_t rows, const void* C,
                                    int64_t c_rows_mem, int64_t row_bytes, int half_type, const Segments* seg,
                                    void* out, int64_t ld, int* status, uint64_t timeout_ns, int sms,
-                                   cudaStream_t stream);
+                                   cudaStream_t stream, bool bits = false);
 // A seed per row (scanned order): a dissimilarity that keep other rows near it do not exceed.  top: the
 // largest |x|^2.
 cudaError_t launch_seeds(int mode, const void* X, int64_t rows_mem, int64_t n, int64_t row_bytes, int keep,
@@ -178,6 +179,16 @@ cudaError_t launch_prune_lists(int mode, int64_t n, int64_t group_rows, int grou
                                const int32_t* group_of, int segments, int64_t ld, const int32_t* U, const float* G,
                                const PruneStats& st, const float* T, int half_len, int32_t* list, int32_t* len,
                                int32_t* block_order, cudaStream_t stream);
+
+// small.cu: the scan of query rows q_row0 .. q_row0+n_q-1 of X against its first n rows (self rule) for
+// sets of at most kSmallRows rows: scores holds small_scan_bytes.  Outputs as launch_tc_scan's.
+constexpr int64_t kSmallRows = 5000;
+bool small_scan_feasible(int mode, int64_t n_k, int keep);
+size_t small_scan_bytes(int64_t n_q, int64_t n_k);
+cudaError_t launch_small_scan(int mode, const void* X, int64_t rows_mem, int64_t n, int64_t q_row0, int64_t n_q,
+                              int64_t row_bytes, int keep, int final_mode, int dtype, void* scores, int32_t* out_idx,
+                              float* out_raw, float* out_dist, float* out_bound, int* status, uint64_t timeout_ns,
+                              const int32_t* pc, int half_type, int sms, cudaStream_t stream);
 
 // sym.cu.  Row j of dst = row j * stride of src for j < m, zero rows up to m_pad.
 cudaError_t launch_gather_strided_rows(const void* src, int64_t row_bytes, int64_t stride, int64_t m, int64_t m_pad,

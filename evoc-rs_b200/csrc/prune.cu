@@ -72,10 +72,11 @@ struct ProductParams {
 
 // Rows x centres on the tensor cores (the scan's pipeline: TMA producer warp,
 // MMA warp, four epilogue warps, two accumulators).  kStore writes the
-// products; otherwise each column's maximum over a segment's rows, as the
+// products (kBits: as the accumulator holds them, s32 for int8); otherwise
+// each column's maximum over a segment's rows, as the
 // signed pattern of a non-negative f32 or s32.  At 1M x 768 against 3,907
 // centres: 6 TFLOP.
-template <bool kInt8, bool kStore>
+template <bool kInt8, bool kStore, bool kBits = false>
 __global__ void __launch_bounds__(192, 1)
 centre_product_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                       const ProductParams p) {
@@ -206,7 +207,7 @@ centre_product_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
               float f[4];
 #pragma unroll
               for (int u = 0; u < 4; u++)
-                f[u] = kInt8 ? __int2float_rn(int32_t(v[4 * j + u])) : __uint_as_float(v[4 * j + u]);
+                f[u] = kInt8 && !kBits ? __int2float_rn(int32_t(v[4 * j + u])) : __uint_as_float(v[4 * j + u]);
               o[j] = make_float4(f[0], f[1], f[2], f[3]);
             }
           }
@@ -911,7 +912,7 @@ block_order_kernel(const int32_t* __restrict__ len, int groups, int64_t n_blocks
 cudaError_t launch_centre_products(int mode, const void* A, int64_t a_rows_mem, int64_t rows, const void* C,
                                    int64_t c_rows_mem, int64_t row_bytes, int half_type, const Segments* seg,
                                    void* out, int64_t ld, int* status, uint64_t timeout_ns, int sms,
-                                   cudaStream_t stream) {
+                                   cudaStream_t stream, bool bits) {
   if (row_bytes % KCB || rows < 1 || a_rows_mem < rows || c_rows_mem % BN || ld < c_rows_mem || ld % 4)
     return cudaErrorInvalidValue;
   const bool store = seg == nullptr;
@@ -940,6 +941,7 @@ cudaError_t launch_centre_products(int mode, const void* A, int64_t a_rows_mem, 
     return cudaGetLastError();
   };
   if (mode == kScanHalf) return store ? go(centre_product_kernel<false, true>) : go(centre_product_kernel<false, false>);
+  if (store && bits) return go(centre_product_kernel<true, true, true>);
   return store ? go(centre_product_kernel<true, true>) : go(centre_product_kernel<true, false>);
 }
 
