@@ -994,7 +994,7 @@ int run_jaccard(evoc_gpu_ctx* ctx, const Job& j, int64_t ldb) {
 int fuzzy_work(evoc_gpu_ctx* ctx, int64_t n, int k, evoc::FuzzyWork* w) {
   const size_t nk = size_t(n) * size_t(k);
   const size_t sizes[] = {64, 64, nk * 4, nk * 4, size_t(n) * 4, size_t(n) * 4, size_t(n + 1) * 8, size_t(n) * 4,
-                          nk * 4, nk * 4, size_t(n) * 4, size_t(n) * 4, 64};
+                          nk * 8, size_t(n) * 4, size_t(n) * 4, 64};
   constexpr int kParts = int(sizeof(sizes) / sizeof(sizes[0]));
   size_t total = 0;
   for (size_t s : sizes) total += (s + 255) / 256 * 256;
@@ -1013,11 +1013,10 @@ int fuzzy_work(evoc_gpu_ctx* ctx, int64_t n, int k, evoc::FuzzyWork* w) {
   w->indeg = static_cast<int32_t*>(ptrs[5]);
   w->colptr = static_cast<int64_t*>(ptrs[6]);
   w->fill = static_cast<int32_t*>(ptrs[7]);
-  w->at_rows = static_cast<int32_t*>(ptrs[8]);
-  w->at_vals = static_cast<float*>(ptrs[9]);
-  w->row_cnt = static_cast<int32_t*>(ptrs[10]);
-  w->big = static_cast<int32_t*>(ptrs[11]);
-  w->n_big = static_cast<int32_t*>(ptrs[12]);
+  w->at = static_cast<uint64_t*>(ptrs[8]);
+  w->row_cnt = static_cast<int32_t*>(ptrs[9]);
+  w->big = static_cast<int32_t*>(ptrs[10]);
+  w->n_big = static_cast<int32_t*>(ptrs[11]);
   return EVOC_OK;
 }
 
@@ -1085,7 +1084,7 @@ int fuzzy_impl(evoc_gpu_ctx* ctx, const int32_t* idx, const float* dist, int64_t
     {
       Stage st(ctx, "union_count");
       EVOC_TRY(evoc::launch_fuzzy_union_count(n, k, symmetrize, w, d_indptr, ctx->sms, ctx->stream), "union count");
-      ctx->launches += symmetrize ? 5 : 2;
+      ctx->launches += symmetrize ? 9 : 3;
     }
     EVOC_TRY(cudaMemcpyAsync(&total_nnz, d_indptr + n, 8, cudaMemcpyDeviceToHost, ctx->stream), "read nnz");
     EVOC_TRY(cudaStreamSynchronize(ctx->stream), "union count");

@@ -289,8 +289,7 @@ struct FuzzyWork {
   int32_t* indeg;     // n: entries per column of A
   int64_t* colptr;    // n + 1: CSR pointer of A^T
   int32_t* fill;      // n
-  int32_t* at_rows;   // n x k capacity: A^T row indices per column bucket
-  float* at_vals;
+  uint64_t* at;       // n x k capacity: A^T per column bucket, row << 32 | value bits
   int32_t* row_cnt;   // n: entries per row of the result
   int32_t* big;       // n: column buckets too large for a warp's sort
   int32_t* n_big;     // 1: their count
