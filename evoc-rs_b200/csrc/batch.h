@@ -21,7 +21,7 @@ struct BatchHeader {
   int32_t status;        // 0 ok; the scan / rerank status codes of any request
   int32_t fail_count;    // f32 requests: rows that failed the certificate
   int64_t total_rows;    // sum of n over the requests (rerank rows)
-  int64_t total_blocks;  // sum of ceil(n / 128) (row-norm blocks)
+  int64_t total_blocks;  // sum of rows / 32 (tiles of the row preparation)
   int32_t* fail_list;    // (request, row) pairs of those rows
   int64_t fail_cap;      // pairs the list holds
 };
@@ -33,7 +33,7 @@ struct BatchRowJob {
   int64_t ld;              // f32 stride in floats (f32 requests)
   int64_t ldb;             // 16-bit / int8 stride in bytes
   int64_t row_base;        // first global row of this request (prefix of n)
-  int64_t blk_base;        // first global 128-row block (prefix of ceil(n/128))
+  int64_t blk_base;        // first global 32-row tile (prefix of rows / 32)
   const uint8_t* src;      // packed input rows on the device
   float* x;                // f32 padded rows (f32 requests)
   uint8_t* xb;             // 16-bit or int8 padded rows
@@ -89,7 +89,7 @@ cudaError_t launch_tc_scan_batch(int mode, BatchHeader* hdr, const ScanJob* jobs
 // Grids are sized by the caller for the batch (grid-stride loops cover any
 // count), so a small batch occupies a few SMs and runs beside other work.
 cudaError_t launch_batch_rows(bool f32, const BatchHeader* hdr, const BatchRowJob* jobs, int grid_rows,
-                              int grid_norms, cudaStream_t stream);
+                              int grid_tiles, cudaStream_t stream);
 // rerank.cu.  f32 requests: FP32 rerank of the scan candidates into the
 // outputs; rows that fail the certificate go to the header's list.
 cudaError_t launch_batch_rerank(BatchHeader* hdr, const BatchRowJob* jobs, int grid, cudaStream_t stream);

@@ -494,7 +494,7 @@ CertLayout cert_layout(int64_t n, int64_t nq) {
   };
   L.rnorm = take(size_t(n) * 4);
   L.hnorm = take(size_t(n) * 4);
-  L.maxes = take(8);
+  L.maxes = take(evoc::kPrepMaxes * 4);
   L.bound = take(size_t(nq) * 4);
   L.bound2 = take(size_t(kRepairChunk) * 4);
   L.counts = take(8);
@@ -786,6 +786,51 @@ int symmetric_scan(evoc_gpu_ctx* ctx, const Job& j, int half, int64_t ldb, int64
   return EVOC_OK;
 }
 
+// The f32 rows a form works on: padded, divided by their norms if some norm is
+// off, and for the forms that scan 16-bit rows those too.  Rows on the device
+// are read where they lie; host rows, and rows off the 4-byte grid, are copied
+// into place first.
+int prepare_f32(evoc_gpu_ctx* ctx, const void* data, int64_t n, int64_t dim, int ld, int64_t nq, int keff, int form,
+                const evoc_gpu_opts& opts, bool on_dev) {
+  evoc::PrepRows p{};
+  p.n = n;
+  p.rows = evoc::padded_rows(n);
+  p.d = dim;
+  p.ld = ld;
+  const bool in_place = !on_dev || (reinterpret_cast<uintptr_t>(data) & 3) != 0;
+  if (in_place) {
+    const int rc = stage_rows(ctx, data, n, dim * 4, p.ld * 4, on_dev);
+    if (rc) return rc;
+  }
+  Stage st(ctx, "prepare_rows");
+  EVOC_TRY(ctx->x.ensure(size_t(p.rows * p.ld) * 4), "alloc rows");
+  EVOC_TRY(ctx->norms.ensure(size_t(n) * 4), "alloc norms");
+  p.x = ctx->x.as<float>();
+  p.src = in_place ? p.x : static_cast<const float*>(data);
+  p.src_ld = in_place ? p.ld : dim;
+  p.norms = ctx->norms.as<float>();
+  p.not_unit = ctx->flag.as<int>();
+  const bool rerank = form == EVOC_FORM_BF16_RERANK && bf16_candidates(opts, n, keff) <= 256 &&
+                      (opts.scan_type == evoc::kHalfF16 || opts.scan_type == evoc::kHalfBf16);
+  if (rerank || form == EVOC_FORM_NNDESCENT) {
+    p.ldb = round_up(dim, 64);
+    EVOC_TRY(ctx->xb.ensure(size_t(p.rows * p.ldb * 2)), "alloc 16-bit rows");
+    p.half = ctx->xb.as<uint16_t>();
+    p.half_type = rerank ? opts.scan_type : int(evoc::kHalfF16);
+  }
+  if (rerank && opts.certify) {
+    const CertLayout CL = cert_layout(n, nq);
+    EVOC_TRY(ctx->cert.ensure(CL.total), "alloc certificate");
+    uint8_t* cb = ctx->cert.as<uint8_t>();
+    p.rnorm = reinterpret_cast<float*>(cb + CL.rnorm);
+    p.hnorm = reinterpret_cast<float*>(cb + CL.hnorm);
+    p.maxes = reinterpret_cast<unsigned int*>(cb + CL.maxes);
+  }
+  EVOC_TRY(evoc::launch_prepare_rows(p, ctx->sms, ctx->stream), "prepare rows");
+  ctx->launches += 2;
+  return EVOC_OK;
+}
+
 // The 16-bit form: FP16 (or BF16) tensor-core scan keeping C candidates per
 // row, FP32 rerank with the per-row certificate (rerank.cu), then for rows
 // that fail it a second scan keeping 256 candidates, and for rows that fail
@@ -810,15 +855,6 @@ int run_bf16_rerank(evoc_gpu_ctx* ctx, const evoc_gpu_opts& opts, const Job& j, 
   auto cf = [&](size_t off) { return reinterpret_cast<float*>(cb + off); };
   auto ci = [&](size_t off) { return reinterpret_cast<int32_t*>(cb + off); };
   unsigned int* maxes = certify ? reinterpret_cast<unsigned int*>(cb + CL.maxes) : nullptr;
-  {
-    Stage st(ctx, "to_half");
-    EVOC_TRY(ctx->xb.ensure(size_t(rows * ldb * 2)), "alloc 16-bit rows");
-    EVOC_TRY(evoc::launch_to_half(ctx->x.as<float>(), rows, j.n, ld, d, ctx->xb.p, int(ldb), half,
-                                  certify ? cf(CL.rnorm) : nullptr, certify ? cf(CL.hnorm) : nullptr, maxes, ctx->sms,
-                                  ctx->stream),
-             "to 16-bit");
-    ctx->launches += 1;
-  }
   const int variant = tuned_variant(ctx, evoc::kScanHalf, int(C), ldb * 2, j.n);
   const int grid = main_scan_grid(ctx, j.nq, int(C), variant);
   EVOC_TRY(ctx->cand.ensure(size_t(j.nq * C) * 4), "alloc candidates");
@@ -1340,30 +1376,13 @@ int knn_impl(evoc_gpu_ctx* ctx, const evoc_gpu_opts* opts_in, int32_t dtype, con
     if (form != EVOC_FORM_FP32 && form != EVOC_FORM_BF16_RERANK && form != EVOC_FORM_NNDESCENT)
       return fail(ctx, EVOC_ERR_UNSUPPORTED, "form not built for f32 in this library");
     const int ld = int(round_up(dim, 16));
-    rc = stage_rows(ctx, data, n, dim * 4, int64_t(ld) * 4, on_dev);
+    rc = prepare_f32(ctx, data, n, dim, ld, nq, keff, form, opts, on_dev);
     if (rc) return rc;
-    {
-      Stage st(ctx, "prepare_float");
-      EVOC_TRY(ctx->norms.ensure(size_t(n) * 4), "alloc norms");
-      EVOC_TRY(evoc::launch_prepare_float(ctx->x.as<float>(), n, ld, int(dim), ctx->norms.as<float>(), d_flags,
-                                          ctx->sms, ctx->stream),
-               "prepare_float");
-      ctx->launches += 2;
-    }
     if (form == EVOC_FORM_FP32) rc = run_fp32(ctx, job, ld);
     else if (form == EVOC_FORM_BF16_RERANK) rc = run_bf16_rerank(ctx, opts, job, ld, int(dim));
     else {
       // The pivot cells come from the FP16 tensor-core scan; the join reads the f32 rows.
       const int64_t ldb = round_up(dim, 64);
-      const int64_t rows = evoc::padded_rows(n);
-      {
-        Stage st(ctx, "to_half");
-        EVOC_TRY(ctx->xb.ensure(size_t(rows * ldb * 2)), "alloc 16-bit rows");
-        EVOC_TRY(evoc::launch_to_half(ctx->x.as<float>(), rows, n, ld, int(dim), ctx->xb.p, int(ldb), evoc::kHalfF16,
-                                      nullptr, nullptr, nullptr, ctx->sms, ctx->stream),
-                 "to 16-bit");
-        ctx->launches += 1;
-      }
       rc = run_nndescent(ctx, opts, job, EVOC_DTYPE_F32, ldb * 2, ctx->xb.p, ld, int(dim), rng_state);
     }
   } else if (dtype == EVOC_DTYPE_I8) {
@@ -1486,7 +1505,7 @@ int batch_layout(bool f32, const evoc_gpu_opts& opts, int32_t n_jobs, const int6
     L->max_keep = std::max(L->max_keep, J.keep);
     L->n_items += (J.n + 127) / 128;
     L->total_rows += J.n;
-    L->total_blocks += (J.n + 127) / 128;
+    L->total_blocks += J.rows / 32;
   }
   if (f32 && opts.certify) {
     L->off_fail = ws;
@@ -1582,7 +1601,7 @@ int knn_batch_impl(evoc_gpu_ctx* ctx, const evoc_gpu_opts* opts_in, int32_t dtyp
     R.row_base = row_base;
     R.blk_base = blk_base;
     row_base += J.n;
-    blk_base += (J.n + 127) / 128;
+    blk_base += J.rows / 32;
     R.src = static_cast<const uint8_t*>(data[i]);
     R.x = f32 ? reinterpret_cast<float*>(W + J.off_x) : nullptr;
     R.xb = W + J.off_xb;
@@ -1657,7 +1676,7 @@ int knn_batch_impl(evoc_gpu_ctx* ctx, const evoc_gpu_opts* opts_in, int32_t dtyp
     if (e == cudaSuccess && f32) e = evoc::launch_batch_rerank(d_hdr, d_rj, grids[3], st);
     return e;
   };
-  ctx->launches += f32 ? 6 : 2;
+  ctx->launches += f32 ? 5 : 2;
   if (ctx->use_graphs && !ctx->sync_check) {
     // Drop graphs captured over an older table buffer.
     for (size_t g = 0; g < ctx->batch_graphs.size();) {

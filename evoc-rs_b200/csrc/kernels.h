@@ -7,8 +7,24 @@
 namespace evoc {
 
 // prep.cu
-cudaError_t launch_prepare_float(float* X, int64_t n, int ld, int d, float* norms, int* not_unit, int sms,
-                                 cudaStream_t stream);
+// prep.cu: f32 rows as the search wants them.
+struct PrepRows {
+  const float* src;  // n rows of d floats, src_ld apart; may be x itself (rows past n zero then)
+  int64_t src_ld;
+  float* x;          // rows x ld floats, zero padded
+  int64_t n, rows;   // rows: a multiple of 32
+  int64_t d, ld;
+  float* norms;      // n
+  int* not_unit;     // some norm is off by more than 1e-5 (zero before); the rows are divided then
+  uint16_t* half;    // null, or rows x ldb 16-bit elements, zero padded (FP16: values below 2^-14 are zero)
+  int64_t ldb;
+  int half_type;
+  float* rnorm;      // null, or each row's |x - half(x)| and |half(x)| rounded up, and kPrepMaxes words, of
+  float* hnorm;      // which the first two come out as their maxima (f32 bit patterns)
+  unsigned int* maxes;
+};
+constexpr int kPrepMaxes = 5;
+cudaError_t launch_prepare_rows(const PrepRows& p, int sms, cudaStream_t stream);
 
 // exact_f32.cu: plain FP32 exact search with fused top-k.
 //   Queries q_begin .. q_end-1 of X against the n rows of X, query q written to output row
@@ -54,12 +70,6 @@ namespace evoc {
 // 16-bit operand type of the f32 tensor-core scan (evoc_gpu_opts.scan_type).
 enum HalfType { kHalfF16 = 0, kHalfBf16 = 1 };
 
-// prep.cu: f32 rows (ld) -> zero-padded 16-bit rows (ldb elements) for rows
-// 0 .. n_rows-1 (rows n .. n_rows-1 zero).  FP16 flushes values below 2^-14
-// to zero.  With rnorm/hnorm (n each) and maxes (2 words): each row's
-// |x - half(x)| and |half(x)| rounded up, and their maxima as f32 bit patterns.
-cudaError_t launch_to_half(const float* X, int64_t n_rows, int64_t n, int ld, int d, void* Y, int ldb, int half_type,
-                           float* rnorm, float* hnorm, unsigned int* maxes, int sms, cudaStream_t stream);
 // prep.cu: dst row i = src row row0 + list[i] (i < count), zero rows up to rows_out.
 cudaError_t launch_gather_rows_list(const void* src, int64_t row_bytes, int64_t row0, const int32_t* list,
                                     int64_t count, int64_t rows_out, void* dst, int sms, cudaStream_t stream);

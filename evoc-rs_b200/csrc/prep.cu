@@ -4,84 +4,26 @@
 // more than 1e-5, every row is divided by its norm (a zero norm divides by 1).
 // The norm is the serial f32 sum of squares followed by sqrt, exactly as the
 // reference rounds it: each product and each partial sum is rounded on its
-// own (no FMA contraction), sqrt and division are IEEE.  One thread owns one
-// row; rows are staged through shared memory in 32-column slabs so the
-// global reads stay coalesced.
+// own (no FMA contraction), sqrt and division are IEEE.
+//
+// One pass reads the caller's rows and writes everything the search wants of
+// them: the padded f32 rows, the norms, the 16-bit rows and their certificate
+// norms, taking the rows as they are.  Only if a norm is off does a second
+// pass divide the rows and write the 16-bit ones again.  Bound by memory
+// (rows read once, written once and a half).  A block takes 32 rows in slabs
+// of 128 columns, a warp four rows of a slab; one warp then adds up the
+// squares, a thread per row, from the slab in shared memory, while the others
+// load the next slab into the other half.  Device to device: 2,000 x 768 rows
+// 26 us, 20,000 x 384 48, 1,000,000 x 768 2,100 (copy, norms, division and
+// 16-bit rows as a pass each, with 128 rows to a block: 191, 161 and 5,800).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+
+#include <algorithm>
 
 #include "batch.h"
 #include "common.cuh"
 #include "kernels.h"
-
-namespace evoc {
-
-namespace {
-constexpr int kRows = 128;
-constexpr int kSlab = 32;
-}
-
-// Norms of rows r0 .. r0+127 (one thread per row, serial f32 sum of squares).
-__device__ __forceinline__ void row_norms_block(const float* __restrict__ X, int64_t n, int ld, int d,
-                                                float* __restrict__ norms, int* __restrict__ not_unit, int64_t r0,
-                                                float (*slab)[kSlab + 1]) {
-  const int tid = threadIdx.x;
-  float acc = 0.0f;
-  for (int c0 = 0; c0 < d; c0 += kSlab) {
-    // cooperative coalesced load: 128 rows x 32 columns
-    for (int e = tid; e < kRows * kSlab; e += kRows) {
-      const int r = e / kSlab, c = e % kSlab;
-      const int64_t g = r0 + r;
-      slab[r][c] = (g < n && c0 + c < d) ? X[g * ld + c0 + c] : 0.0f;
-    }
-    __syncthreads();
-    const int lim = min(kSlab, d - c0);
-    for (int c = 0; c < lim; c++) {
-      const float v = slab[tid][c];
-      acc = __fadd_rn(acc, __fmul_rn(v, v));
-    }
-    __syncthreads();
-  }
-  const int64_t row = r0 + tid;
-  if (row < n) {
-    const float nrm = __fsqrt_rn(acc);
-    norms[row] = nrm;
-    if (fabsf(__fsub_rn(nrm, 1.0f)) > 1e-5f) atomicOr(not_unit, 1);
-  }
-}
-
-__global__ void __launch_bounds__(kRows)
-row_norms_kernel(const float* __restrict__ X, int64_t n, int ld, int d, float* __restrict__ norms,
-                 int* __restrict__ not_unit) {
-  __shared__ float slab[kRows][kSlab + 1];
-  row_norms_block(X, n, ld, d, norms, not_unit, int64_t(blockIdx.x) * kRows, slab);
-}
-
-__global__ void normalize_rows_kernel(float* __restrict__ X, int64_t n, int ld, int d,
-                                      const float* __restrict__ norms, const int* __restrict__ not_unit) {
-  if (*not_unit == 0) return;
-  const int64_t total = n * int64_t(d);
-  for (int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < total; e += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t r = e / d, c = e % d;
-    float nrm = norms[r];
-    if (nrm == 0.0f) nrm = 1.0f;
-    X[r * ld + c] = __fdiv_rn(X[r * ld + c], nrm);
-  }
-}
-
-cudaError_t launch_prepare_float(float* X, int64_t n, int ld, int d, float* norms, int* not_unit, int sms,
-                                 cudaStream_t stream) {
-  cudaError_t e = cudaMemsetAsync(not_unit, 0, sizeof(int), stream);
-  if (e != cudaSuccess) return e;
-  const int64_t blocks = (n + kRows - 1) / kRows;
-  row_norms_kernel<<<unsigned(blocks), kRows, 0, stream>>>(X, n, ld, d, norms, not_unit);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  normalize_rows_kernel<<<sms * 8, 256, 0, stream>>>(X, n, ld, d, norms, not_unit);
-  return cudaGetLastError();
-}
-
-}  // namespace evoc
 
 namespace evoc {
 
@@ -100,55 +42,145 @@ __device__ __forceinline__ float half_value(uint16_t b, int half_type) {
   return half_type == kHalfBf16 ? __bfloat162float(__ushort_as_bfloat16(b)) : __half2float(__ushort_as_half(b));
 }
 
-// f32 rows (ld floats) -> 16-bit rows (ldb elements, zero padded).  Warp per
-// row.  With `cert`, also the two norms the BF16/FP16 form certifies its rows
-// with: |x - half(x)| (the residual, exact in f32) and |half(x)|, summed in
-// f64 and rounded up to f32, and their maxima over all rows (non-negative
-// floats compare as their bit patterns).
-__global__ void to_half_kernel(const float* __restrict__ X, int64_t n_rows, int64_t n, int ld, int d,
-                               uint16_t* __restrict__ Y, int ldb, int half_type, float* __restrict__ rnorm,
-                               float* __restrict__ hnorm, unsigned int* __restrict__ maxes) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warps = int64_t(gridDim.x) * (blockDim.x >> 5);
-  for (int64_t r = int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); r < n_rows; r += warps) {
-    double rr = 0.0, hh = 0.0;
-    for (int c = lane; c < ldb; c += 32) {
-      const float v = (c < d && r < n) ? X[r * ld + c] : 0.0f;
-      const uint16_t b = half_bits(v, half_type);
-      Y[r * ldb + c] = b;
-      const float h = half_value(b, half_type);
-      const double res = double(v) - double(h);
-      rr += res * res;
-      hh += double(h) * double(h);
-    }
-    if (rnorm && r < n) {
+namespace {
+constexpr int kTileRows = 32;
+constexpr int kTileCols = 128;
+constexpr int kPrepWarps = 8;
+constexpr int kWarpRows = kTileRows / kPrepWarps;
+}  // namespace
+
+// One value's share of the two norms the BF16/FP16 form certifies its rows
+// with: |x - half(x)| (the residual, exact in f32) and |half(x)|, summed in f64.
+__device__ __forceinline__ uint16_t half_and_norms(float v, int half_type, double& rr, double& hh) {
+  const uint16_t b = half_bits(v, half_type);
+  const float h = half_value(b, half_type);
+  const double res = double(__fsub_rn(v, h));  // exact
+  rr += res * res;
+  hh += double(h) * double(h);
+  return b;
+}
+
+// A row's sums over its warp, rounded up to f32; their maxima over all rows
+// (non-negative floats compare as their bit patterns).
+__device__ __forceinline__ void write_cert_norms(double rr, double hh, int lane, float* rnorm, float* hnorm,
+                                                 unsigned int* maxes) {
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        rr += __shfl_xor_sync(0xffffffffu, rr, o);
-        hh += __shfl_xor_sync(0xffffffffu, hh, o);
-      }
-      if (lane == 0) {
-        // f64 sums of at most 2^16 squares are within a relative 2^-36 of
-        // exact: one part in 2^-30 more before rounding up covers them.
-        const float a = __double2float_ru(__dsqrt_ru(rr * (1.0 + 0x1p-30)));
-        const float b = __double2float_ru(__dsqrt_ru(hh * (1.0 + 0x1p-30)));
-        rnorm[r] = a;
-        hnorm[r] = b;
-        atomicMax(&maxes[0], __float_as_uint(a));
-        atomicMax(&maxes[1], __float_as_uint(b));
-      }
-    }
+  for (int o = 16; o > 0; o >>= 1) {
+    rr += __shfl_xor_sync(0xffffffffu, rr, o);
+    hh += __shfl_xor_sync(0xffffffffu, hh, o);
+  }
+  if (lane == 0) {
+    // f64 sums of at most 2^16 squares are within a relative 2^-36 of
+    // exact: one part in 2^-30 more before rounding up covers them.
+    const float a = __double2float_ru(__dsqrt_ru(rr * (1.0 + 0x1p-30)));
+    const float b = __double2float_ru(__dsqrt_ru(hh * (1.0 + 0x1p-30)));
+    *rnorm = a;
+    *hnorm = b;
+    // one address for all rows: only those that raise the maximum take the atomic
+    volatile unsigned int* seen = maxes;
+    if (__float_as_uint(a) > seen[0]) atomicMax(&maxes[0], __float_as_uint(a));
+    if (__float_as_uint(b) > seen[1]) atomicMax(&maxes[1], __float_as_uint(b));
   }
 }
 
-cudaError_t launch_to_half(const float* X, int64_t n_rows, int64_t n, int ld, int d, void* Y, int ldb, int half_type,
-                           float* rnorm, float* hnorm, unsigned int* maxes, int sms, cudaStream_t stream) {
-  if (rnorm) {
-    cudaError_t e = cudaMemsetAsync(maxes, 0, 2 * sizeof(unsigned int), stream);
+// Rows r0 .. r0+31 of one matrix, as they are.
+__device__ __forceinline__ void prepare_tile(const PrepRows& p, int64_t r0, float (*slab)[kTileRows][kTileCols + 1]) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t row0 = r0 + warp * kWarpRows;
+  const int64_t width = p.half ? max(p.ld, p.ldb) : p.ld;
+  double rr[kWarpRows] = {}, hh[kWarpRows] = {};
+  float acc = 0.0f;
+  int s = 0;
+  for (int64_t c0 = 0; c0 < width; c0 += kTileCols, s ^= 1) {
+    float v[kWarpRows][kTileCols / 32];
+#pragma unroll
+    for (int a = 0; a < kWarpRows; a++)
+#pragma unroll
+      for (int b = 0; b < kTileCols / 32; b++) {
+        const int64_t c = c0 + 32 * b + lane;
+        v[a][b] = row0 + a < p.n && c < p.d ? p.src[(row0 + a) * p.src_ld + c] : 0.0f;
+      }
+#pragma unroll
+    for (int a = 0; a < kWarpRows; a++)
+#pragma unroll
+      for (int b = 0; b < kTileCols / 32; b++) {
+        const int64_t r = row0 + a, c = c0 + 32 * b + lane;
+        slab[s][warp * kWarpRows + a][32 * b + lane] = v[a][b];
+        if (p.src != p.x && c < p.ld) p.x[r * p.ld + c] = v[a][b];
+        if (p.half && c < p.ldb) p.half[r * p.ldb + c] = half_and_norms(v[a][b], p.half_type, rr[a], hh[a]);
+      }
+    __syncthreads();  // this slab is full, and the sums over the one before it are done
+    if (warp == 0) {
+      const int lim = int(min(int64_t(kTileCols), p.d - c0));
+#pragma unroll 8
+      for (int c = 0; c < lim; c++) {
+        const float x = slab[s][lane][c];
+        acc = __fadd_rn(acc, __fmul_rn(x, x));
+      }
+    }
+  }
+  if (warp == 0) {
+    const bool real = r0 + lane < p.n;
+    const float nrm = __fsqrt_rn(acc);
+    if (real) p.norms[r0 + lane] = nrm;
+    if (__any_sync(0xffffffffu, real && fabsf(__fsub_rn(nrm, 1.0f)) > 1e-5f) && lane == 0) atomicOr(p.not_unit, 1);
+  }
+  if (p.rnorm) {
+#pragma unroll
+    for (int a = 0; a < kWarpRows; a++)
+      if (row0 + a < p.n) write_cert_norms(rr[a], hh[a], lane, p.rnorm + row0 + a, p.hnorm + row0 + a, p.maxes);
+  }
+}
+
+// A warp per row: the row divided by its norm, and its 16-bit row again.  The
+// maxima gather beside those of the undivided rows, and the last block of
+// the grid puts them in their place.
+__device__ __forceinline__ void renormalize_rows(const PrepRows& p) {
+  const int lane = threadIdx.x & 31;
+  const int64_t warps = int64_t(gridDim.x) * (blockDim.x >> 5);
+  for (int64_t r = int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); r < p.n; r += warps) {
+    float nrm = p.norms[r];
+    if (nrm == 0.0f) nrm = 1.0f;
+    double rr = 0.0, hh = 0.0;
+    for (int64_t c = lane; c < p.d; c += 32) {
+      const float v = __fdiv_rn(p.x[r * p.ld + c], nrm);
+      p.x[r * p.ld + c] = v;
+      if (p.half) p.half[r * p.ldb + c] = half_and_norms(v, p.half_type, rr, hh);
+    }
+    if (p.rnorm) write_cert_norms(rr, hh, lane, p.rnorm + r, p.hnorm + r, p.maxes + 2);
+  }
+  if (!p.rnorm) return;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0 && atomicAdd(&p.maxes[4], 1u) == gridDim.x - 1) {
+    p.maxes[0] = atomicMax(&p.maxes[2], 0u);
+    p.maxes[1] = atomicMax(&p.maxes[3], 0u);
+  }
+}
+
+__global__ void __launch_bounds__(kPrepWarps * 32) prepare_rows_kernel(PrepRows p) {
+  __shared__ float slab[2][kTileRows][kTileCols + 1];
+  for (int64_t r0 = int64_t(blockIdx.x) * kTileRows; r0 < p.rows; r0 += int64_t(gridDim.x) * kTileRows) {
+    prepare_tile(p, r0, slab);
+    __syncthreads();
+  }
+}
+
+__global__ void renormalize_rows_kernel(PrepRows p) {
+  if (*p.not_unit != 0) renormalize_rows(p);
+}
+
+cudaError_t launch_prepare_rows(const PrepRows& p, int sms, cudaStream_t stream) {
+  if (p.rows % kTileRows != 0 || p.rows < p.n || p.src_ld < p.d || p.ld < p.d || (p.half && p.ldb < p.d) ||
+      (reinterpret_cast<uintptr_t>(p.src) & 3))
+    return cudaErrorInvalidValue;
+  if (p.rnorm) {
+    cudaError_t e = cudaMemsetAsync(p.maxes, 0, kPrepMaxes * sizeof(unsigned int), stream);
     if (e != cudaSuccess) return e;
   }
-  to_half_kernel<<<sms * 8, 256, 0, stream>>>(X, n_rows, n, ld, d, static_cast<uint16_t*>(Y), ldb, half_type, rnorm,
-                                               hnorm, maxes);
+  prepare_rows_kernel<<<unsigned(std::min<int64_t>(p.rows / kTileRows, int64_t(sms) * 6)), kPrepWarps * 32, 0,
+                        stream>>>(p);
+  renormalize_rows_kernel<<<sms * 8, 256, 0, stream>>>(p);
   return cudaGetLastError();
 }
 
@@ -229,125 +261,86 @@ __device__ __forceinline__ int find_block_job(const BatchRowJob* __restrict__ jo
 }
 }  // namespace
 
-// Packed input rows -> padded rows (f32: x, ld floats; i8: xb, ldb bytes),
-// zero-filled past the data; also clears each request's prepare_float flag.
-__global__ void batch_copy_kernel(const BatchHeader* __restrict__ hdr, const BatchRowJob* __restrict__ jobs,
-                                  bool f32) {
+// Packed int8 rows -> padded rows (xb, ldb bytes), zero-filled past the data.
+__global__ void batch_copy_kernel(const BatchHeader* __restrict__ hdr, const BatchRowJob* __restrict__ jobs) {
   const int nj = hdr->n_jobs;
   for (int j = 0; j < nj; j++) {
     const BatchRowJob& J = jobs[j];
-    if (blockIdx.x == 0 && threadIdx.x == 0 && J.flag) *J.flag = 0;
-    if (blockIdx.x == 0 && threadIdx.x == 0 && J.maxes) J.maxes[0] = J.maxes[1] = 0u;
-    uint8_t* dst = f32 ? reinterpret_cast<uint8_t*>(J.x) : J.xb;
-    const int64_t ld_bytes = f32 ? J.ld * 4 : J.ldb;
     if (J.row_bytes % 4 == 0) {
-      const int64_t wpr = ld_bytes / 4, src_w = J.row_bytes / 4, total = J.rows * wpr;
+      const int64_t wpr = J.ldb / 4, src_w = J.row_bytes / 4, total = J.rows * wpr;
       for (int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < total;
            e += int64_t(gridDim.x) * blockDim.x) {
         const int64_t r = e / wpr, c = e % wpr;
         uint32_t v = 0u;
         if (r < J.n && c < src_w) v = reinterpret_cast<const uint32_t*>(J.src + r * J.row_bytes)[c];
-        reinterpret_cast<uint32_t*>(dst + r * ld_bytes)[c] = v;
+        reinterpret_cast<uint32_t*>(J.xb + r * J.ldb)[c] = v;
       }
     } else {
-      const int64_t total = J.rows * ld_bytes;
+      const int64_t total = J.rows * J.ldb;
       for (int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < total;
            e += int64_t(gridDim.x) * blockDim.x) {
-        const int64_t r = e / ld_bytes, c = e % ld_bytes;
-        dst[e] = (r < J.n && c < J.row_bytes) ? J.src[r * J.row_bytes + c] : uint8_t(0);
+        const int64_t r = e / J.ldb, c = e % J.ldb;
+        J.xb[e] = (r < J.n && c < J.row_bytes) ? J.src[r * J.row_bytes + c] : uint8_t(0);
       }
     }
   }
 }
 
-__global__ void __launch_bounds__(kRows)
-batch_row_norms_kernel(const BatchHeader* __restrict__ hdr, const BatchRowJob* __restrict__ jobs) {
-  __shared__ float slab[kRows][kSlab + 1];
+__device__ __forceinline__ PrepRows job_rows(const BatchRowJob& J) {
+  PrepRows p{};
+  p.src = reinterpret_cast<const float*>(J.src);
+  p.src_ld = J.row_bytes / 4;
+  p.x = J.x;
+  p.n = J.n;
+  p.rows = J.rows;
+  p.d = J.dim;
+  p.ld = J.ld;
+  p.norms = J.norms;
+  p.not_unit = J.flag;
+  p.half = reinterpret_cast<uint16_t*>(J.xb);
+  p.ldb = J.ldb / 2;
+  p.half_type = J.half_type;
+  p.rnorm = J.rnorm;
+  p.hnorm = J.hnorm;
+  p.maxes = J.maxes;
+  return p;
+}
+
+__global__ void batch_clear_kernel(const BatchHeader* __restrict__ hdr, const BatchRowJob* __restrict__ jobs) {
+  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < hdr->n_jobs; j += gridDim.x * blockDim.x) {
+    *jobs[j].flag = 0;
+    if (jobs[j].maxes)
+      for (int i = 0; i < kPrepMaxes; i++) jobs[j].maxes[i] = 0u;
+  }
+}
+
+__global__ void __launch_bounds__(kPrepWarps * 32)
+batch_prepare_kernel(const BatchHeader* __restrict__ hdr, const BatchRowJob* __restrict__ jobs) {
+  __shared__ float slab[2][kTileRows][kTileCols + 1];
   const int nj = hdr->n_jobs;
   const int64_t total = hdr->total_blocks;
   for (int64_t g = blockIdx.x; g < total; g += gridDim.x) {
     const BatchRowJob& J = jobs[find_block_job(jobs, nj, g)];
-    row_norms_block(J.x, J.n, int(J.ld), int(J.dim), J.norms, J.flag, (g - J.blk_base) * kRows, slab);
+    prepare_tile(job_rows(J), (g - J.blk_base) * kTileRows, slab);
+    __syncthreads();
   }
 }
 
-__global__ void batch_normalize_kernel(const BatchHeader* __restrict__ hdr, const BatchRowJob* __restrict__ jobs) {
+__global__ void batch_renormalize_kernel(const BatchHeader* __restrict__ hdr, const BatchRowJob* __restrict__ jobs) {
   const int nj = hdr->n_jobs;
-  for (int j = 0; j < nj; j++) {
-    const BatchRowJob& J = jobs[j];
-    if (*J.flag == 0) continue;
-    const int64_t d = J.dim, total = J.n * d;
-    for (int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < total; e += int64_t(gridDim.x) * blockDim.x) {
-      const int64_t r = e / d, c = e % d;
-      float nrm = J.norms[r];
-      if (nrm == 0.0f) nrm = 1.0f;
-      J.x[r * J.ld + c] = __fdiv_rn(J.x[r * J.ld + c], nrm);
-    }
-  }
-}
-
-__global__ void batch_to_half_kernel(const BatchHeader* __restrict__ hdr, const BatchRowJob* __restrict__ jobs) {
-  const int nj = hdr->n_jobs;
-  for (int j = 0; j < nj; j++) {
-    const BatchRowJob& J = jobs[j];
-    const int64_t lde = J.ldb / 2, total = J.rows * lde;
-    uint16_t* Y = reinterpret_cast<uint16_t*>(J.xb);
-    for (int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < total; e += int64_t(gridDim.x) * blockDim.x) {
-      const int64_t r = e / lde, c = e % lde;
-      Y[e] = half_bits((c < J.dim && r < J.n) ? J.x[r * J.ld + c] : 0.0f, J.half_type);
-    }
-  }
-}
-
-// The certificate's row norms of every f32 request (warp per row, as
-// to_half_kernel computes them).
-__global__ void batch_half_norms_kernel(const BatchHeader* __restrict__ hdr, const BatchRowJob* __restrict__ jobs) {
-  const int nj = hdr->n_jobs;
-  const int64_t total = hdr->total_rows;
-  const int lane = threadIdx.x & 31;
-  const int64_t warps = int64_t(gridDim.x) * (blockDim.x >> 5);
-  for (int64_t w = int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); w < total; w += warps) {
-    int lo = 0, hi = nj - 1;
-    while (lo < hi) {  // last request with row_base <= w
-      const int mid = (lo + hi + 1) >> 1;
-      if (jobs[mid].row_base <= w) lo = mid;
-      else hi = mid - 1;
-    }
-    const BatchRowJob& J = jobs[lo];
-    if (!J.rnorm) continue;
-    const int64_t r = w - J.row_base;
-    double rr = 0.0, hh = 0.0;
-    for (int c = lane; c < J.dim; c += 32) {
-      const float v = J.x[r * J.ld + c];
-      const float h = half_value(half_bits(v, J.half_type), J.half_type);
-      const double res = double(v) - double(h);
-      rr += res * res;
-      hh += double(h) * double(h);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      rr += __shfl_xor_sync(0xffffffffu, rr, o);
-      hh += __shfl_xor_sync(0xffffffffu, hh, o);
-    }
-    if (lane == 0) {
-      const float a = __double2float_ru(__dsqrt_ru(rr * (1.0 + 0x1p-30)));
-      const float b = __double2float_ru(__dsqrt_ru(hh * (1.0 + 0x1p-30)));
-      J.rnorm[r] = a;
-      J.hnorm[r] = b;
-      atomicMax(&J.maxes[0], __float_as_uint(a));
-      atomicMax(&J.maxes[1], __float_as_uint(b));
-    }
-  }
+  for (int j = 0; j < nj; j++)
+    if (*jobs[j].flag != 0) renormalize_rows(job_rows(jobs[j]));
 }
 
 cudaError_t launch_batch_rows(bool f32, const BatchHeader* hdr, const BatchRowJob* jobs, int grid_rows,
-                              int grid_norms, cudaStream_t stream) {
-  batch_copy_kernel<<<grid_rows, 256, 0, stream>>>(hdr, jobs, f32);
-  if (!f32) return cudaGetLastError();
-  batch_row_norms_kernel<<<grid_norms, kRows, 0, stream>>>(hdr, jobs);
-  batch_normalize_kernel<<<grid_rows, 256, 0, stream>>>(hdr, jobs);
-  batch_to_half_kernel<<<grid_rows, 256, 0, stream>>>(hdr, jobs);
-  batch_half_norms_kernel<<<grid_norms, kRows, 0, stream>>>(hdr, jobs);
+                              int grid_tiles, cudaStream_t stream) {
+  if (!f32) {
+    batch_copy_kernel<<<grid_rows, 256, 0, stream>>>(hdr, jobs);
+    return cudaGetLastError();
+  }
+  batch_clear_kernel<<<1, 256, 0, stream>>>(hdr, jobs);
+  batch_prepare_kernel<<<grid_tiles, kPrepWarps * 32, 0, stream>>>(hdr, jobs);
+  batch_renormalize_kernel<<<grid_rows, 256, 0, stream>>>(hdr, jobs);
   return cudaGetLastError();
 }
 
