@@ -10,7 +10,7 @@
 //   pca_init + small-graph norm . src/label_prop.rs:251-309   pca_kernel
 //   final centring / scaling .... src/label_prop.rs:660-672   center_* kernels
 //   make_epochs_per_sample ...... src/embed.rs:10-23          ne_schedule_kernel
-//   node_embedding_epoch_repr ... src/embed.rs:138-248        ne_block_kernel, ne_heavy_kernel, ne_apply_kernel
+//   node_embedding_epoch_repr ... src/embed.rs:138-248        ne_epoch_kernel
 //   node_embedding_epoch ........ src/embed.rs:57-135         ne_hogwild_kernel (lock-free, not bit-exact)
 //
 // Every result matches the reference's rounding: f32 expressions are written
@@ -32,6 +32,7 @@
 //     e) list each (p, q) group in temp's row order; a group's head (largest
 //     first e) is where q first appears, so the row's output order is the
 //     heads' first e ascending.
+#include <cooperative_groups.h>
 #include <cub/cub.cuh>
 #include <thrust/iterator/counting_iterator.h>
 
@@ -202,8 +203,11 @@ __global__ void validate_csr_kernel(Csr g, int32_t* bad) {
     if (g.indices[e] < 0 || g.indices[e] >= g.n) atomicExch(bad, 1);
 }
 
+// labels[idx[i]] = i over labels of -1; of a repeated index the last one stays.
+// One thread took 0.5 ms for the five levels of 200,000 rows, the atomics 0.01.
 __global__ void seed_labels_kernel(int32_t* labels, const int64_t* idx, int64_t count) {
-  for (int64_t i = 0; i < count; i++) labels[idx[i]] = (int32_t)i;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x)
+    atomicMax(&labels[idx[i]], (int32_t)i);
 }
 
 // Unlabelled-row flags and the largest label, before the outlier walk.
@@ -1097,13 +1101,6 @@ __device__ __forceinline__ uint64_t neg_count(float nf, float eon, float rate) {
 
 __device__ __forceinline__ float clip4(float v) { return v > 4.0f ? 4.0f : (v < -4.0f ? -4.0f : v); }
 
-// Rows of more than min_deg edges, deferred by ne_block_kernel to ne_heavy_kernel.
-struct HeavyRows {
-  int64_t min_deg;
-  uint32_t* rows;
-  int32_t* count;
-};
-
 // The positive move of one edge (scaled by alpha); false when the squared
 // distance is 0 (the reference adds nothing then).
 template <int MAXD>
@@ -1130,9 +1127,12 @@ __device__ __forceinline__ bool ne_pos(const float* cur, const float* yt, int nc
 // Negative sample p of edge `raw` (scaled and clipped); false when it adds nothing.
 template <int MAXD>
 __device__ __forceinline__ bool ne_neg(const float* cur, const float* emb, const uint32_t* order, uint64_t nv,
-                                       uint64_t raw, uint64_t p, uint32_t epoch, uint32_t rng_state, int ncomp,
+                                       uint64_t nv_inv, uint64_t raw, uint64_t p, uint32_t epoch, uint32_t rng_state, int ncomp,
                                        float gamma, float alpha, float* out) {
-  const uint64_t idx = (raw * ((uint64_t)epoch + p + 1ull) * (uint64_t)rng_state) % nv;
+  const uint64_t x = raw * ((uint64_t)epoch + p + 1ull) * (uint64_t)rng_state;
+  // x % nv: the quotient by the rounded-down reciprocal is at most two short
+  uint64_t idx = x - __umul64hi(x, nv_inv) * nv;
+  while (idx >= nv) idx -= nv;
   const uint64_t tn = order[idx];
   if (tn >= nv) return false;
   const float* yn = emb + tn * ncomp;
@@ -1152,279 +1152,419 @@ __device__ __forceinline__ bool ne_neg(const float* cur, const float* emb, const
   return true;
 }
 
-constexpr int kHeavyWarps = 16;
-constexpr int kHeavySlots = 4;  // positive move + 3 negative samples staged per edge
-constexpr uint32_t kHeavyOverflow = 0x80000000u;
+constexpr int kNegSlots = 3;           // negative samples of an edge staged at once
+constexpr int kSlots = 1 + kNegSlots;  // with the positive move
+constexpr uint32_t kUnstaged = 0x80000000u;
+constexpr int kMaxBlocks = kNeCounts / 2;  // of an epoch: n / max(1024, n / 8), rounded up, is at most 9
 
-__host__ __device__ inline int heavy_tile_edges(int ncomp) { return ncomp <= 8 ? 512 : (ncomp <= 16 ? 256 : 128); }
-__host__ __device__ inline size_t heavy_smem_bytes(int ncomp) {
-  return size_t(2) * heavy_tile_edges(ncomp) * (size_t(kHeavySlots) * ncomp + 2) * sizeof(float) +
-         size_t(heavy_tile_edges(ncomp)) * kHeavySlots * sizeof(uint32_t);
+template <int MAXD>
+struct NeShape {
+  // Registers and shared memory for as many warps as an SM holds at that
+  // width: two CTAs of 16 warps up to 8 components, one above.
+  static constexpr int kWarps = MAXD <= 16 ? 16 : 8;
+  static constexpr int kCtas = MAXD <= 8 ? 2 : 1;
+  static constexpr int kTile = 16 * kWarps;  // edges of a heavy row staged at once, twice
+  static constexpr int kWidth = MAXD <= 8 ? 8 : MAXD <= 16 ? 16 : 32;  // lanes of a row's components
+  static constexpr int kRows = 32 / kWidth;                            // rows of a warp
+};
+
+// A warp's staging: 32 edges of kSlots contributions (an odd stride), the
+// offsets of those that are added, the rows' own embedding, 64 queued edges.
+__host__ __device__ inline int ne_edge_stride(int ncomp) { return (kSlots * ncomp) | 1; }
+__host__ __device__ inline int ne_stage_floats(int ncomp) { return 32 * ne_edge_stride(ncomp) + 32 * kSlots + 32 + 5 * 64; }
+
+struct NeEpoch {
+  Csr g;
+  float *emb, *upd;
+  const uint32_t* order;
+  const float *eps, *epns;
+  float *eonn, *eons;
+  uint64_t nv_inv;  // floor((2^64 - 1) / n)
+  uint32_t rng_state;
+  int ncomp;
+  float alpha;
+  uint32_t epoch;
+  float noise, gamma, decay;
+  int apply_decay;
+  int64_t block;        // nodes of a block
+  int64_t heavy_deg;    // rows with more edges take a CTA
+  int take;             // rows that a warp takes at once, up to kRows
+  uint32_t* heavy;      // those of block b from b * block on
+  int32_t* counts;      // kMaxBlocks numbers of heavy rows, kMaxBlocks work counters; zeros at the start
+};
+
+// Adds component d of `total` staged contributions, whose offsets stand in
+// `offs`, to a row's update, in the order listed (the reference's order of f32
+// additions for that component).  `slow` adds an unstaged entry.
+template <class Slow>
+__device__ __forceinline__ float ne_add(float ud, const float* buf, const uint32_t* offs, int total, int d,
+                                        Slow slow) {
+  int q = 0;
+  while (q < total) {
+    for (; q + 4 <= total; q += 4) {
+      uint32_t o4[4];
+      float v4[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) o4[j] = offs[q + j];
+      if ((o4[0] | o4[1] | o4[2] | o4[3]) & kUnstaged) break;
+#pragma unroll
+      for (int j = 0; j < 4; j++) v4[j] = buf[o4[j] + d];
+#pragma unroll
+      for (int j = 0; j < 4; j++) ud = __fadd_rn(ud, v4[j]);
+    }
+    const int stop = min(q + 4, total);
+    for (; q < stop; q++) {
+      const uint32_t o = offs[q];
+      if (o & kUnstaged) slow(o & ~kUnstaged, ud);
+      else ud = __fadd_rn(ud, buf[o + d]);
+    }
+  }
+  return ud;
 }
 
-// One CTA per deferred row.  Warps 1..15 compute the contributions of a tile
-// of the row's edges into shared memory while warp 0 adds the previous
-// tile's, in edge order, lane d keeping component d of the update row (the
-// reference's order of f32 additions for that component).  An edge wanting
-// more negative samples than the staging holds is flagged and its samples
-// are computed by warp 0 in order.
-template <int MAXD, int MINB>
-__global__ void __launch_bounds__(kHeavyWarps * 32, MINB)
-    ne_heavy_kernel(Csr g, float* emb, float* upd, const uint32_t* order, const float* eps, const float* epns,
-                    float* eonn, float* eons, uint32_t rng_state, int ncomp, float alpha, uint32_t epoch,
-                    float noise, float gamma, float decay, int apply_decay, HeavyRows heavy) {
-  extern __shared__ float hv_sh[];
+// A row of more than heavy_deg edges, by one CTA.  Warps 1 and up compute the
+// contributions of a tile of its edges while warp 0 adds the previous tile's.
+// An edge that wants more negative samples than its slots is flagged, and warp
+// 0 computes them in order.
+template <int MAXD>
+__device__ void ne_heavy_row(const NeEpoch& E, uint64_t from, float* sh) {
+  constexpr int te = NeShape<MAXD>::kTile;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int te = heavy_tile_edges(ncomp);
-  const int stride = kHeavySlots * ncomp + 2;  // floats per staged edge: slots, mask, count
-  const uint64_t nv = (uint64_t)g.n;
-  const float nf = (float)epoch;
-  const int32_t cnt = *heavy.count;
-  for (int32_t h = blockIdx.x; h < cnt; h += gridDim.x) {
-    const uint64_t from = heavy.rows[h];
+  const int ncomp = E.ncomp;
+  const int stride = kSlots * ncomp + 2;  // floats of a staged edge: slots, mask, samples
+  const uint64_t nv = (uint64_t)E.g.n;
+  const float nf = (float)E.epoch;
+  float cur[MAXD];
+#pragma unroll
+  for (int d = 0; d < MAXD; d++)
+    if (d < ncomp) cur[d] = E.emb[from * ncomp + d];
+  const uint64_t e0 = (uint64_t)E.g.indptr[from], e1 = (uint64_t)E.g.indptr[from + 1];
+  const int64_t tiles = (int64_t)((e1 - e0 + te - 1) / te);
+  float ud = 0.0f;
+  if (warp == 0 && lane < ncomp)
+    ud = E.apply_decay ? __fmul_rn(E.upd[from * ncomp + lane], E.decay) : E.upd[from * ncomp + lane];
+  auto stage = [&](int64_t tile, int first_thread, int threads) {
+    float* buf = sh + (size_t)(tile & 1) * te * stride;
+    for (int i = (int)threadIdx.x - first_thread; i < te; i += threads) {
+      const uint64_t raw = e0 + (uint64_t)tile * te + i;
+      float* ent = buf + (size_t)i * stride;
+      uint32_t m = 0, nn = 0;
+      if (raw < e1) {
+        const float on = E.eons[raw], onn = E.eonn[raw], rate = E.epns[raw];
+        const uint64_t to = (uint64_t)(uint32_t)E.g.indices[raw];
+        if (!(on > nf) && to < nv) {
+          if (ne_pos<MAXD>(cur, E.emb + to * ncomp, ncomp, E.noise, E.alpha, ent)) m |= 1u;
+          E.eons[raw] = __fadd_rn(on, E.eps[raw]);
+          const uint64_t nneg = neg_count(nf, onn, rate);
+          nn = (uint32_t)nneg;
+          if (nneg < (uint64_t)kSlots) {
+            for (uint64_t p = 0; p < nneg; p++)
+              if (ne_neg<MAXD>(cur, E.emb, E.order, nv, E.nv_inv, raw, p, E.epoch, E.rng_state, ncomp, E.gamma,
+                               E.alpha, ent + (1 + p) * ncomp))
+                m |= 2u << p;
+          } else {
+            m |= kUnstaged;
+          }
+          E.eonn[raw] = __fadd_rn(onn, __fmul_rn(__ull2float_rn(nneg), rate));
+        }
+      }
+      reinterpret_cast<uint32_t*>(ent)[kSlots * ncomp] = m;
+      reinterpret_cast<uint32_t*>(ent)[kSlots * ncomp + 1] = nn;
+    }
+  };
+  stage(0, 0, blockDim.x);
+  __syncthreads();
+  uint32_t* offs = reinterpret_cast<uint32_t*>(sh + (size_t)2 * te * stride);  // te * kSlots
+  for (int64_t t = 0; t < tiles; t++) {
+    if (warp == 0) {
+      const float* buf = sh + (size_t)(t & 1) * te * stride;
+      const int64_t left = (int64_t)(e1 - e0) - t * te;
+      const int n_in = (int)(left < te ? left : te);
+      // offsets of the contributions in edge and slot order; an edge whose samples were not staged
+      // is listed as kUnstaged | edge
+      const int per = (n_in + 31) / 32;
+      const int i0 = lane * per, i1 = min(n_in, i0 + per);
+      int mine = 0;
+      for (int i = i0; i < i1; i++) {
+        const uint32_t m = reinterpret_cast<const uint32_t*>(buf + (size_t)i * stride)[kSlots * ncomp];
+        mine += (m & kUnstaged) ? (int)(m & 1u) + 1 : __popc(m);
+      }
+      int at = mine;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(kFull, at, o);
+        if (lane >= o) at += v;
+      }
+      const int total = __shfl_sync(kFull, at, 31);
+      at -= mine;
+      for (int i = i0; i < i1; i++) {
+        const uint32_t m = reinterpret_cast<const uint32_t*>(buf + (size_t)i * stride)[kSlots * ncomp];
+        for (uint32_t bits = m & ~kUnstaged; bits; bits &= bits - 1u)
+          offs[at++] = (uint32_t)(i * stride + (__ffs(bits) - 1) * ncomp);
+        if (m & kUnstaged) offs[at++] = kUnstaged | (uint32_t)i;
+      }
+      __syncwarp();
+      ud = ne_add(ud, buf, offs, total, lane < ncomp ? lane : 0, [&](uint32_t i, float& u) {
+        const uint32_t nn = reinterpret_cast<const uint32_t*>(buf + (size_t)i * stride)[kSlots * ncomp + 1];
+        const uint64_t raw = e0 + (uint64_t)t * te + i;
+        float c[MAXD];
+        for (uint64_t p = 0; p < nn; p++)
+          if (ne_neg<MAXD>(cur, E.emb, E.order, nv, E.nv_inv, raw, p, E.epoch, E.rng_state, ncomp, E.gamma, E.alpha,
+                           c)) {
+#pragma unroll
+            for (int d = 0; d < MAXD; d++)
+              if (d == lane && d < ncomp) u = __fadd_rn(u, c[d]);
+          }
+      });
+    } else if (t + 1 < tiles) {
+      stage(t + 1, 32, blockDim.x - 32);
+    }
+    __syncthreads();
+  }
+  if (warp == 0 && lane < ncomp) E.upd[from * ncomp + lane] = ud;
+  __syncthreads();
+}
+
+// The other rows, up to kRows of them by one warp: lane k holds row k (`deg` 0
+// for none).  An epoch samples a part of a row's edges, so those due are
+// queued in row and edge order, 32 of them compute their contributions at a
+// time (positive move, then each negative sample), and the contributions are
+// added with a lane to each (row, component), in edge order and within an edge
+// in sample order.  The next edges' schedules and ends are loaded meanwhile.
+// When an edge of the 32 wants more than kNegSlots samples, they are handed
+// through the staging one at a time.
+template <int MAXD>
+__device__ __forceinline__ void ne_light_rows(const NeEpoch& E, uint64_t from, uint64_t e0, uint32_t deg, bool valid,
+                                              float* sh) {
+  constexpr int kWidth = NeShape<MAXD>::kWidth, kRows = NeShape<MAXD>::kRows;
+  const int lane = threadIdx.x & 31;
+  const int ncomp = E.ncomp;
+  const int stride = ne_edge_stride(ncomp);
+  uint32_t* offs = reinterpret_cast<uint32_t*>(sh + 32 * stride);
+  float* curs = sh + 32 * stride + 32 * kSlots;
+  uint32_t* q_at = reinterpret_cast<uint32_t*>(curs + 32);  // row << 28 | position among the rows' edges
+  uint32_t* q_to = q_at + 64;
+  float *q_on = curs + 32 + 128, *q_onn = q_on + 64, *q_rate = q_onn + 64;
+  const uint64_t nv = (uint64_t)E.g.n;
+  const float nf = (float)E.epoch;
+  uint32_t end = lane < kRows ? deg : 0u;
+#pragma unroll
+  for (int o = 1; o < kRows; o <<= 1) {
+    const uint32_t v = __shfl_up_sync(kFull, end, o);
+    if (lane >= o) end += v;
+  }
+  const uint64_t first = e0 - (end - deg);  // + a position: the edge
+  uint32_t ends[kRows];
+#pragma unroll
+  for (int k = 0; k < kRows; k++) ends[k] = __shfl_sync(kFull, end, k);
+  const uint32_t total = ends[kRows - 1];
+  const int mk = lane / kWidth, md = lane % kWidth;
+  const uint64_t my_from = __shfl_sync(kFull, from, mk);
+  const bool mine = __shfl_sync(kFull, (int)valid, mk) && md < ncomp;
+  float ud = 0.0f;
+  if (mine) {
+    ud = E.upd[my_from * ncomp + md];
+    if (E.apply_decay) ud = __fmul_rn(ud, E.decay);
+    curs[lane] = E.emb[my_from * ncomp + md];
+  }
+  float on = 0.0f, onn = 0.0f, rate = 0.0f;
+  uint32_t to = 0, at_row = 0;
+  auto fetch = [&](uint32_t t) {
+    uint32_t k = 0;
+#pragma unroll
+    for (int j = 0; j + 1 < kRows; j++) k += t >= ends[j];
+    const uint64_t raw = __shfl_sync(kFull, first, k) + t;
+    at_row = k << 28 | t;
+    if (t >= total) return;
+    on = E.eons[raw];
+    to = (uint32_t)E.g.indices[raw];
+    onn = E.eonn[raw];
+    rate = E.epns[raw];
+  };
+  fetch(lane);
+  uint32_t base = 0;
+  int queued = 0;
+  for (;;) {
+    while (queued < 32 && base < total) {
+      const bool due = base + lane < total && !(on > nf) && (uint64_t)to < nv;
+      const unsigned m = __ballot_sync(kFull, due);
+      if (due) {
+        const int at = queued + __popc(m & ((1u << lane) - 1u));
+        q_at[at] = at_row;
+        q_to[at] = to;
+        q_on[at] = on;
+        q_onn[at] = onn;
+        q_rate[at] = rate;
+      }
+      queued += __popc(m);
+      base += 32;
+      fetch(base + lane);
+    }
+    __syncwarp();
+    if (queued == 0) break;
+    const bool in = lane < queued;
+    const uint32_t a = in ? q_at[lane] : 0u;
+    const uint32_t k = a >> 28;
+    const uint64_t raw = __shfl_sync(kFull, first, k) + (a & 0x0fffffffu);
+    float* vec = sh + lane * stride;
     float cur[MAXD];
-#pragma unroll
-    for (int d = 0; d < MAXD; d++)
-      if (d < ncomp) cur[d] = emb[from * ncomp + d];
-    const uint64_t e0 = (uint64_t)g.indptr[from], e1 = (uint64_t)g.indptr[from + 1];
-    const int64_t tiles = (int64_t)((e1 - e0 + te - 1) / te);
-    float ud = 0.0f;
-    if (warp == 0 && lane < ncomp)
-      ud = apply_decay ? __fmul_rn(upd[from * ncomp + lane], decay) : upd[from * ncomp + lane];
-    auto stage = [&](int64_t tile, int first_thread, int threads) {
-      float* buf = hv_sh + (size_t)(tile & 1) * te * stride;
-      for (int i = (int)threadIdx.x - first_thread; i < te; i += threads) {
-        const uint64_t raw = e0 + (uint64_t)tile * te + i;
-        float* ent = buf + (size_t)i * stride;
-        uint32_t m = 0, nn = 0;
-        if (raw < e1 && !(eons[raw] > nf)) {
-          const uint64_t to = (uint64_t)(uint32_t)g.indices[raw];
-          if (to < nv) {
-            if (ne_pos<MAXD>(cur, emb + to * ncomp, ncomp, noise, alpha, ent)) m |= 1u;
-            eons[raw] = __fadd_rn(eons[raw], eps[raw]);
-            const float rate = epns[raw];
-            const uint64_t nneg = neg_count(nf, eonn[raw], rate);
-            nn = (uint32_t)nneg;
-            if (nneg < (uint64_t)kHeavySlots) {
-              for (uint64_t p = 0; p < nneg; p++)
-                if (ne_neg<MAXD>(cur, emb, order, nv, raw, p, epoch, rng_state, ncomp, gamma, alpha,
-                                 ent + (1 + p) * ncomp))
-                  m |= 2u << p;
-            } else {
-              m |= kHeavyOverflow;
-            }
-            eonn[raw] = __fadd_rn(eonn[raw], __fmul_rn(__ull2float_rn(nneg), rate));
-          }
-        }
-        reinterpret_cast<uint32_t*>(ent)[kHeavySlots * ncomp] = m;
-        reinterpret_cast<uint32_t*>(ent)[kHeavySlots * ncomp + 1] = nn;
-      }
-    };
-    stage(0, 0, blockDim.x);
-    __syncthreads();
-    uint32_t* offs = reinterpret_cast<uint32_t*>(hv_sh + (size_t)2 * te * stride);  // te * kHeavySlots
-    for (int64_t t = 0; t < tiles; t++) {
-      if (warp == 0) {
-        const float* buf = hv_sh + (size_t)(t & 1) * te * stride;
-        const int64_t left = (int64_t)(e1 - e0) - t * te;
-        const int n_in = (int)(left < te ? left : te);
-        // offsets (in floats) of the applied contributions, in edge order and slot order; an edge
-        // whose negative samples were not staged is listed as 0x80000000 | edge
-        const int per = (n_in + 31) / 32;
-        const int i0 = lane * per, i1 = min(n_in, i0 + per);
-        int mine = 0;
-        for (int i = i0; i < i1; i++) {
-          const uint32_t m = reinterpret_cast<const uint32_t*>(buf + (size_t)i * stride)[kHeavySlots * ncomp];
-          mine += (m & kHeavyOverflow) ? (int)(m & 1u) + 1 : __popc(m);
-        }
-        int at = mine;
-        for (int o = 1; o < 32; o <<= 1) {
-          const int v = __shfl_up_sync(kFull, at, o);
-          if (lane >= o) at += v;
-        }
-        const int total = __shfl_sync(kFull, at, 31);
-        at -= mine;
-        for (int i = i0; i < i1; i++) {
-          const uint32_t m = reinterpret_cast<const uint32_t*>(buf + (size_t)i * stride)[kHeavySlots * ncomp];
-          for (uint32_t bits = m & ~kHeavyOverflow; bits; bits &= bits - 1u)
-            offs[at++] = (uint32_t)(i * stride + (__ffs(bits) - 1) * ncomp);
-          if (m & kHeavyOverflow) offs[at++] = kHeavyOverflow | (uint32_t)i;
-        }
-        __syncwarp();
-        int q = 0;
-        for (; q + 4 <= total; q += 4) {
-          uint32_t o4[4];
-          float v4[4];
-#pragma unroll
-          for (int j = 0; j < 4; j++) o4[j] = offs[q + j];
-          if ((o4[0] | o4[1] | o4[2] | o4[3]) & kHeavyOverflow) break;
-#pragma unroll
-          for (int j = 0; j < 4; j++) v4[j] = lane < ncomp ? buf[o4[j] + lane] : 0.0f;
-#pragma unroll
-          for (int j = 0; j < 4; j++)
-            if (lane < ncomp) ud = __fadd_rn(ud, v4[j]);
-        }
-        for (; q < total; q++) {
-          const uint32_t o = offs[q];
-          if (o & kHeavyOverflow) {
-            const int i = (int)(o & ~kHeavyOverflow);
-            const uint32_t nn = reinterpret_cast<const uint32_t*>(buf + (size_t)i * stride)[kHeavySlots * ncomp + 1];
-            const uint64_t raw = e0 + (uint64_t)t * te + i;
-            float c[MAXD];
-            for (uint64_t p = 0; p < nn; p++)
-              if (ne_neg<MAXD>(cur, emb, order, nv, raw, p, epoch, rng_state, ncomp, gamma, alpha, c)) {
-#pragma unroll
-                for (int d = 0; d < MAXD; d++)
-                  if (d == lane && d < ncomp) ud = __fadd_rn(ud, c[d]);
-              }
-          } else if (lane < ncomp) {
-            ud = __fadd_rn(ud, buf[o + lane]);
-          }
-        }
-      } else if (t + 1 < tiles) {
-        stage(t + 1, 32, blockDim.x - 32);
-      }
-      __syncthreads();
-    }
-    if (warp == 0 && lane < ncomp) upd[from * ncomp + lane] = ud;
-    __syncthreads();
-  }
-}
-
-constexpr int kNeWarps = 4;    // warps (nodes in flight) per CTA
-constexpr int kNegSlots = 3;   // negative samples per edge staged at once
-
-// Per-warp staging: [32 lanes][1 + kNegSlots][ncomp] contributions, then 32
-// flags (and 32 spare words).
-__host__ __device__ inline int ne_stage_floats(int ncomp) { return 32 * (1 + kNegSlots) * ncomp + 64; }
-
-// One warp per node of the block.  The lanes take 32 consecutive edges and
-// compute their contributions (positive move, then each negative sample)
-// from the embedding as it stood at the block's start; then every lane adds
-// them, in edge order and within an edge in sample order, to its own copy of
-// the node's update row -- the reference's serial order of f32 additions.
-// Edges wanting more than kNegSlots negative samples in a chunk are handed
-// through the staging one contribution at a time instead.
-template <int MAXD, int MINB>
-__global__ void __launch_bounds__(kNeWarps * 32, MINB)
-    ne_block_kernel(Csr g, float* emb, float* upd, const uint32_t* order, int64_t bs, int64_t be, const float* eps,
-                    const float* epns, float* eonn, float* eons, uint32_t rng_state, int ncomp, float alpha,
-                    uint32_t epoch, float noise, float gamma, float decay, int apply_decay, HeavyRows heavy) {
-  extern __shared__ float ne_sh[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  constexpr int kSlots = 1 + kNegSlots;
-  float* vec = ne_sh + (size_t)warp * ne_stage_floats(ncomp);
-  uint32_t* fmask = reinterpret_cast<uint32_t*>(vec + 32 * kSlots * ncomp);
-  const uint64_t nv = (uint64_t)g.n;
-  const float nf = (float)epoch;
-  const int64_t step = (int64_t)gridDim.x * kNeWarps;
-  int64_t ni = bs + (int64_t)blockIdx.x * kNeWarps + warp;
-  // the next node's id and row bounds are loaded while the current one runs
-  uint64_t nfrom = ni < be ? order[ni] : nv;
-  uint64_t ne0 = 0, ne1 = 0;
-  if (nfrom < nv) {
-    ne0 = (uint64_t)g.indptr[nfrom];
-    ne1 = (uint64_t)g.indptr[nfrom + 1];
-  }
-  for (; ni < be; ni += step) {
-    const uint64_t from = nfrom, e0 = ne0, e1 = ne1;
-    nfrom = ni + step < be ? order[ni + step] : nv;
-    if (nfrom < nv) {
-      ne0 = (uint64_t)g.indptr[nfrom];
-      ne1 = (uint64_t)g.indptr[nfrom + 1];
-    }
-    if (from >= nv) continue;
-    if ((int64_t)(e1 - e0) > heavy.min_deg) {  // deferred to ne_heavy_kernel
-      if (lane == 0) heavy.rows[atomicAdd(heavy.count, 1)] = (uint32_t)from;
-      continue;
-    }
-    float cur[MAXD], u[MAXD];
-#pragma unroll
-    for (int d = 0; d < MAXD; d++)
-      if (d < ncomp) {
-        cur[d] = emb[from * ncomp + d];
-        u[d] = apply_decay ? __fmul_rn(upd[from * ncomp + d], decay) : upd[from * ncomp + d];
-      }
-    for (uint64_t base = e0; base < e1; base += 32) {
-      const uint64_t raw = base + lane;
-      bool act = false;
-      uint64_t to = 0;
-      if (raw < e1 && !(eons[raw] > nf)) {
-        to = (uint64_t)(uint32_t)g.indices[raw];
-        act = to < nv;
-      }
-      if (!__any_sync(kFull, act)) continue;
-      uint32_t fl = 0;
-      uint64_t nneg = 0;
-      float rate = 0.0f;
-      float cp[MAXD];
-      if (act) {
-        if (ne_pos<MAXD>(cur, emb + to * ncomp, ncomp, noise, alpha, cp)) fl = 1u;
-        eons[raw] = __fadd_rn(eons[raw], eps[raw]);
-        rate = epns[raw];
-        nneg = neg_count(nf, eonn[raw], rate);
-      }
-      auto add_slot = [&](int L, int slot) {
-        const float* src = vec + ((size_t)L * kSlots + slot) * ncomp;
-#pragma unroll
-        for (int d = 0; d < MAXD; d++)
-          if (d < ncomp) u[d] = __fadd_rn(u[d], src[d]);
-      };
-      const int maxneg = (int)__reduce_max_sync(kFull, (unsigned)(nneg < (1ull << 30) ? nneg : (1ull << 30)));
-      if (maxneg <= kNegSlots) {
-        if (fl) {
-          float* dst = vec + (size_t)lane * kSlots * ncomp;
-#pragma unroll
-          for (int d = 0; d < MAXD; d++)
-            if (d < ncomp) dst[d] = cp[d];
-        }
-        for (int p = 0; p < maxneg; p++)
-          if ((uint64_t)p < nneg &&
-              ne_neg<MAXD>(cur, emb, order, nv, raw, (uint64_t)p, epoch, rng_state, ncomp, gamma, alpha,
-                           vec + ((size_t)lane * kSlots + 1 + p) * ncomp))
-            fl |= 2u << p;
-        __syncwarp();
-        // lanes with something to add, in lane (= edge) order; their slots in sample order
-        for (unsigned live = __ballot_sync(kFull, fl != 0); live; live &= live - 1u) {
-          const int L = __ffs(live) - 1;
-          const uint32_t f = __shfl_sync(kFull, fl, L);
-          for (uint32_t bits = f; bits; bits &= bits - 1u) add_slot(L, __ffs(bits) - 1);
-        }
-        __syncwarp();
-      } else {
-        for (int L = 0; L < 32; L++) {
-          const uint64_t nL = __shfl_sync(kFull, nneg, L);
-          const uint32_t fL = __shfl_sync(kFull, fl, L);
-          if (fL) {
-            if (lane == L) {
-              float* dst = vec + (size_t)lane * kSlots * ncomp;
-#pragma unroll
-              for (int d = 0; d < MAXD; d++)
-                if (d < ncomp) dst[d] = cp[d];
-            }
-            __syncwarp();
-            add_slot(L, 0);
-            __syncwarp();
-          }
-          for (uint64_t p = 0; p < nL; p++) {
-            if (lane == L)
-              fmask[L] = ne_neg<MAXD>(cur, emb, order, nv, raw, p, epoch, rng_state, ncomp, gamma, alpha,
-                                      vec + (size_t)lane * kSlots * ncomp + ncomp)
-                             ? 1u
-                             : 0u;
-            __syncwarp();
-            if (fmask[L]) add_slot(L, 1);
-            __syncwarp();
-          }
-        }
-      }
-      if (act) eonn[raw] = __fadd_rn(eonn[raw], __fmul_rn(__ull2float_rn(nneg), rate));
-    }
-    if (lane == 0) {
+    uint32_t fl = 0;
+    uint64_t nneg = 0;
+    if (in) {
+      const float step = E.eps[raw], onn_now = q_onn[lane], rate_now = q_rate[lane];
 #pragma unroll
       for (int d = 0; d < MAXD; d++)
-        if (d < ncomp) upd[from * ncomp + d] = u[d];
+        if (d < ncomp) cur[d] = curs[k * kWidth + d];
+      nneg = neg_count(nf, onn_now, rate_now);
+      if (ne_pos<MAXD>(cur, E.emb + (uint64_t)q_to[lane] * ncomp, ncomp, E.noise, E.alpha, vec)) fl = 1u;
+      E.eons[raw] = __fadd_rn(q_on[lane], step);
+      E.eonn[raw] = __fadd_rn(onn_now, __fmul_rn(__ull2float_rn(nneg), rate_now));
     }
+    const int maxneg = (int)__reduce_max_sync(kFull, (unsigned)(nneg < (1ull << 30) ? nneg : (1ull << 30)));
+    if (maxneg <= kNegSlots) {
+      for (int p = 0; p < maxneg; p++)
+        if ((uint64_t)p < nneg &&
+            ne_neg<MAXD>(cur, E.emb, E.order, nv, E.nv_inv, raw, (uint64_t)p, E.epoch, E.rng_state, ncomp, E.gamma,
+                         E.alpha, vec + (1 + p) * ncomp))
+          fl |= 2u << p;
+      int stop = __popc(fl);
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(kFull, stop, o);
+        if (lane >= o) stop += v;
+      }
+      int at = stop - __popc(fl);
+      int begin = 0, count = 0;  // of my row's contributions
+#pragma unroll
+      for (int j = 0; j < kRows; j++) {
+        const unsigned m = __ballot_sync(kFull, in && k == (uint32_t)j);
+        const int b = __shfl_sync(kFull, at, m ? __ffs(m) - 1 : 0), e = __shfl_sync(kFull, stop, m ? 31 - __clz(m) : 0);
+        if (mk == j && m) {
+          begin = b;
+          count = e - b;
+        }
+      }
+      for (uint32_t bits = fl; bits; bits &= bits - 1u)
+        offs[at++] = (uint32_t)(lane * stride + (__ffs(bits) - 1) * ncomp);
+      __syncwarp();
+      ud = ne_add(ud, sh, offs + begin, count, md < ncomp ? md : 0, [](uint32_t, float&) {});
+    } else {
+      const int d = md < ncomp ? md : 0;
+      __syncwarp();
+      for (int L = 0; L < 32; L++) {
+        const uint64_t nL = __shfl_sync(kFull, nneg, L);
+        const bool here = (int)__shfl_sync(kFull, k, L) == mk;
+        if (__shfl_sync(kFull, fl, L) && here) ud = __fadd_rn(ud, sh[L * stride + d]);
+        for (uint64_t p = 0; p < nL; p++) {
+          bool some = false;
+          if (lane == L)
+            some = ne_neg<MAXD>(cur, E.emb, E.order, nv, E.nv_inv, raw, p, E.epoch, E.rng_state, ncomp, E.gamma,
+                                E.alpha, vec + ncomp);
+          __syncwarp();
+          if (__any_sync(kFull, some) && here) ud = __fadd_rn(ud, sh[L * stride + ncomp + d]);
+          __syncwarp();
+        }
+      }
+    }
+    // what is queued beyond the 32 moves to the front
+    const int left = queued > 32 ? queued - 32 : 0;
+    uint32_t m_at = 0, m_to = 0;
+    float m_on = 0.0f, m_onn = 0.0f, m_rate = 0.0f;
+    if (lane < left) {
+      m_at = q_at[32 + lane];
+      m_to = q_to[32 + lane];
+      m_on = q_on[32 + lane];
+      m_onn = q_onn[32 + lane];
+      m_rate = q_rate[32 + lane];
+    }
+    __syncwarp();
+    if (lane < left) {
+      q_at[lane] = m_at;
+      q_to[lane] = m_to;
+      q_on[lane] = m_on;
+      q_onn[lane] = m_onn;
+      q_rate[lane] = m_rate;
+    }
+    queued = left;
+  }
+  if (mine) E.upd[my_from * ncomp + md] = ud;
+  __syncwarp();
+}
+
+// One reproducible epoch (node_embedding_epoch_repr, src/embed.rs:138-248) in
+// one cooperative launch.  Within a block every node reads the embedding as it
+// stood at the block's start, so a block is two phases between grid barriers:
+// the nodes' update rows (heavy rows by a CTA each, the others a few to a
+// warp), and their addition to the embedding.
+//
+// Bound by latency: a node is a chain of dependent gathers (order, row, edges'
+// schedules and ends, their rows) with ordered additions at its end, and a
+// block of a reduced graph has fewer nodes than the chip has warps.  A launch
+// each for the two kinds of rows, the addition and a clear cost a block 5 to 6
+// us besides.  100,000 rows of 23 edges, 5 components: 412 -> 220 us an epoch
+// (of which 4 us are the barriers of each of the 8 blocks).
+template <int MAXD>
+__global__ void __launch_bounds__(NeShape<MAXD>::kWarps * 32, NeShape<MAXD>::kCtas) ne_epoch_kernel(const NeEpoch E) {
+  extern __shared__ float ne_sh[];
+  const cooperative_groups::grid_group all = cooperative_groups::this_grid();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t n = E.g.n;
+  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, threads = (int64_t)gridDim.x * blockDim.x;
+  float* vec = ne_sh + (size_t)warp * ne_stage_floats(E.ncomp);
+  // rows i .. i + take - 1 of the block at bs, a lane each; their edges are theirs alone, so they
+  // can be read before the block's turn
+  uint64_t nfrom = 0, ne0 = 0, ne1 = 0;
+  bool nvalid = false;
+  auto load = [&](int64_t bs, int64_t i) {
+    const int64_t be = bs + E.block < n ? bs + E.block : n;
+    nvalid = lane < E.take && bs + i + lane < be;
+    if (nvalid) nfrom = E.order[bs + i + lane];
+    nvalid = nvalid && nfrom < (uint64_t)n;
+    ne0 = ne1 = 0;
+    if (nvalid) {
+      ne0 = (uint64_t)E.g.indptr[nfrom];
+      ne1 = (uint64_t)E.g.indptr[nfrom + 1];
+    }
+    return bs + i < be;
+  };
+  // every warp's first rows are fixed, with the last CTAs, which have none when a block is small,
+  // first at the heavy rows; the others are taken from a counter
+  const int64_t mine = (int64_t)(blockIdx.x * (blockDim.x >> 5) + warp) * E.take, fixed = threads / 32 * E.take;
+  bool more = load(0, mine);
+  for (int64_t i = tid; i < n; i += threads) {
+    const uint64_t from = E.order[i];
+    if (from < (uint64_t)n && E.g.indptr[from + 1] - E.g.indptr[from] > E.heavy_deg) {
+      const int64_t b = i / E.block;
+      E.heavy[b * E.block + atomicAdd(&E.counts[b], 1)] = (uint32_t)from;
+    }
+  }
+  all.sync();
+  int b = 0;
+  for (int64_t bs = 0; bs < n; bs += E.block, b++) {
+    const int64_t be = bs + E.block < n ? bs + E.block : n;
+    const int n_heavy = E.counts[b];
+    for (int h = gridDim.x - 1 - blockIdx.x; h < n_heavy; h += gridDim.x)
+      ne_heavy_row<MAXD>(E, E.heavy[bs + h], ne_sh);
+    while (more) {
+      const uint64_t from = nfrom, e0 = ne0, e1 = ne1;
+      const bool valid = nvalid && (int64_t)(e1 - e0) <= E.heavy_deg;
+      more = false;
+      if (be - bs > fixed) {
+        int32_t i = 0;
+        if (lane == 0) i = atomicAdd(E.counts + kMaxBlocks + b, E.take);
+        i = __shfl_sync(kFull, i, 0);
+        more = load(bs, fixed + i);
+      }
+      ne_light_rows<MAXD>(E, from, e0, valid ? (uint32_t)(e1 - e0) : 0u, valid, vec);
+    }
+    if (be < n) more = load(be, mine);
+    all.sync();
+    for (int64_t i = tid; i < (be - bs) * E.ncomp; i += threads) {
+      const uint64_t from = E.order[bs + i / E.ncomp];
+      if (from >= (uint64_t)n) continue;
+      const uint64_t o = from * E.ncomp + i % E.ncomp;
+      E.emb[o] = __fadd_rn(E.emb[o], E.upd[o]);
+    }
+    all.sync();
   }
 }
 
@@ -1505,17 +1645,6 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-__global__ void ne_apply_kernel(float* emb, const float* upd, const uint32_t* order, int64_t bs, int64_t be,
-                                uint64_t nv, int ncomp) {
-  const int64_t total = (be - bs) * ncomp;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const uint64_t from = order[bs + i / ncomp];
-    if (from >= nv) continue;
-    const uint64_t o = from * ncomp + i % ncomp;
-    emb[o] = __fadd_rn(emb[o], upd[o]);
-  }
-}
-
 inline int grid_for(int64_t work, int threads, int cap) {
   const int64_t b = (work + threads - 1) / threads;
   return (int)(b < 1 ? 1 : (b > cap ? cap : b));
@@ -1547,7 +1676,7 @@ cudaError_t launch_validate_csr(const Csr& g, int32_t* bad, cudaStream_t s) {
 
 cudaError_t launch_seed_labels(int32_t* labels, const int64_t* idx, int64_t count, cudaStream_t s) {
   if (count <= 0) return cudaSuccess;
-  seed_labels_kernel<<<1, 1, 0, s>>>(labels, idx, count);
+  seed_labels_kernel<<<grid_for(count, 256, 1024), 256, 0, s>>>(labels, idx, count);
   return cudaGetLastError();
 }
 
@@ -1851,35 +1980,43 @@ cudaError_t launch_ne_schedule(const float* w, int64_t m, int32_t n_epochs, floa
   return cudaGetLastError();
 }
 
-cudaError_t launch_ne_block(const Csr& g, float* emb, float* upd, const uint32_t* order, int64_t bs, int64_t be,
+namespace {
+template <int MAXD>
+cudaError_t run_ne_epoch(NeEpoch E, int sms, cudaStream_t s) {
+  using Shape = NeShape<MAXD>;
+  const size_t smem = std::max(size_t(Shape::kWarps) * ne_stage_floats(E.ncomp) * 4,
+                               size_t(Shape::kTile) * (2 * (kSlots * E.ncomp + 2) + kSlots) * 4);
+  cudaError_t e = cudaFuncSetAttribute(ne_epoch_kernel<MAXD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  int resident = 0;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, ne_epoch_kernel<MAXD>, Shape::kWarps * 32, smem);
+  if (e != cudaSuccess) return e;
+  if (resident < 1) return cudaErrorLaunchOutOfResources;
+  // a warp to each node of a block, and a CTA an SM at least for the heavy rows
+  const int64_t want = (std::min(E.block, E.g.n) + Shape::kWarps - 1) / Shape::kWarps;
+  const int grid = (int)std::min<int64_t>(std::max<int64_t>(want, sms), int64_t(resident) * sms);
+  // several rows to a warp once every warp has its own
+  const int64_t warps = int64_t(grid) * Shape::kWarps;
+  E.take = (int)std::min<int64_t>(Shape::kRows, (std::min(E.block, E.g.n) + warps - 1) / warps);
+  void* args[] = {&E};
+  return cudaLaunchCooperativeKernel((const void*)ne_epoch_kernel<MAXD>, dim3(grid), dim3(Shape::kWarps * 32), args,
+                                     smem, s);
+}
+}  // namespace
+
+cudaError_t launch_ne_epoch(const Csr& g, float* emb, float* upd, const uint32_t* order, int64_t block,
                             const float* eps, const float* epns, float* eonn, float* eons, uint32_t rng_state,
                             int ncomp, float alpha, uint8_t epoch, float noise, float gamma, float decay,
-                            int apply_decay, int64_t heavy_deg, uint32_t* heavy_rows, int32_t* heavy_count, int sms,
+                            int apply_decay, int64_t heavy_deg, uint32_t* heavy, int32_t* counts, int sms,
                             cudaStream_t s) {
-  const int64_t warps = be - bs;
-  if (warps <= 0) return cudaSuccess;
-  cudaError_t e = cudaMemsetAsync(heavy_count, 0, 4, s);
+  if (g.n <= 0) return cudaSuccess;
+  cudaError_t e = cudaMemsetAsync(counts, 0, kNeCounts * 4, s);
   if (e != cudaSuccess) return e;
-  const HeavyRows heavy{heavy_deg, heavy_rows, heavy_count};
-  const int grid = (int)std::min<int64_t>((warps + kNeWarps - 1) / kNeWarps, 1 << 20);
-  const size_t smem = size_t(kNeWarps) * ne_stage_floats(ncomp) * sizeof(float);
-  const size_t hsmem = heavy_smem_bytes(ncomp);
-  auto run = [&](auto block_kernel, auto heavy_kernel) -> cudaError_t {
-    cudaError_t err = cudaFuncSetAttribute(block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (err != cudaSuccess) return err;
-    block_kernel<<<grid, kNeWarps * 32, smem, s>>>(g, emb, upd, order, bs, be, eps, epns, eonn, eons, rng_state, ncomp,
-                                                   alpha, epoch, noise, gamma, decay, apply_decay, heavy);
-    if ((err = cudaGetLastError()) != cudaSuccess) return err;
-    if ((err = cudaFuncSetAttribute(heavy_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsmem)))
-      return err;
-    heavy_kernel<<<sms * 2, kHeavyWarps * 32, hsmem, s>>>(g, emb, upd, order, eps, epns, eonn, eons, rng_state, ncomp,
-                                                          alpha, epoch, noise, gamma, decay, apply_decay, heavy);
-    return cudaGetLastError();
-  };
-  // narrow rows: more warps per SM (64 registers); wider rows keep their values in registers
-  if (ncomp <= 8) return run(ne_block_kernel<8, 8>, ne_heavy_kernel<8, 2>);
-  if (ncomp <= 16) return run(ne_block_kernel<16, 1>, ne_heavy_kernel<16, 1>);
-  return run(ne_block_kernel<32, 1>, ne_heavy_kernel<32, 1>);
+  const NeEpoch E{g,     emb,   upd,   order, eps,         epns,  eonn,      eons,  ~0ull / (uint64_t)g.n, rng_state, ncomp,
+                  alpha, epoch, noise, gamma, decay,       apply_decay, block, heavy_deg, 1, heavy, counts};
+  if (ncomp <= 8) return run_ne_epoch<8>(E, sms, s);
+  if (ncomp <= 16) return run_ne_epoch<16>(E, sms, s);
+  return run_ne_epoch<32>(E, sms, s);
 }
 
 cudaError_t launch_edge_head(const int64_t* indptr, int64_t n, uint32_t* head, cudaStream_t s) {
@@ -1900,13 +2037,6 @@ cudaError_t launch_ne_hogwild(const Csr& g, const uint32_t* head, float* emb, co
   else
     ne_hogwild_kernel<32><<<grid, 256, 0, s>>>(g, head, emb, eps, epns, eonn, eons, rng_state, ncomp, alpha, epoch,
                                                noise);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_ne_apply(float* emb, const float* upd, const uint32_t* order, int64_t bs, int64_t be, int64_t nv,
-                            int ncomp, cudaStream_t s) {
-  ne_apply_kernel<<<grid_for((be - bs) * ncomp, 256, 4096), 256, 0, s>>>(emb, upd, order, bs, be, (uint64_t)nv,
-                                                                         ncomp);
   return cudaGetLastError();
 }
 

@@ -146,15 +146,14 @@ cudaError_t launch_edge_head(const int64_t* indptr, int64_t n, uint32_t* head, c
 cudaError_t launch_ne_hogwild(const Csr& g, const uint32_t* head, float* emb, const float* eps, const float* epns,
                               float* eonn, float* eons, uint32_t rng_state, int ncomp, float alpha, uint8_t epoch,
                               float noise, int sms, cudaStream_t s);
-// One block of one epoch: nodes order[bs, be), rows of more than heavy_deg
-// edges by one CTA each (heavy_rows holds be - bs ids); then the apply launch.
-cudaError_t launch_ne_block(const Csr& g, float* emb, float* upd, const uint32_t* order, int64_t bs, int64_t be,
+// One reproducible epoch over blocks of `block` nodes of `order`: one cooperative
+// launch.  Rows of more than heavy_deg edges take a CTA each (`heavy` holds n ids).
+constexpr int kNeCounts = 32;  // words of `counts`
+cudaError_t launch_ne_epoch(const Csr& g, float* emb, float* upd, const uint32_t* order, int64_t block,
                             const float* eps, const float* epns, float* eonn, float* eons, uint32_t rng_state,
                             int ncomp, float alpha, uint8_t epoch, float noise, float gamma, float decay,
-                            int apply_decay, int64_t heavy_deg, uint32_t* heavy_rows, int32_t* heavy_count, int sms,
+                            int apply_decay, int64_t heavy_deg, uint32_t* heavy, int32_t* counts, int sms,
                             cudaStream_t s);
-cudaError_t launch_ne_apply(float* emb, const float* upd, const uint32_t* order, int64_t bs, int64_t be, int64_t nv,
-                            int ncomp, cudaStream_t s);
 
 }  // namespace lp
 }  // namespace evoc

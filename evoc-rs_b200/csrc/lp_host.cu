@@ -380,8 +380,8 @@ int node_embedding_dev(evoc_gpu_ctx* ctx, Arena& A, const lp::Csr& g, const floa
   EVOC_TRY(A.get(&maxw, 1), "alloc");
   EVOC_TRY(A.get(&upd, size_t(n * ncomp)), "alloc updates");
   EVOC_TRY(A.get(&d_order, size_t(2 * n)), "alloc node order");
-  EVOC_TRY(A.get(&heavy_rows, size_t(std::max<int64_t>(1024, n / 8))), "alloc heavy rows");
-  EVOC_TRY(A.get(&heavy_count, 1), "alloc");
+  EVOC_TRY(A.get(&heavy_rows, size_t(n)), "alloc heavy rows");
+  EVOC_TRY(A.get(&heavy_count, lp::kNeCounts), "alloc");
   EVOC_TRY(cudaMemsetAsync(upd, 0, size_t(n * ncomp) * 4, s), "memset updates");
   {
     Stage st(ctx, "epochs_per_sample");
@@ -421,15 +421,12 @@ int node_embedding_dev(evoc_gpu_ctx* ctx, Arena& A, const lp::Csr& g, const floa
     }
     if (e == cudaSuccess) e = cudaEventRecord(up[slot], s);
     const float gamma = n_epochs <= 1 ? 1.0f : 0.5f + (float(ep) / float(n_epochs - 1)) * 1.0f;
-    for (int64_t bs = 0; bs < n && e == cudaSuccess; bs += block) {
-      const int64_t be = std::min(n, bs + block);
-      e = lp::launch_ne_block(g, emb, upd, d_order + size_t(slot) * n, bs, be, eps, epns, eonn, eons,
+    if (e == cudaSuccess)
+      e = lp::launch_ne_epoch(g, emb, upd, d_order + size_t(slot) * n, block, eps, epns, eonn, eons,
                               seeds[size_t(ep)], ncomp, alpha, uint8_t(ep), noise, gamma, decay, ep > 0 ? 1 : 0,
-                              be - bs < kSmallBlock ? kHeavyDegreeSmallBlock : kHeavyDegree, heavy_rows,
-                              heavy_count, ctx->sms, s);
-      if (e == cudaSuccess) e = lp::launch_ne_apply(emb, upd, d_order + size_t(slot) * n, bs, be, n, ncomp, s);
-      ctx->launches += 3;
-    }
+                              block < kSmallBlock ? kHeavyDegreeSmallBlock : kHeavyDegree, heavy_rows, heavy_count,
+                              ctx->sms, s);
+    ctx->launches += 1;
     if (e != cudaSuccess) {
       rc = cuda_fail(ctx, e, "node embedding epoch");
       break;
