@@ -254,7 +254,8 @@ __device__ __forceinline__ int64_t block_inclusive(int64_t v, int64_t* part) {
   return warp ? v + part[warp - 1] : v;
 }
 
-__global__ void __launch_bounds__(1024) count_sums_kernel(const int32_t* __restrict__ cnt, int64_t n, int64_t* out) {
+template <class T>
+__global__ void __launch_bounds__(1024) count_sums_kernel(const T* __restrict__ cnt, int64_t n, int64_t* out) {
   __shared__ int64_t part[32];
   const int64_t b0 = int64_t(blockIdx.x) * kScanBlock;
   int64_t s = 0;
@@ -285,11 +286,12 @@ __global__ void __launch_bounds__(1024) scan_sums_kernel(int64_t blocks, int64_t
   }
 }
 
-__global__ void __launch_bounds__(1024) scan_counts_kernel(const int32_t* __restrict__ cnt, int64_t n, int64_t* out) {
+template <class T>
+__global__ void __launch_bounds__(1024) scan_counts_kernel(const T* __restrict__ cnt, int64_t n, int64_t* out) {
   __shared__ int64_t part[32];
   const int64_t b0 = int64_t(blockIdx.x) * kScanBlock, end = scan_end(blockIdx.x, n);
   const int64_t at = b0 + int64_t(threadIdx.x) * kScanItems;
-  int32_t v[kScanItems];
+  T v[kScanItems];
   int64_t s = 0;
 #pragma unroll
   for (int i = 0; i < kScanItems; i++) {
@@ -601,12 +603,21 @@ __global__ void copy_rows_csr_kernel(int64_t n, int k, const int32_t* __restrict
   }
 }
 
-cudaError_t launch_scan_counts(const int32_t* cnt, int64_t n, int64_t* out, cudaStream_t stream) {
+template <class T>
+static cudaError_t scan_counts(const T* cnt, int64_t n, int64_t* out, cudaStream_t stream) {
   const unsigned blocks = unsigned((n + kScanBlock - 1) / kScanBlock);
   count_sums_kernel<<<blocks, 1024, 0, stream>>>(cnt, n, out);
   scan_sums_kernel<<<1, 1024, 0, stream>>>(blocks, n, out);
   scan_counts_kernel<<<blocks, 1024, 0, stream>>>(cnt, n, out);
   return cudaGetLastError();
+}
+
+cudaError_t launch_scan_counts(const int32_t* cnt, int64_t n, int64_t* out, cudaStream_t stream) {
+  return scan_counts(cnt, n, out, stream);
+}
+
+cudaError_t launch_scan_counts(const int64_t* cnt, int64_t n, int64_t* out, cudaStream_t stream) {
+  return scan_counts(cnt, n, out, stream);
 }
 
 cudaError_t launch_smooth_and_membership(const int32_t* idx, const float* dist, int64_t n, int k, float n_neighbors,

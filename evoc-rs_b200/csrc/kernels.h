@@ -315,6 +315,7 @@ cudaError_t launch_fuzzy_union_write(int64_t n, int k, int symmetrize, const Fuz
 namespace evoc {
 // graph.cu: out[0] = 0, out[i+1] = cnt[0] + ... + cnt[i].
 cudaError_t launch_scan_counts(const int32_t* cnt, int64_t n, int64_t* out, cudaStream_t stream);
+cudaError_t launch_scan_counts(const int64_t* cnt, int64_t n, int64_t* out, cudaStream_t stream);
 // jaccard.cu: per-row popcounts of rows of ldw 32-bit words.
 cudaError_t launch_popcount_rows(const void* X, int64_t n, int ldw, int32_t* pc, int sms, cudaStream_t stream);
 // jaccard.cu: the smallest of each 32 popcounts (the last group of what there is).

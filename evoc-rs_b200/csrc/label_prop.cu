@@ -36,6 +36,7 @@
 #include <cub/cub.cuh>
 #include <thrust/iterator/counting_iterator.h>
 
+#include "kernels.h"
 #include "lp.h"
 
 namespace evoc {
@@ -531,30 +532,6 @@ __global__ void reduced_write_kernel(const uint32_t* idx, int64_t m, const uint3
     r_indices[t] = (int32_t)oq[i];
     r_data[t] = fminf(fmaxf(__uint_as_float(osum[i]), 0.0f), 1.0f);
   }
-}
-
-// Exclusive scan of `count` (m entries) into indptr (m + 1), one block.
-__global__ void __launch_bounds__(1024) scan_i64_kernel(const int64_t* count, int64_t m, int64_t* indptr) {
-  __shared__ int64_t part[1024];
-  const int t = threadIdx.x;
-  const int64_t per = (m + 1023) / 1024;
-  const int64_t b = t * per, e = min(m, b + per);
-  int64_t s = 0;
-  for (int64_t i = b; i < e; i++) s += count[i];
-  part[t] = s;
-  __syncthreads();
-  for (int o = 1; o < 1024; o <<= 1) {
-    const int64_t v = t >= o ? part[t - o] : 0;
-    __syncthreads();
-    part[t] += v;
-    __syncthreads();
-  }
-  int64_t run = part[t] - s;
-  for (int64_t i = b; i < e; i++) {
-    indptr[i] = run;
-    run += count[i];
-  }
-  if (t == 1023) indptr[m] = part[1023];
 }
 
 // ------------------------------------------------------------------ hadamard_symmetric
@@ -1868,8 +1845,7 @@ cudaError_t launch_reduce_graph(const Csr& g, const int32_t* part, const float* 
     reduced_write_kernel<<<grid_for(n_red, 256, 8192), 256, 0, s>>>(w.v1, n_red, w.v2, w.v3, r_indices, r_data);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
-  scan_i64_kernel<<<1, 1024, 0, s>>>(w.rcount, n_parts, r_indptr);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  if ((e = launch_scan_counts(w.rcount, n_parts, r_indptr, s)) != cudaSuccess) return e;
   const int64_t nr = n_red;
   return cudaMemcpyAsync(r_nnz, &nr, 8, cudaMemcpyHostToDevice, s);
 }
@@ -1901,8 +1877,7 @@ cudaError_t launch_hadamard_sym(const Csr& g, const ReduceScratch& w, int64_t* s
     e = cub::DeviceScan::ExclusiveSum(w.tmp, tb, w.head, w.pos, (int)g.nnz, s);
     if (e != cudaSuccess) return e;
   }
-  scan_i64_kernel<<<1, 1024, 0, s>>>(w.rcount, g.n, s_indptr);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  if ((e = launch_scan_counts(w.rcount, g.n, s_indptr, s)) != cudaSuccess) return e;
   if (g.nnz > 0) {
     sym_write_kernel<<<grid_for(g.nnz, 256, 8192), 256, 0, s>>>(w.k1, w.v2, w.head, w.pos, g.nnz, s_indices, s_data);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
