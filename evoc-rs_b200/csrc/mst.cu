@@ -398,9 +398,9 @@ __device__ __forceinline__ void warp_walk(const TreeView& t, const float (&q)[P]
 // registers, the first KQ - kq of them below every distance, so the last one
 // is the kq-th nearest whatever kq is.
 //
-// Bound by instructions: one distance is 3 P / 32 of them a point and lane.
-// 300,000 x 7, kq 6: 7.9 ms with a stack and a binary heap per thread,
-// 5.0 ms now, 69 % of the issue slots used.  Padded to 8 dimensions.
+// Bound by instructions: a warp tests a point in 3 P of them, and the union of
+// its lanes' paths is most of their cluster.  300,000 x 7, kq 6: 7.9 ms with a
+// stack and a binary heap per thread, 5.0 ms now, 69 % of the issue slots used.
 template <int P, int KQ>
 __global__ void __launch_bounds__(128) knn_kernel(TreeView t, int kq, float* __restrict__ core,
                                                   int32_t* __restrict__ knn_pos, float* __restrict__ knn_d,
