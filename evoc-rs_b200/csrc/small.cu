@@ -27,6 +27,8 @@ namespace evoc {
 
 namespace {
 constexpr int kWarps = 8;
+constexpr uint32_t kNoKey = 0xffffffffu;   // ordering word of no column
+constexpr uint32_t kLastKey = kNoKey - 1;  // no score's word is above it
 
 template <int MODE>
 __device__ __forceinline__ float score_raw(uint32_t bits, int32_t pa, int32_t pb) {
@@ -35,6 +37,15 @@ __device__ __forceinline__ float score_raw(uint32_t bits, int32_t pa, int32_t pb
     return uni > 0 ? -__fdiv_rn(__int2float_rn(inter), __int2float_rn(uni)) : 0.0f;
   }
   return MODE == kScanInt8 ? -__int2float_rn(int32_t(bits)) : raw_cosine(__uint_as_float(bits));
+}
+
+// Ordering word of a score; a NaN (of a row that holds one) passes no threshold of the scan and is
+// never kept.
+template <int MODE>
+__device__ __forceinline__ uint32_t score_word(uint32_t bits, bool self, int32_t pa, int32_t pb) {
+  if (self) return orderable(-1.0f);
+  if (MODE == kScanHalf && isnan(__uint_as_float(bits))) return kNoKey;
+  return orderable(score_raw<MODE>(bits, pa, pb));
 }
 }  // namespace
 
@@ -60,14 +71,13 @@ select_scores_kernel(const uint32_t* __restrict__ S, int64_t ld, int n_q, int n_
     const int self = q_row0 + q;
     const int32_t pa = MODE == kScanJaccard ? pc[self] : 0;
     auto key_of = [&](int c) {  // ordering word of column c
-      const uint32_t v = s[c];
-      return orderable(c == self ? -1.0f : score_raw<MODE>(v, pa, MODE == kScanJaccard ? pc[c] : 0));
+      return score_word<MODE>(s[c], c == self, pa, MODE == kScanJaccard ? pc[c] : 0);
     };
     // a bound that about 2.5 keep keys reach, and six sampled ones more for the spread
-    uint32_t bound = 0xfffffffeu;
+    uint32_t bound = kLastKey;
     if (n_k > 256) {
       uint32_t v[kSample];
-      uint32_t lo = 0xffffffffu, hi = 0u;
+      uint32_t lo = kNoKey, hi = 0u;
 #pragma unroll
       for (int i = 0; i < kSample; i++) {
         v[i] = key_of(int((int64_t(i * 32 + lane) * n_k) >> 8));
@@ -91,10 +101,10 @@ select_scores_kernel(const uint32_t* __restrict__ S, int64_t ld, int n_q, int n_
           lo = mid + 1;
         }
       }
-      bound = hi;
+      bound = min(hi, kLastKey);
     }
     int m = 0;  // keys within the bound; the first `cap` are listed, in row order
-    uint32_t lo = 0xffffffffu, hi = 0u;
+    uint32_t lo = kNoKey, hi = 0u;
     for (int b = 0; b < n_k; b += 32 * kAhead) {
       uint32_t v[kAhead];
       int32_t pb[MODE == kScanJaccard ? kAhead : 1];
@@ -108,8 +118,7 @@ select_scores_kernel(const uint32_t* __restrict__ S, int64_t ld, int n_q, int n_
       for (int i = 0; i < kAhead; i++) {
         const int c = b + 32 * i + lane;
         const uint32_t o =
-            c < n_k ? orderable(c == self ? -1.0f : score_raw<MODE>(v[i], pa, pb[MODE == kScanJaccard ? i : 0]))
-                    : 0xffffffffu;
+            c < n_k ? score_word<MODE>(v[i], c == self, pa, pb[MODE == kScanJaccard ? i : 0]) : kNoKey;
         const bool in = o <= bound;
         const uint32_t who = __ballot_sync(0xffffffffu, in);
         const int at = m + __popc(who & below);
@@ -122,7 +131,7 @@ select_scores_kernel(const uint32_t* __restrict__ S, int64_t ld, int n_q, int n_
     __syncwarp();
     const bool listed = m >= want && m <= cap;
     lo = __reduce_min_sync(0xffffffffu, lo);
-    hi = listed ? __reduce_max_sync(0xffffffffu, hi) : 0xfffffffeu;
+    hi = listed ? __reduce_max_sync(0xffffffffu, hi) : kLastKey;
     const int len = listed ? m : n_k;  // what the cut is searched in
     auto word = [&](int i) { return listed ? uint32_t(list[i] >> 32) : key_of(i); };
     int upto = len;  // words <= hi
@@ -149,7 +158,7 @@ select_scores_kernel(const uint32_t* __restrict__ S, int64_t ld, int n_q, int n_
     uint32_t worst = 0u;
     for (int b = 0; b < len; b += 32) {  // in row order, so the smaller indices of a tie come first
       const int i = b + lane;
-      const uint32_t o = i < len ? word(i) : 0xffffffffu;
+      const uint32_t o = i < len ? word(i) : kNoKey;
       const uint32_t equal = __ballot_sync(0xffffffffu, o == hi);
       const bool in = o < hi || (o == hi && seen + __popc(equal & below) < ties);
       const uint32_t who = __ballot_sync(0xffffffffu, in);
