@@ -43,9 +43,8 @@ __device__ __forceinline__ float score_raw(uint32_t bits, int32_t pa, int32_t pb
 // never kept.
 template <int MODE>
 __device__ __forceinline__ uint32_t score_word(uint32_t bits, bool self, int32_t pa, int32_t pb) {
-  if (self) return orderable(-1.0f);
-  if (MODE == kScanHalf && isnan(__uint_as_float(bits))) return kNoKey;
-  return orderable(score_raw<MODE>(bits, pa, pb));
+  const uint32_t word = orderable(self ? -1.0f : score_raw<MODE>(bits, pa, pb));
+  return MODE == kScanHalf && !self && isnan(__uint_as_float(bits)) ? kNoKey : word;
 }
 }  // namespace
 
