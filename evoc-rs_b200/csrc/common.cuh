@@ -233,7 +233,8 @@ struct KeyHeap {
 // load-compare-store steps down a path, at 20 registers more.  In the scan the
 // inserts of a warp's 32 rows mostly run one after the other, so their latency
 // paces it: 2,000 x 128 f32 rows at k = 15 scan in 205 us (heap: 287), 50,000 x
-// 200 in 2.97 ms (3.59).
+// 200 in 2.97 ms (3.59).  An insert reads cap / 8 slots, so the set is for few
+// keys: takes_heap (tc_scan.cu) says where the line lies.  At most 65,535 slots.
 struct KeySet {
   uint64_t* h;
   int size;

@@ -7,7 +7,7 @@
 // epilogue read tile t while the MMAs of tile t+1 run.  Nothing of the n x n
 // score matrix is written to HBM: each epilogue thread owns one query row,
 // reads its 256 scores straight from TMEM and offers the few that beat its
-// row threshold to a thread-private key set (common.cuh).
+// row threshold to a thread-private key set or heap (common.cuh).
 //
 // Warp roles (192 threads):
 //   warp 0      TMA producer (one elected lane, no multicast)
@@ -301,6 +301,21 @@ __device__ __forceinline__ uint32_t chunk_mask(const uint32_t (&v)[32], uint32_t
   return ~((f[0] << 24) | (f[1] << 16) | (f[2] << 8) | f[3]);
 }
 
+// A row's kept keys as a binary heap or as a set of eight groups (common.cuh).
+// Four groups of epilogue warps take the heap: the set's registers would not
+// fit.  In global memory the set's keep / 8 slots an insert, each in 32 places
+// a warp, cost more than the heap's log2(keep): 10,000 x 128 int8 at k = 130,
+// 300 and 1,000 7.4, 20.5 and 169 ms (heap: 6.1, 15.7 and 111), f32 at k = 52
+// (130 candidates) 5.65 (4.3) and at 100 (250) 11.0 (7.0).  Binary rows gain
+// by the set up to kBitsSet keys (k = 130, 300 and 1,000: 6.2, 19.0 and 136
+// against 8.5, 20.5 and 122).  Beside two stages in shared memory (84 to 128
+// keys) the two are level at 100 keys and the heap is ahead at 128 (10,000 x
+// 128 int8: 1.57 against 1.64 ms).
+constexpr int kBitsSet = 384;
+template <int MODE, int STAGES, int GROUPS, bool kSmemHeap, bool kList>
+constexpr bool takes_heap =
+    GROUPS == 4 || !kSmemHeap || (STAGES == 2 && GROUPS == 1 && MODE != kModeJaccard && !kList);
+
 // Symmetric mode, mirror side.  The keys for later rows wait in a per-warp
 // shared-memory stage and go to the mailboxes kMirrorStage at a time: one
 // round trip of the global atomics per flush, both halves' atomics issued
@@ -523,7 +538,7 @@ __device__ __forceinline__ bool epilogue_vote(int nthreads, bool ok) {
 }  // namespace
 
 template <int MODE, int STAGES, int GROUPS, bool kSmemHeap, bool kBatch, bool kPair = false, bool kSym = false,
-          bool kList = false>
+          bool kList = false, bool kHeap = takes_heap<MODE, STAGES, GROUPS, kSmemHeap, kList>>
 __global__ void __launch_bounds__(64 + GROUPS * 128, 1)
 tc_scan_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const ScanParams p) {
   using namespace sm100;
@@ -742,8 +757,7 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       // symmetric mode: qg is the scanned row, qd its row of the data set (keys and outputs)
       const int32_t* const perm = kList ? p.lists.perm : p.sym_perm;
       const int32_t qd = kSym || kList ? (valid ? perm[q] : -1) : int32_t(qg);
-      // four groups: a binary heap, the other's registers would not fit
-      std::conditional_t<GROUPS == 4, KeyHeap, KeySet> heap;
+      std::conditional_t<kHeap, KeyHeap, KeySet> heap;
       heap.init(hstore, v.keep);
       if (valid && v.self_mode && group == 0) heap.offer(make_key(-1.0f, qd));
       const int32_t pa = (MODE == kModeJaccard && valid) ? v.pc[qg] : 0;
@@ -951,10 +965,11 @@ bool encode_row_map(CUtensorMap* m, const void* base, int64_t rows, int64_t row_
 size_t tc_scan_smem_bytes() { return smem_bytes(4, 1, 0); }
 
 namespace {
-template <int MODE, int STAGES, int GROUPS, bool kSmemHeap, bool kBatch = false>
+template <int MODE, int STAGES, int GROUPS, bool kSmemHeap, bool kBatch = false,
+          bool kHeap = takes_heap<MODE, STAGES, GROUPS, kSmemHeap, false>>
 cudaError_t launch_variant(const CUtensorMap& ma, const CUtensorMap& mb, const ScanParams& p, int grid, size_t smem,
                            cudaStream_t stream) {
-  auto kern = tc_scan_kernel<MODE, STAGES, GROUPS, kSmemHeap, kBatch>;
+  auto kern = tc_scan_kernel<MODE, STAGES, GROUPS, kSmemHeap, kBatch, false, false, false, kHeap>;
   // The opt-in limit, not `smem`: the launch's shared memory varies with keep,
   // and concurrent callers (serving lanes) must not lower each other's limit
   // between this call and their launch.
@@ -1021,6 +1036,14 @@ bool variant_feasible(int v, int keep, bool has_scratch) {
 }
 
 template <int MODE>
+cudaError_t launch_global(const CUtensorMap& ma, const CUtensorMap& mb, ScanParams p, int grid, cudaStream_t stream) {
+  p.heap_stride = p.keep;
+  if (MODE == kModeJaccard && p.keep <= kBitsSet)
+    return launch_variant<MODE, 4, 1, false, false, MODE != kModeJaccard>(ma, mb, p, grid, smem_bytes(4, 1, 0), stream);
+  return launch_variant<MODE, 4, 1, false>(ma, mb, p, grid, smem_bytes(4, 1, 0), stream);
+}
+
+template <int MODE>
 cudaError_t launch_forced(const CUtensorMap& ma, const CUtensorMap& mb, ScanParams p, int grid, int v,
                           cudaStream_t stream) {
   const int odd = p.keep | 1;
@@ -1040,9 +1063,7 @@ cudaError_t launch_forced(const CUtensorMap& ma, const CUtensorMap& mb, ScanPara
     case 12: return launch_pair<MODE, 5, 1>(ma, mb, p, grid, smem_bytes(5, 1, odd, true), stream);
     case 13: return launch_pair<MODE, 2, 2>(ma, mb, p, grid, smem_bytes(2, 2, odd, true), stream);
     case 14: return launch_variant<MODE, 2, 1, true>(ma, mb, p, grid, smem_bytes(2, 1, odd), stream);
-    default:
-      p.heap_stride = p.keep;
-      return launch_variant<MODE, 4, 1, false>(ma, mb, p, grid, smem_bytes(4, 1, 0), stream);
+    default: return launch_global<MODE>(ma, mb, p, grid, stream);
   }
 }
 
@@ -1077,8 +1098,7 @@ cudaError_t launch_mode(const CUtensorMap& ma, const CUtensorMap& mb, ScanParams
   if (smem_bytes(2, 1, odd) <= SMEM_LIMIT)
     return launch_variant<MODE, 2, 1, true>(ma, mb, p, grid, smem_bytes(2, 1, odd), stream);
   if (!p.scratch) return cudaErrorInvalidValue;
-  p.heap_stride = p.keep;
-  return launch_variant<MODE, 4, 1, false>(ma, mb, p, grid, smem_bytes(4, 1, 0), stream);
+  return launch_global<MODE>(ma, mb, p, grid, stream);
 }
 }  // namespace
 
