@@ -259,7 +259,7 @@ PruneLayout prune_layout(int64_t n, int64_t row_bytes, int64_t xs_bytes) {
   L.attach = take(size_t(piv) * 4);
   L.cells = take(size_t(6 * piv) * 4 + 256);
   L.second = take(size_t(n) * 4);  // the strays' second labels, and their dissimilarities
-  L.raw2 = take(size_t(n) * 4);
+  L.raw2 = take(size_t(n) * 4);    // (binary: then the smallest popcount of each 32 scanned rows)
   L.cuts = take(size_t(piv) * 4);
   L.start = take(size_t(L.segments + 1) * 4);
   L.first = take(size_t(L.groups + 1) * 4);
@@ -415,7 +415,9 @@ int list_scan(evoc_gpu_ctx* ctx, const Job& j, int mode, const void* rows, int64
       EVOC_TRY(evoc::launch_expand_bits(b + L.rows, n, ldp, nbytes, ctx->xb.p, rows_mem, row_bytes, ctx->sms,
                                         ctx->stream),
                "expand bits");
-      ctx->launches += 2;
+      // the place of the strays' second dissimilarities, which have been used
+      EVOC_TRY(evoc::launch_least_popcounts(i32(L.sq), n, i32(L.raw2), ctx->sms, ctx->stream), "popcounts");
+      ctx->launches += 3;
     }
     segments = read_count(ctx, counters + 2, &rc);
     if (rc) return rc;
@@ -450,7 +452,7 @@ int list_scan(evoc_gpu_ctx* ctx, const Job& j, int mode, const void* rows, int64
   }
   Stage st(ctx, stage);
   const evoc::ScanLists lists{ctx->order.as<int32_t>(), i32(L.list), i32(L.len), i32(L.blocks), f(L.seed),
-                              ctx->popc.as<int32_t>(), int(L.groups), L.lg};
+                              ctx->popc.as<int32_t>(), binary ? i32(L.raw2) : nullptr, int(L.groups), L.lg};
   const int grid = ctx->scan_per_block ? int((n + 127) / 128) : scan_grid(ctx, n);
   EVOC_TRY(evoc::launch_tc_scan_list(mode, xs, rows_mem, n, row_bytes, keep, grid, final_mode, dtype, idx, raw, dist,
                                      bound, j.status, ctx->timeout_ns, pc, ctx->stream, half, lists, ctx->delay_ns),

@@ -114,7 +114,8 @@ cudaError_t launch_tc_scan_sym(const void* X, int64_t rows, int64_t n, int64_t r
 // `groups` entries per group, the first len[group] of them; blocks visited as
 // block_order says) and admits only scores reaching seed[row], a dissimilarity
 // no better than the row's keep-th; outputs go to data-set rows.  pc:
-// popcounts in scanned order, pc_rows by data-set row (Jaccard).
+// popcounts in scanned order, pc_rows by data-set row, pc_least the smallest of
+// each 32 scanned rows (Jaccard).
 struct ScanLists {
   const int32_t* perm;
   const int32_t* list;
@@ -122,6 +123,7 @@ struct ScanLists {
   const int32_t* block_order;
   const float* seed;
   const int32_t* pc_rows;
+  const int32_t* pc_least;
   int groups, lg;
 };
 bool tc_scan_list_feasible(int keep);

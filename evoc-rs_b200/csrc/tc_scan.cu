@@ -177,7 +177,9 @@ __device__ __forceinline__ uint32_t raw_threshold(float raw, int32_t pa) {
 // Jaccard: the row's threshold for a chunk whose keys have at least `least`
 // bits.  Without it every row of the query's own cluster passes the bound that
 // only knows pa, and is divided and compared to no end: 250,000 x 1,024 bits,
-// whose clusters keep two thirds of their bits, scanned in 97 ms.
+// whose clusters keep two thirds of their bits, scanned in 97 ms (now 53),
+// and over tile lists, where own clusters are what is left, 60,000 x 1,024 with
+// 100 clusters took 7.2 ms (3.9; the full scan 5.7).
 __device__ __forceinline__ uint32_t chunk_threshold(uint32_t thr, float sim, int32_t pa, int32_t least) {
   const float t = sim / (1.0f + sim) * float(pa + least) * (1.0f - 2e-6f);
   return sim > 0.0f ? uint32_t(max(int32_t(thr), int32_t(floorf(t)))) : thr;
@@ -1256,7 +1258,8 @@ cudaError_t launch_tc_scan_list(int mode, const void* X, int64_t rows, int64_t n
   if ((reinterpret_cast<uintptr_t>(X) & 15) || !lists.perm || !lists.list || !lists.len || !lists.block_order ||
       !lists.seed || !out_idx)
     return cudaErrorInvalidValue;
-  if (mode < kModeHalf || mode > kModeJaccard || (mode == kModeJaccard && (!pc || !lists.pc_rows)))
+  if (mode < kModeHalf || mode > kModeJaccard ||
+      (mode == kModeJaccard && (!pc || !lists.pc_rows || !lists.pc_least)))
     return cudaErrorInvalidValue;
   if (half_type != kHalfF16 && half_type != kHalfBf16) return cudaErrorInvalidValue;
   const int eb = mode == kModeHalf ? 2 : 1;
@@ -1282,6 +1285,7 @@ cudaError_t launch_tc_scan_list(int mode, const void* X, int64_t rows, int64_t n
   p.drain_ns = timeout_ns > kDrainNs ? timeout_ns : kDrainNs;
   p.delay_ns = delay_ns;
   p.pc = pc;
+  p.pc_least = lists.pc_least;
   p.half_type = half_type;
   p.lists = lists;
   if (mode == kModeInt8) return launch_list_mode<kModeInt8>(ma, mb, p, grid, stream);
