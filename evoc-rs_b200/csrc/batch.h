@@ -68,10 +68,11 @@ struct ScanItem {
   int32_t job, qb;
 };
 
-// tc_scan.cu.  Tensor map over `rows` rows of `row_bytes` (a multiple of 128):
-// boxes of 128 bytes x box_rows, 128-byte swizzle.
+// tc_scan.cu.  Tensor map over `rows` rows of `row_bytes` (a multiple of 128),
+// `stride` bytes apart (a multiple of 16; 0: row_bytes): boxes of 128 bytes x
+// box_rows, 128-byte swizzle.
 bool encode_row_map(CUtensorMap* m, const void* base, int64_t rows, int64_t row_bytes, int elem_bytes, int box_rows,
-                    int half_type);
+                    int half_type, int64_t stride = 0);
 
 // tc_scan.cu.  Encodes a request's tensor maps and parameters (self mode:
 // every row is a query and a key).  mode 0: 16-bit float rows (half_type);

@@ -208,9 +208,8 @@ int32_t read_count(evoc_gpu_ctx* ctx, const int32_t* d_count, int* rc) {
   return v;
 }
 
-// Exact self-joins over tile lists (prune.cu): at least kPruneMinRows rows, a
-// pivot per 512, at most 2,048, and as many more for the strays.
-constexpr int64_t kPruneMinRows = 16384;
+// Exact self-joins over tile lists (prune.cu): a pivot per 512 rows, at most
+// 2,048, and as many more for the strays.
 constexpr int64_t kStrayPivots = 2048;
 
 int64_t list_pivots(int64_t n) { return std::max<int64_t>(2, std::min<int64_t>(n / 512, 2048)); }
@@ -268,24 +267,48 @@ PruneLayout prune_layout(int64_t n, int64_t row_bytes, int64_t xs_bytes) {
   return L;
 }
 
-// Whether a whole-graph request may take the lists: enough rows for them to
-// pay (16,384: 1.1 ms against 1.3 for the full scan at 384 features; below,
-// the plan's launches cost more than the scan), heaps in shared memory, rows
-// short enough for the group statistics.
-bool use_lists(int64_t n, int64_t r0, int64_t nq, int64_t keep, int64_t row_elems) {
-  return r0 == 0 && nq == n && n >= kPruneMinRows && keep <= n && evoc::tc_scan_list_feasible(int(keep)) &&
-         row_elems <= 51200;
+// Whether a whole-graph request may take the lists: more query blocks than SMs
+// (up to there the full scan is one round of blocks and the plan costs as much:
+// 17,000 x 96 f32, 20 clusters 0.69 against 0.73 ms, 100 clusters 1.15 against
+// 0.72), twice as many where few keys are kept and the scan is cheap (30,000 x
+// 128 int8 at k = 3 0.53 against 0.44 ms); heaps in shared memory, rows short
+// enough for the group statistics.
+bool use_lists(const evoc_gpu_ctx* ctx, int64_t n, int64_t r0, int64_t nq, int64_t keep, int64_t row_elems) {
+  return r0 == 0 && nq == n && n > int64_t(keep < 8 ? 256 : 128) * ctx->sms && keep <= n &&
+         evoc::tc_scan_list_feasible(int(keep)) && row_elems <= 51200;
 }
 
-// The lists are taken when a quarter of a sample of rows reaches this cosine
-// with its nearest pivot.  With a the cosine of a row and its group's centre,
-// the bound is at least 1 - a^2 and the rows' neighbours score about a^2, and
-// a^2 is about the cosine with a pivot of the same cluster: below a half
-// nothing can be skipped.  Binary rows differ from their centre by single bits,
-// whose number varies from row to row; their bound needs 0.8 (bit rows that
-// keep 0.66, 1,024 bits with a twentieth flipped, skip no tile at all).
-constexpr int64_t kFitSample = 2048;
-constexpr float kFitCosine = 0.5f, kFitCosineBits = 0.8f;
+// The lists are taken when enough rows of a sample are near enough to their
+// nearest pivot.  With a the cosine of a row and its group's centre and g that
+// of two groups' centres, the bound on a row of the other group is at least
+// a^2 g + 1 - a^2 and the row's neighbours score about a^2, so the other group
+// can be skipped from 1 - a^2 < (1 - a^2 g) / 2 on.  a^2 is about the cosine
+// with a pivot of the same cluster and a^2 g the one with the other pivots,
+// whose mean also falls with the share of the rows that can be skipped.  (A
+// cosine of a half with the nearest pivot alone let rows in that share a mean
+// and nothing else: 120,000 x 256 int8 took 8.6 ms, the full scan 7.2.)  Binary
+// rows differ from their centre by single bits, whose number varies from row
+// to row; their bound needs twice as much (bit rows that keep 0.66, 1,024 bits
+// with a twentieth flipped, skip no tile at all).
+//
+// Up to two rounds of query blocks the plan is a third of a f32 scan and more
+// of an integer one, so fewer tiles may be left: rows nearer to their pivot
+// (24,000 x 96 f32, 50 clusters about a common mean: 1.67 against 1.49 ms), and
+// for integer scans, which are cheaper, pivots in most clusters (24,000 x 96
+// int8: 20 clusters 0.61 against 0.76 ms, 50 about a mean 0.95).  Binary rows
+// whose pivots miss most clusters lose at any size (60,000 x 1,024 bits: 300
+// clusters 6.3 against 5.5 ms, 100 3.8 against 5.7).  A sample that declines
+// costs 35 us.
+struct FitRule {
+  float part;    // of the distance to the pivots' mean (1 - cosine) that the nearest pivot's may be
+  float sample;  // share of the sample that must be as near
+};
+FitRule fit_rule(const evoc_gpu_ctx* ctx, int mode, int64_t n) {
+  const bool few = n <= int64_t(256) * ctx->sms;
+  if (mode == evoc::kScanJaccard) return few ? FitRule{0.2f, 0.75f} : FitRule{0.25f, 0.5f};
+  if (!few) return {0.5f, 0.25f};
+  return {0.3f, mode == evoc::kScanInt8 ? 0.75f : 0.25f};
+}
 
 // Plans the lists of a self-join of all rows and scans over them; *taken is
 // false when the rows call for the full scan.  rows: the operand rows in data-set order (binary
@@ -298,13 +321,28 @@ int list_scan(evoc_gpu_ctx* ctx, const Job& j, int mode, const void* rows, int64
   *taken = false;
   const bool binary = mode == evoc::kScanJaccard;
   const int64_t n = j.n, rows_mem = evoc::padded_rows(n);
+  const int gemm = mode == evoc::kScanHalf ? evoc::kScanHalf : evoc::kScanInt8;
+  const int64_t piv1 = list_pivots(n);
+  {
+    Stage st(ctx, "scan_sample");
+    const evoc::Sample sample = evoc::list_sample(n, piv1);
+    EVOC_TRY(ctx->scratch.ensure(evoc::sample_fit_bytes(sample)), "alloc scratch");
+    int32_t* fit = nullptr;
+    const FitRule rule = fit_rule(ctx, mode, n);
+    EVOC_TRY(evoc::launch_sample_fit(gemm, rows, row_bytes, half, sample, rule.part, ctx->scratch.p, &fit, j.status,
+                                     ctx->timeout_ns, ctx->sms, ctx->stream),
+             "sample fit");
+    ctx->launches += gemm == evoc::kScanHalf ? 2 : 3;
+    int rc = EVOC_OK;
+    const int32_t near = read_count(ctx, fit, &rc);
+    if (rc || float(near) < rule.sample * float(sample.rows)) return rc;
+  }
   const PruneLayout L = prune_layout(n, row_bytes, binary ? ldp : row_bytes);
   EVOC_TRY(ctx->prune.ensure(L.total), "alloc tile lists");
+  *taken = true;
   uint8_t* b = ctx->prune.as<uint8_t>();
   auto f = [&](size_t off) { return reinterpret_cast<float*>(b + off); };
   auto i32 = [&](size_t off) { return reinterpret_cast<int32_t*>(b + off); };
-  const int gemm = mode == evoc::kScanHalf ? evoc::kScanHalf : evoc::kScanInt8;
-  const int64_t piv1 = list_pivots(n);
   int64_t piv2 = 0;
   int32_t segments = 0;
   const evoc::Segments seg{i32(L.start), i32(L.first), L.group_rows};
@@ -324,27 +362,12 @@ int list_scan(evoc_gpu_ctx* ctx, const Job& j, int mode, const void* rows, int64
     // counters, then the first pivots' cells (all rows, the closer ones), then every pivot's rows
     // without the strays
     const int64_t piv_max = piv1 + kStrayPivots;
-    int32_t* counters = i32(L.cells);  // close sample rows, strays, segments
+    int32_t* counters = i32(L.cells);  // strays, segments
     float *sum = f(L.cells) + 4, *top_sum = sum + 2 * piv1, *own_sum = sum + 4 * piv1;
     int32_t *cnt = i32(L.cells) + 4 + piv1, *top_cnt = cnt + 2 * piv1, *own_cnt = cnt + 3 * piv1 + piv_max;
     EVOC_TRY(cudaMemsetAsync(b + L.cells, 0, size_t(4 + 4 * piv1 + 2 * piv_max) * 4, ctx->stream), "clear cells");
     EVOC_TRY(ctx->labels.ensure(size_t(n) * 4), "alloc labels");
     int32_t* label = ctx->labels.as<int32_t>();
-    // the sample's rows pass through the place of the scanned rows
-    const int64_t stride = n / kFitSample;
-    EVOC_TRY(evoc::launch_gather_strided_rows(rows, row_bytes, stride, kFitSample, kFitSample, b + L.rows, ctx->sms,
-                                              ctx->stream),
-             "sample rows");
-    rc = nearest_pivots(ctx, b + L.rows, kFitSample, 0, kFitSample, row_bytes, int8, half, ctx->pivots.p, piv1, label,
-                        f(L.seed), j.status);
-    if (rc) return rc;
-    EVOC_TRY(evoc::launch_sample_fit(label, f(L.seed), int(kFitSample), stride, n, int(piv1), sq,
-                                     binary ? kFitCosineBits : kFitCosine, counters, ctx->stream),
-             "sample fit");
-    ctx->launches += 2;
-    const int32_t close = read_count(ctx, counters, &rc);
-    if (rc || close < kFitSample / 4) return rc;
-    *taken = true;
     rc = nearest_pivots(ctx, rows, rows_mem, 0, n, row_bytes, int8, half, ctx->pivots.p, piv1, label, f(L.seed),
                         j.status);
     if (rc) return rc;
@@ -357,10 +380,10 @@ int list_scan(evoc_gpu_ctx* ctx, const Job& j, int mode, const void* rows, int64
                                    ctx->stream),
              "cell fit");
     EVOC_TRY(evoc::launch_strays(label, f(L.seed), n, int(piv1), sq, top_sum, top_cnt, own_sum, own_cnt, strays,
-                                 counters + 1, ctx->sms, ctx->stream),
+                                 counters, ctx->sms, ctx->stream),
              "strays");
     ctx->launches += 3;
-    const int32_t n_strays = read_count(ctx, counters + 1, &rc);
+    const int32_t n_strays = read_count(ctx, counters, &rc);
     if (rc) return rc;
     // their operand rows are gathered in the arena's place for the scanned rows (binary data: packed
     // rows' place, which holds an eighth of the 0/1 rows; strays past that keep their first cell)
@@ -404,7 +427,7 @@ int list_scan(evoc_gpu_ctx* ctx, const Job& j, int mode, const void* rows, int64
     if (rc) return rc;
     EVOC_TRY(evoc::launch_segments(i32(L.rank), f(L.attach), own_sum, own_cnt, int(piv), ctx->cursor.as<int32_t>(),
                                    ctx->hist.as<int32_t>(), n, L.group_rows, int(L.groups), int(L.segments),
-                                   i32(L.cuts), seg, counters + 2, i32(L.group_of), ctx->stream),
+                                   i32(L.cuts), seg, counters + 1, i32(L.group_of), ctx->stream),
              "segments");
     EVOC_TRY(evoc::launch_gather_rows_list(binary ? packed : rows, binary ? ldp : row_bytes, 0,
                                            ctx->order.as<int32_t>(), n, rows_mem, b + L.rows, ctx->sms, ctx->stream),
@@ -419,7 +442,7 @@ int list_scan(evoc_gpu_ctx* ctx, const Job& j, int mode, const void* rows, int64
       EVOC_TRY(evoc::launch_least_popcounts(i32(L.sq), n, i32(L.raw2), ctx->sms, ctx->stream), "popcounts");
       ctx->launches += 3;
     }
-    segments = read_count(ctx, counters + 2, &rc);
+    segments = read_count(ctx, counters + 1, &rc);
     if (rc) return rc;
     if (segments < L.groups || segments > L.segments)
       return fail(ctx, EVOC_ERR_CUDA, "device self-check failed (segments)");
@@ -861,7 +884,7 @@ int run_bf16_rerank(evoc_gpu_ctx* ctx, const evoc_gpu_opts& opts, const Job& j, 
   const int grid = main_scan_grid(ctx, j.nq, int(C), variant);
   EVOC_TRY(ctx->cand.ensure(size_t(j.nq * C) * 4), "alloc candidates");
   const bool sym = use_symmetric(ctx, certify, j.n, j.r0, j.nq, C);
-  bool lists = !sym && use_lists(j.n, j.r0, j.nq, C, ldb);
+  bool lists = !sym && use_lists(ctx, j.n, j.r0, j.nq, C, ldb);
   if (lists) {
     int rc = list_scan(ctx, j, evoc::kScanHalf, ctx->xb.p, ldb * 2, half, int(C), 0, 0, ctx->cand.as<int32_t>(),
                        nullptr, nullptr, certify ? cf(CL.bound) : nullptr, "bf16_scan", &lists);
@@ -934,7 +957,7 @@ int run_bf16_rerank(evoc_gpu_ctx* ctx, const evoc_gpu_opts& opts, const Job& j, 
 }
 
 int run_int8(evoc_gpu_ctx* ctx, const Job& j, int64_t ldb) {
-  if (use_lists(j.n, j.r0, j.nq, j.keff, ldb)) {
+  if (use_lists(ctx, j.n, j.r0, j.nq, j.keff, ldb)) {
     bool taken = false;
     const int rc = list_scan(ctx, j, evoc::kScanInt8, ctx->x.p, ldb, evoc::kHalfF16, j.keff, 1, EVOC_DTYPE_I8, j.idx,
                              j.raw, j.dist, nullptr, "int8_scan", &taken);
@@ -984,7 +1007,7 @@ int run_jaccard_tc(evoc_gpu_ctx* ctx, const Job& j, int64_t ldb, int64_t nbytes)
              "expand bits");
     ctx->launches += 2;
   }
-  if (use_lists(j.n, j.r0, j.nq, j.keff, lde)) {
+  if (use_lists(ctx, j.n, j.r0, j.nq, j.keff, lde)) {
     bool taken = false;
     const int rc = list_scan(ctx, j, evoc::kScanJaccard, ctx->xb.p, lde, evoc::kHalfF16, j.keff, 1, EVOC_DTYPE_U8,
                              j.idx, j.raw, j.dist, nullptr, "jaccard_scan", &taken, ctx->x.p, ldb, nbytes);
@@ -2137,7 +2160,7 @@ void knn_buffer_needs(const evoc_gpu_ctx* ctx, const evoc_gpu_opts& opts, int32_
     if (use_small(ctx, mode, n, keep, -1)) b[kBufScratch] = std::max(b[kBufScratch], small_scan_bytes(n, n));
   };
   auto list_plan = [&](int64_t keep, int64_t row_bytes, int64_t elems, int64_t xs_bytes) {
-    if (!use_lists(n, 0, n, keep, elems)) return;
+    if (!use_lists(ctx, n, 0, n, keep, elems)) return;
     const int64_t piv = list_pivots(n);
     auto at_least = [&](int buf, size_t bytes) { b[buf] = std::max(b[buf], bytes); };
     at_least(kBufPivots, size_t((padded_rows(piv) + kStrayPivots + 256) * row_bytes));
@@ -2145,6 +2168,7 @@ void knn_buffer_needs(const evoc_gpu_ctx* ctx, const evoc_gpu_opts& opts, int32_
     at_least(kBufOrder, size_t(n) * 4);
     at_least(kBufHist, size_t(piv + kStrayPivots) * 4);
     at_least(kBufCursor, size_t(piv + kStrayPivots) * 4);
+    at_least(kBufScratch, sample_fit_bytes(list_sample(n, piv)));
     b[kBufPrune] = prune_layout(n, row_bytes, xs_bytes).total;
   };
   auto nnd = [&]() {

@@ -159,11 +159,19 @@ cudaError_t launch_seeds(int mode, const void* X, int64_t rows_mem, int64_t n, i
                          int half_type, const unsigned int* top, const int32_t* pc, float* seed, int* status,
                          uint64_t timeout_ns, int grid, cudaStream_t stream);
 cudaError_t launch_int8_sq(const void* rows, int64_t row_bytes, int64_t n, int32_t* sq, int sms, cudaStream_t stream);
-// *close += the sampled rows (sample i is row i * stride) whose cosine with their pivot reaches `least`.
-cudaError_t launch_sample_fit(const int32_t* label, const float* raw, int m, int64_t stride, int64_t n, int n_piv,
-                              const int32_t* sq, float least, int32_t* close, cudaStream_t stream);
-// How well rows fit their pivots: per cell sum and count (cleared by the caller) of the cosines.  raw: the
-// pivot scan's dissimilarities; sq: squared norms (null: unit rows), of row map[i] for row i where given;
+// Rows and pivots that tell whether the lists pay: `rows` evenly spaced rows from row `first` on, against
+// `pivots` evenly spaced ones.
+struct Sample {
+  int64_t first, stride, pivot_stride;
+  int rows, pivots;
+};
+Sample list_sample(int64_t n, int64_t n_piv);  // n at least 2,048, n_piv at least 1 and at most n
+size_t sample_fit_bytes(const Sample& s);
+// *fit (in `work`): how many of the sampled rows lie nearer to their nearest pivot than to the pivots'
+// mean, as `part` demands.  mode: kScanHalf or kScanInt8 operand rows.
+cudaError_t launch_sample_fit(int mode, const void* rows, int64_t row_bytes, int half_type, const Sample& s, float part,
+                              void* work, int32_t** fit, int* status, uint64_t timeout_ns, int sms,
+                              cudaStream_t stream);
 // all_sum / all_count (an earlier call's; or null): only rows above their cell's mean.
 cudaError_t launch_cell_fit(const int32_t* label, const float* raw, int64_t n, int n_piv, const int32_t* sq,
                             const int32_t* map, const float* all_sum, const int32_t* all_count, float* sum,

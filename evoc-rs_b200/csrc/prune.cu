@@ -27,8 +27,9 @@
 // then scores strictly below keep keys of the row, so the kept sets are those
 // of the full scan, ties included.
 //
-// Where rows are not alike enough for the bound to skip anything (a sample's
-// cosines with the pivots tell), the full scan runs instead.
+// Where rows are not alike enough for the bound to skip anything, or no more
+// unlike the others than they are alike (a sample's cosines with the pivots
+// tell), the full scan runs instead.
 //
 // Slack.  The products with the centres and the scores the bound is compared
 // with are tensor-core sums: at most e = (L/4 + 2) 2^-21 |x||y| off for 16-bit
@@ -39,6 +40,7 @@
 //
 // Replaces nothing in the reference, which prunes by its RP forest and
 // NN-descent (src/nndescent/float.rs:775-879) without a guarantee.
+#include <algorithm>
 #include <cfloat>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -489,21 +491,26 @@ prim_order_kernel(const float* __restrict__ sim, int64_t ld, int n, int active, 
   }
 }
 
-// Squared norms of int8 rows (row_bytes a multiple of 16), warp per row.
+// A warp's sum of squares of an int8 row (row_bytes a multiple of 16).
+__device__ __forceinline__ int row_sq(const uint8_t* row, int64_t row_bytes, int lane) {
+  const int4* x = reinterpret_cast<const int4*>(row);
+  int s = 0;
+  for (int c = lane; c < row_bytes / 16; c += 32) {
+    const int4 v = x[c];
+    s = __dp4a(v.x, v.x, s);
+    s = __dp4a(v.y, v.y, s);
+    s = __dp4a(v.z, v.z, s);
+    s = __dp4a(v.w, v.w, s);
+  }
+  return __reduce_add_sync(0xffffffffu, s);
+}
+
+// Squared norms of int8 rows, warp per row.
 __global__ void int8_sq_kernel(const uint8_t* __restrict__ rows, int64_t row_bytes, int64_t n, int32_t* __restrict__ sq) {
   const int lane = threadIdx.x & 31;
   const int64_t warps = int64_t(gridDim.x) * (blockDim.x >> 5);
   for (int64_t r = int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); r < n; r += warps) {
-    const int4* x = reinterpret_cast<const int4*>(rows + r * row_bytes);
-    int s = 0;
-    for (int c = lane; c < row_bytes / 16; c += 32) {
-      const int4 v = x[c];
-      s = __dp4a(v.x, v.x, s);
-      s = __dp4a(v.y, v.y, s);
-      s = __dp4a(v.z, v.z, s);
-      s = __dp4a(v.w, v.w, s);
-    }
-    s = __reduce_add_sync(0xffffffffu, s);
+    const int s = row_sq(rows + r * row_bytes, row_bytes, lane);
     if (lane == 0) sq[r] = s;
   }
 }
@@ -519,20 +526,40 @@ __device__ __forceinline__ float pivot_cosine(int64_t i, int32_t label, int n_pi
   return w > 0.0f ? s * rsqrtf(w) : 0.0f;
 }
 
-// Of m sampled rows (sample i is row i * stride) those whose cosine with their
-// pivot reaches `least`.
-__global__ void sample_fit_kernel(const int32_t* __restrict__ label, const float* __restrict__ raw, int m,
-                                  int64_t stride, int64_t n, int n_piv, const int32_t* __restrict__ sq, float least,
-                                  int32_t* __restrict__ close) {
-  int c = 0;
-  for (int i = threadIdx.x; i < m; i += blockDim.x) {
-    const int32_t b = min(max(label[i], 0), n_piv - 1);
-    float s = fmaxf(-raw[i], 0.0f);
-    if (sq) s *= rsqrtf(fmaxf(float(sq[i * stride]) * float(sq[int64_t(b) * n / n_piv]), 1.0f));
-    c += s >= least ? 1 : 0;
+// Squared norms of the sampled rows, then of the sampled pivots (int8 rows), warp per row.
+__global__ void sample_sq_kernel(const uint8_t* __restrict__ rows, int64_t row_bytes, Sample s,
+                                 int32_t* __restrict__ sq) {
+  const int lane = threadIdx.x & 31;
+  const int warps = gridDim.x * (blockDim.x >> 5);
+  for (int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < s.rows + s.pivots; i += warps) {
+    const int64_t r = i < s.rows ? s.first + i * s.stride : (i - s.rows) * s.pivot_stride;
+    const int v = row_sq(rows + r * row_bytes, row_bytes, lane);
+    if (lane == 0) sq[i] = v;
   }
-  c = __reduce_add_sync(0xffffffffu, c);
-  if ((threadIdx.x & 31) == 0) atomicAdd(close, c);
+}
+
+// Counts the sampled rows that the lists may serve, warp per row: with c the
+// cosine with the nearest pivot and b the mean over all pivots (0 at least),
+// those with 1 - c below `part` of 1 - b.
+__global__ void sample_fit_kernel(const float* __restrict__ products, int64_t ld, Sample s,
+                                  const int32_t* __restrict__ sq, float part, int32_t* __restrict__ fit) {
+  const int lane = threadIdx.x & 31;
+  const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (i >= s.rows) return;
+  const float* row = products + i * ld;
+  const float own = sq ? rsqrtf(fmaxf(float(sq[i]), 1.0f)) : 1.0f;  // f32 rows have unit length
+  float most = 0.0f, sum = 0.0f;
+  for (int p = lane; p < s.pivots; p += 32) {
+    const float c = row[p] * own * (sq ? rsqrtf(fmaxf(float(sq[s.rows + p]), 1.0f)) : 1.0f);
+    most = fmaxf(most, c);
+    sum += c;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
+    sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  }
+  if (lane == 0 && 1.0f - most < part * (1.0f - fmaxf(sum / float(s.pivots), 0.0f))) atomicAdd(fit, 1);
 }
 
 // Per cell the sum of its rows' cosines with the pivot and their number; with
@@ -983,10 +1010,58 @@ cudaError_t launch_int8_sq(const void* rows, int64_t row_bytes, int64_t n, int32
   return cudaGetLastError();
 }
 
-cudaError_t launch_sample_fit(const int32_t* label, const float* raw, int m, int64_t stride, int64_t n, int n_piv,
-                              const int32_t* sq, float least, int32_t* close, cudaStream_t stream) {
-  if (m < 1 || (m - 1) * stride >= n) return cudaErrorInvalidValue;
-  sample_fit_kernel<<<1, 1024, 0, stream>>>(label, raw, m, stride, n, n_piv, sq, least, close);
+Sample list_sample(int64_t n, int64_t n_piv) {
+  Sample s{};
+  s.rows = 1024;
+  s.stride = n / s.rows;
+  s.first = s.stride / 2;
+  s.pivots = int(n_piv);
+  s.pivot_stride = n / n_piv;
+  return s;
+}
+
+size_t sample_fit_bytes(const Sample& s) {
+  return size_t(s.rows) * size_t((s.pivots + BN - 1) / BN * BN) * 4 + size_t(s.rows + s.pivots) * 4 + 256;
+}
+
+cudaError_t launch_sample_fit(int mode, const void* rows, int64_t row_bytes, int half_type, const Sample& s, float part,
+                              void* work, int32_t** fit, int* status, uint64_t timeout_ns, int sms,
+                              cudaStream_t stream) {
+  if (row_bytes % KCB || s.rows % BM || s.stride < 1 || s.pivot_stride < 1) return cudaErrorInvalidValue;
+  const bool half = mode == kScanHalf;
+  const int eb = half ? 2 : 1;
+  alignas(64) CUtensorMap ma, mb;
+  if (!encode_row_map(&ma, static_cast<const uint8_t*>(rows) + s.first * row_bytes, s.rows, row_bytes, eb, BM, half_type,
+                      s.stride * row_bytes) ||
+      !encode_row_map(&mb, rows, s.pivots, row_bytes, eb, BN, half_type, s.pivot_stride * row_bytes))
+    return cudaErrorInvalidValue;
+  ProductParams p{};
+  p.rows = s.rows;
+  p.n_ctiles = (s.pivots + BN - 1) / BN;
+  p.n_kchunks = int(row_bytes / KCB);
+  p.half_type = half_type;
+  p.ld = p.n_ctiles * BN;
+  int32_t* counter = static_cast<int32_t*>(work);
+  float* products = reinterpret_cast<float*>(counter + 64);
+  int32_t* sq = half ? nullptr : reinterpret_cast<int32_t*>(products + s.rows * p.ld);
+  p.out = products;
+  p.status = status;
+  p.timeout_ns = timeout_ns;
+  p.drain_ns = timeout_ns > 4000000000ull ? timeout_ns : 4000000000ull;
+  cudaError_t e = cudaMemsetAsync(counter, 0, 4, stream);
+  if (e != cudaSuccess) return e;
+  if (sq) sample_sq_kernel<<<sms * 2, 256, 0, stream>>>(static_cast<const uint8_t*>(rows), row_bytes, s, sq);
+  const int64_t items = s.rows / BM * p.n_ctiles;
+  auto go = [&](auto kern) {
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmem));
+    if (e != cudaSuccess) return e;
+    kern<<<unsigned(std::min<int64_t>(items, sms)), 192, kSmem, stream>>>(ma, mb, p);
+    return cudaGetLastError();
+  };
+  e = half ? go(centre_product_kernel<false, true>) : go(centre_product_kernel<true, true>);
+  if (e != cudaSuccess) return e;
+  sample_fit_kernel<<<(s.rows + 7) / 8, 256, 0, stream>>>(products, p.ld, s, sq, part, counter);
+  *fit = counter;
   return cudaGetLastError();
 }
 

@@ -946,13 +946,12 @@ PFN_cuTensorMapEncodeTiled_v12000 get_encode() {
 
 }  // namespace
 
-// 2-D map over `rows` rows of `row_bytes` (a multiple of 128); box = 128 bytes x box_rows.
 bool encode_row_map(CUtensorMap* m, const void* base, int64_t rows, int64_t row_bytes, int elem_bytes, int box_rows,
-                    int half_type) {
+                    int half_type, int64_t stride) {
   auto enc = get_encode();
   if (!enc) return false;
   const cuuint64_t dims[2] = {cuuint64_t(row_bytes / elem_bytes), cuuint64_t(rows)};
-  const cuuint64_t strides[1] = {cuuint64_t(row_bytes)};
+  const cuuint64_t strides[1] = {cuuint64_t(stride ? stride : row_bytes)};
   const cuuint32_t box[2] = {cuuint32_t(KCB / elem_bytes), cuuint32_t(box_rows)};
   const cuuint32_t estr[2] = {1, 1};
   const CUtensorMapDataType dt = elem_bytes == 1          ? CU_TENSOR_MAP_DATA_TYPE_UINT8

@@ -10,7 +10,7 @@ from evoc import _lib
 
 pytestmark = pytest.mark.gpu
 
-ROWS = 40000  # of any type above the smallest whole graph over lists
+ROWS = 40000  # above the smallest whole graph over lists, whatever the type and k
 
 
 def graph(x, k, form=_lib.FORM_AUTO, rows=None, scan_type=0, certify=1):
