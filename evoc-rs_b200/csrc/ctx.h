@@ -16,6 +16,7 @@ namespace evoc {
 struct DevBuf {
   void* p = nullptr;
   size_t bytes = 0;
+  DevBuf* spare = nullptr;  // freed when an allocation fails, which is then tried again
   cudaError_t ensure(size_t want) {
     if (want <= bytes) return cudaSuccess;
     if (p) cudaFree(p);
@@ -23,12 +24,23 @@ struct DevBuf {
     bytes = 0;
     size_t grow = want + want / 8;
     cudaError_t e = cudaMalloc(&p, grow);
+    if (e == cudaErrorMemoryAllocation && spare && spare->p) {
+      cudaGetLastError();
+      spare->release();  // waits for the kernels that use it
+      e = cudaMalloc(&p, grow);
+    }
     if (e != cudaSuccess) {
       p = nullptr;
       return e;
     }
     bytes = grow;
     return cudaSuccess;
+  }
+  // ensure() for what the call can do without: false, and no error left behind, when there is no room.
+  bool room(size_t want) {
+    if (ensure(want) == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
   }
   void release() {
     if (p) cudaFree(p);
@@ -72,7 +84,13 @@ struct evoc_gpu_ctx {
   evoc::DevBuf sym;
   int64_t sym_min_rows = 0;
   int64_t sym_sample = 0, sym_cap = 0, sym_max_offers = 0, sym_overflow = 0;
-  evoc::DevBuf prune;  // exact self-joins over tile lists (prune.cu): rows in scanned order, centres, lists
+  // Exact self-joins over tile lists (prune.cu): rows in scanned order, centres,
+  // lists.  Nothing needs it once a call's list scan is queued, so every other
+  // allocation of the context may have it (DevBuf::spare), and a call that
+  // leaves it larger than kKeepLists gives it back.
+  evoc::DevBuf prune;
+  static constexpr size_t kKeepLists = size_t(4) << 30;
+  bool lean = false;  // plain scans only, without the memory of lists and small forms (a server short of budget)
   evoc::DevBuf batch_ws, batch_tab;  // batches: per-request work arena, device tables
   void* batch_host = nullptr;  // pinned staging of the tables
   size_t batch_host_bytes = 0;
@@ -101,6 +119,13 @@ struct evoc_gpu_ctx {
   // Stream-ordered pool of the label-propagation / embedding calls; it keeps
   // freed blocks (release threshold = max) so repeated calls do not remap.
   cudaMemPool_t lp_pool = nullptr;
+
+  evoc_gpu_ctx() {
+    for (evoc::DevBuf* b : {&x, &scratch, &norms, &flag, &out_idx, &out_raw, &out_dist, &xb, &cand, &labels, &order,
+                            &hist, &cursor, &pivots, &popc, &g_idx, &g_dist, &g_sigma, &g_rho, &g_indptr, &g_indices,
+                            &g_data, &g_work, &nnd_work, &cert, &repair, &sym, &batch_ws, &batch_tab})
+      b->spare = &prune;
+  }
 };
 
 namespace evoc {
@@ -124,6 +149,21 @@ inline int cuda_fail(evoc_gpu_ctx* ctx, cudaError_t e, const char* where) {
       if (_e != cudaSuccess) return cuda_fail(ctx, _e, where); \
     }                                                        \
   } while (0)
+
+// `count` words of T from the context's pool, freed on its stream by the caller.
+template <class T>
+inline cudaError_t pool_get(evoc_gpu_ctx* ctx, T** out, size_t count) {
+  void* p = nullptr;
+  const size_t bytes = (count < 1 ? 1 : count) * sizeof(T);
+  cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, ctx->lp_pool, ctx->stream);
+  if (e == cudaErrorMemoryAllocation && ctx->prune.p) {
+    cudaGetLastError();
+    ctx->prune.release();
+    e = cudaMallocFromPoolAsync(&p, bytes, ctx->lp_pool, ctx->stream);
+  }
+  *out = static_cast<T*>(p);
+  return e;
+}
 
 // Records CUDA events around one stage on the context's stream when profiling.
 struct Stage {

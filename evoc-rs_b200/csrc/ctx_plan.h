@@ -43,9 +43,9 @@ struct CtxSizes {
 
 // Bytes each buffer must hold for evoc_gpu_knn_graph(ctx, opts, dtype, ., n,
 // dim, k, ...) with buffers_on_device = 1 and all rows as queries: the sizes
-// the form runners pass to DevBuf::ensure.
+// the form runners pass to DevBuf::ensure; lean: on a context with ctx->lean set.
 void knn_buffer_needs(const evoc_gpu_ctx* ctx, const evoc_gpu_opts& opts, int32_t dtype, int64_t n, int64_t dim,
-                      int32_t k, CtxSizes* need);
+                      int32_t k, bool lean, CtxSizes* need);
 
 // The buffers evoc_gpu_knn_graph_batch needs for these requests (all other
 // entries zero).  Returns false when the batch path does not take them

@@ -104,8 +104,13 @@ int main_scan_grid(const evoc_gpu_ctx* ctx, int64_t n_q, int keep, int variant) 
 // Whether a request's scan takes the small form (small.cu): few enough rows,
 // no tuned variant, no delayed producer (a test's).
 bool use_small(const evoc_gpu_ctx* ctx, int mode, int64_t n, int64_t keep, int variant) {
-  return variant < 0 && ctx->delay_ns == 0 &&
+  return variant < 0 && ctx->delay_ns == 0 && !ctx->lean &&
          evoc::small_scan_feasible(mode, n, int(std::min<int64_t>(keep, 1 << 20)));
+}
+
+// The same with room for its scores.
+bool take_small(evoc_gpu_ctx* ctx, int mode, int64_t n, int64_t nq, int64_t keep, int variant) {
+  return use_small(ctx, mode, n, keep, variant) && ctx->scratch.room(evoc::small_scan_bytes(nq, n));
 }
 
 // One kNN request: all n rows are keys; query rows r0 .. r0+nq-1 are output rows 0 .. nq-1.
@@ -274,7 +279,7 @@ PruneLayout prune_layout(int64_t n, int64_t row_bytes, int64_t xs_bytes) {
 // 128 int8 at k = 3 0.53 against 0.44 ms); heaps in shared memory, rows short
 // enough for the group statistics.
 bool use_lists(const evoc_gpu_ctx* ctx, int64_t n, int64_t r0, int64_t nq, int64_t keep, int64_t row_elems) {
-  return r0 == 0 && nq == n && n > int64_t(keep < 8 ? 256 : 128) * ctx->sms && keep <= n &&
+  return !ctx->lean && r0 == 0 && nq == n && n > int64_t(keep < 8 ? 256 : 128) * ctx->sms && keep <= n &&
          evoc::tc_scan_list_feasible(int(keep)) && row_elems <= 51200;
 }
 
@@ -326,7 +331,7 @@ int list_scan(evoc_gpu_ctx* ctx, const Job& j, int mode, const void* rows, int64
   {
     Stage st(ctx, "scan_sample");
     const evoc::Sample sample = evoc::list_sample(n, piv1);
-    EVOC_TRY(ctx->scratch.ensure(evoc::sample_fit_bytes(sample)), "alloc scratch");
+    if (!ctx->scratch.room(evoc::sample_fit_bytes(sample))) return EVOC_OK;
     int32_t* fit = nullptr;
     const FitRule rule = fit_rule(ctx, mode, n);
     EVOC_TRY(evoc::launch_sample_fit(gemm, rows, row_bytes, half, sample, rule.part, ctx->scratch.p, &fit, j.status,
@@ -338,7 +343,14 @@ int list_scan(evoc_gpu_ctx* ctx, const Job& j, int mode, const void* rows, int64
     if (rc || float(near) < rule.sample * float(sample.rows)) return rc;
   }
   const PruneLayout L = prune_layout(n, row_bytes, binary ? ldp : row_bytes);
-  EVOC_TRY(ctx->prune.ensure(L.total), "alloc tile lists");
+  // All the memory of the lists now: where there is none the full scan does without, and from here
+  // on no allocation takes the arena away.
+  const int64_t piv_max = piv1 + kStrayPivots;
+  if (!ctx->labels.room(size_t(n) * 4) || !ctx->order.room(size_t(n) * 4) || !ctx->hist.room(size_t(piv_max) * 4) ||
+      !ctx->cursor.room(size_t(piv_max) * 4) ||
+      !ctx->pivots.room(size_t((evoc::padded_rows(piv1) + kStrayPivots + 256) * row_bytes)) ||
+      !ctx->prune.room(L.total))
+    return EVOC_OK;
   *taken = true;
   uint8_t* b = ctx->prune.as<uint8_t>();
   auto f = [&](size_t off) { return reinterpret_cast<float*>(b + off); };
@@ -361,17 +373,14 @@ int list_scan(evoc_gpu_ctx* ctx, const Job& j, int mode, const void* rows, int64
     }
     // counters, then the first pivots' cells (all rows, the closer ones), then every pivot's rows
     // without the strays
-    const int64_t piv_max = piv1 + kStrayPivots;
     int32_t* counters = i32(L.cells);  // strays, segments
     float *sum = f(L.cells) + 4, *top_sum = sum + 2 * piv1, *own_sum = sum + 4 * piv1;
     int32_t *cnt = i32(L.cells) + 4 + piv1, *top_cnt = cnt + 2 * piv1, *own_cnt = cnt + 3 * piv1 + piv_max;
     EVOC_TRY(cudaMemsetAsync(b + L.cells, 0, size_t(4 + 4 * piv1 + 2 * piv_max) * 4, ctx->stream), "clear cells");
-    EVOC_TRY(ctx->labels.ensure(size_t(n) * 4), "alloc labels");
     int32_t* label = ctx->labels.as<int32_t>();
     rc = nearest_pivots(ctx, rows, rows_mem, 0, n, row_bytes, int8, half, ctx->pivots.p, piv1, label, f(L.seed),
                         j.status);
     if (rc) return rc;
-    EVOC_TRY(ctx->order.ensure(size_t(n) * 4), "alloc order");
     int32_t* strays = ctx->order.as<int32_t>();  // until the order is known
     EVOC_TRY(evoc::launch_cell_fit(label, f(L.seed), n, int(piv1), sq, nullptr, nullptr, nullptr, sum, cnt, ctx->sms,
                                    ctx->stream),
@@ -893,9 +902,8 @@ int run_bf16_rerank(evoc_gpu_ctx* ctx, const evoc_gpu_opts& opts, const Job& j, 
   if (sym) {
     int rc = symmetric_scan(ctx, j, half, ldb, rows, C, cf(CL.bound), cf(CL.hnorm), maxes);
     if (rc) return rc;
-  } else if (!lists && use_small(ctx, evoc::kScanHalf, j.n, C, variant)) {
+  } else if (!lists && take_small(ctx, evoc::kScanHalf, j.n, j.nq, C, variant)) {
     Stage st(ctx, "bf16_scan");
-    EVOC_TRY(ctx->scratch.ensure(evoc::small_scan_bytes(j.nq, j.n)), "alloc scratch");
     EVOC_TRY(evoc::launch_small_scan(evoc::kScanHalf, ctx->xb.p, rows, j.n, j.r0, j.nq, ldb * 2, int(C), 0, 0,
                                      ctx->scratch.p, ctx->cand.as<int32_t>(), nullptr, nullptr,
                                      certify ? cf(CL.bound) : nullptr, j.status, ctx->timeout_ns, nullptr, half,
@@ -967,8 +975,7 @@ int run_int8(evoc_gpu_ctx* ctx, const Job& j, int64_t ldb) {
   const int variant = tuned_variant(ctx, evoc::kScanInt8, j.keff, ldb, j.n);
   const int grid = main_scan_grid(ctx, j.nq, j.keff, variant);
   const int64_t rows = evoc::padded_rows(j.n);
-  if (use_small(ctx, evoc::kScanInt8, j.n, j.keff, variant)) {
-    EVOC_TRY(ctx->scratch.ensure(evoc::small_scan_bytes(j.nq, j.n)), "alloc scratch");
+  if (take_small(ctx, evoc::kScanInt8, j.n, j.nq, j.keff, variant)) {
     EVOC_TRY(evoc::launch_small_scan(evoc::kScanInt8, ctx->x.p, rows, j.n, j.r0, j.nq, ldb, j.keff, 1, EVOC_DTYPE_I8,
                                      ctx->scratch.p, j.idx, j.raw, j.dist, nullptr, j.status, ctx->timeout_ns, nullptr,
                                      evoc::kHalfF16, ctx->sms, ctx->stream),
@@ -1015,8 +1022,7 @@ int run_jaccard_tc(evoc_gpu_ctx* ctx, const Job& j, int64_t ldb, int64_t nbytes)
   }
   Stage st(ctx, "jaccard_scan");
   const int variant = tuned_variant(ctx, evoc::kScanJaccard, j.keff, lde, j.n);
-  if (use_small(ctx, evoc::kScanJaccard, j.n, j.keff, variant)) {
-    EVOC_TRY(ctx->scratch.ensure(evoc::small_scan_bytes(j.nq, j.n)), "alloc scratch");
+  if (take_small(ctx, evoc::kScanJaccard, j.n, j.nq, j.keff, variant)) {
     EVOC_TRY(evoc::launch_small_scan(evoc::kScanJaccard, ctx->xb.p, rows, j.n, j.r0, j.nq, lde, j.keff, 1,
                                      EVOC_DTYPE_U8, ctx->scratch.p, j.idx, j.raw, j.dist, nullptr, j.status,
                                      ctx->timeout_ns, ctx->popc.as<int32_t>(), evoc::kHalfF16, ctx->sms, ctx->stream),
@@ -1442,6 +1448,7 @@ int knn_impl(evoc_gpu_ctx* ctx, const evoc_gpu_opts* opts_in, int32_t dtype, con
   EVOC_TRY(cudaMemcpyAsync(flags, d_flags, sizeof(flags), cudaMemcpyDeviceToHost, ctx->stream), "read status");
   total.end();
   EVOC_TRY(cudaStreamSynchronize(ctx->stream), "knn_graph");
+  if (ctx->prune.bytes > evoc_gpu_ctx::kKeepLists) ctx->prune.release();
   if (flags[1] == evoc::kStatusBadOrder || flags[1] == evoc::kStatusBadCandidate)
     return fail(ctx, EVOC_ERR_CUDA, "device self-check failed (code " + std::to_string(flags[1]) + ")");
   if (flags[1] != 0)
@@ -2139,7 +2146,7 @@ namespace evoc {
 // whole-graph request with device-resident outputs.  A form that fails its
 // own checks (k or candidate limits) allocates no more than listed here.
 void knn_buffer_needs(const evoc_gpu_ctx* ctx, const evoc_gpu_opts& opts, int32_t dtype, int64_t n, int64_t dim,
-                      int32_t k, CtxSizes* need) {
+                      int32_t k, bool lean, CtxSizes* need) {
   *need = CtxSizes{};
   size_t* b = need->b;
   const int64_t keff = std::max<int64_t>(1, std::min<int64_t>(k, n - 1));
@@ -2157,10 +2164,10 @@ void knn_buffer_needs(const evoc_gpu_ctx* ctx, const evoc_gpu_opts& opts, int32_
   };
   auto scratch_plan = [&](int mode, int64_t keep) {  // the scan's heaps, or the small form's scores
     b[kBufScratch] = size_t(grid) * 256 * size_t(keep) * 8;
-    if (use_small(ctx, mode, n, keep, -1)) b[kBufScratch] = std::max(b[kBufScratch], small_scan_bytes(n, n));
+    if (!lean && use_small(ctx, mode, n, keep, -1)) b[kBufScratch] = std::max(b[kBufScratch], small_scan_bytes(n, n));
   };
   auto list_plan = [&](int64_t keep, int64_t row_bytes, int64_t elems, int64_t xs_bytes) {
-    if (!use_lists(ctx, n, 0, n, keep, elems)) return;
+    if (lean || !use_lists(ctx, n, 0, n, keep, elems)) return;
     const int64_t piv = list_pivots(n);
     auto at_least = [&](int buf, size_t bytes) { b[buf] = std::max(b[buf], bytes); };
     at_least(kBufPivots, size_t((padded_rows(piv) + kStrayPivots + 256) * row_bytes));

@@ -156,21 +156,17 @@ struct Mt {
 // ------------------------------------------------------------------ stream-ordered device buffers
 
 struct Arena {
-  cudaStream_t s;
-  cudaMemPool_t pool;
+  evoc_gpu_ctx* ctx;
   std::vector<void*> ptrs;
-  explicit Arena(evoc_gpu_ctx* ctx) : s(ctx->stream), pool(ctx->lp_pool) {}
+  explicit Arena(evoc_gpu_ctx* c) : ctx(c) {}
   ~Arena() {
-    for (void* p : ptrs) cudaFreeAsync(p, s);
+    for (void* p : ptrs) cudaFreeAsync(p, ctx->stream);
   }
   template <class T>
   cudaError_t get(T** out, size_t count) {
-    void* p = nullptr;
-    cudaError_t e = cudaMallocFromPoolAsync(&p, std::max<size_t>(count, 1) * sizeof(T), pool, s);
-    if (e != cudaSuccess) return e;
-    ptrs.push_back(p);
-    *out = static_cast<T*>(p);
-    return cudaSuccess;
+    const cudaError_t e = evoc::pool_get(ctx, out, count);
+    if (e == cudaSuccess) ptrs.push_back(*out);
+    return e;
   }
 };
 

@@ -869,21 +869,17 @@ __global__ void scatter_core_kernel(int64_t n, const int32_t* __restrict__ order
 // ------------------------------------------------------------------ host
 
 struct Arena {
-  cudaStream_t s;
-  cudaMemPool_t pool;
+  evoc_gpu_ctx* ctx;
   std::vector<void*> ptrs;
-  Arena(cudaStream_t st, cudaMemPool_t pl) : s(st), pool(pl) {}
+  explicit Arena(evoc_gpu_ctx* c) : ctx(c) {}
   ~Arena() {
-    for (void* p : ptrs) cudaFreeAsync(p, s);
+    for (void* p : ptrs) cudaFreeAsync(p, ctx->stream);
   }
   template <class T>
   cudaError_t get(T** out, size_t count) {
-    void* p = nullptr;
-    cudaError_t e = cudaMallocFromPoolAsync(&p, std::max<size_t>(count, 1) * sizeof(T), pool, s);
-    if (e != cudaSuccess) return e;
-    ptrs.push_back(p);
-    *out = static_cast<T*>(p);
-    return cudaSuccess;
+    const cudaError_t e = pool_get(ctx, out, count);
+    if (e == cudaSuccess) ptrs.push_back(*out);
+    return e;
   }
 };
 
@@ -1073,7 +1069,7 @@ int boruvka_impl(evoc_gpu_ctx* ctx, const float* data, int64_t n, int32_t dim, i
   Stage total(ctx, "total");
   int rc = EVOC_OK;
   {
-    Arena A(ctx->stream, ctx->lp_pool);
+    Arena A(ctx);
     const float* d_x = data;
     float *d_edges = out_edges, *d_core = out_core;
     if (!on_dev) {

@@ -67,6 +67,8 @@ struct Job {
   int64_t row_bytes_total = 0;  // n*dim*size(dtype) when the server copies the rows in
   int64_t out_bytes = 0;        // n*k_eff*8
   evoc::CtxSizes need;          // context buffers the request needs alone
+  evoc::CtxSizes need_lean;     // the same without tile lists and small forms
+  bool lean = false;            // admitted with need_lean
   bool batch_ok = false;        // small enough for a multi-request batch
   int32_t form = 0;             // resolved form
   double work = 0.0;            // 2 n^2 dim: the scan's operations
@@ -205,6 +207,7 @@ void run_work(evoc_gpu_server* s, int lane, const std::vector<Job*>& group, bool
   cudaStream_t st = small ? s->urgent[size_t(lane)] : s->streams[size_t(lane)];
   ctx->stream = st;  // the lane's previous call left its streams idle
   ctx->scan_per_block = !small;
+  ctx->lean = !batch && group.front()->lean;
   nvtxRangePushA(batch ? "evoc_batch" : "evoc_job");
   const size_t m = group.size();
   int rc = EVOC_OK;
@@ -389,9 +392,15 @@ void worker(evoc_gpu_server* s, int lane) {
           batch = true;
           break;
         }
-        const evoc::CtxSizes grown = evoc::grown_sizes(mine, j->need);
-        const int64_t grow = int64_t(grown.total()) - int64_t(mine.total());
-        const int64_t need = j->row_bytes_total + j->out_bytes + grow;
+        // With the memory of the faster scans where the budget has it, else without.
+        evoc::CtxSizes grown;
+        int64_t need = 0;
+        for (const bool lean : {false, true}) {
+          grown = evoc::grown_sizes(mine, lean ? j->need_lean : j->need);
+          need = j->row_bytes_total + j->out_bytes + int64_t(grown.total()) - int64_t(mine.total());
+          j->lean = lean;
+          if (s->in_use + need <= s->budget) break;
+        }
         if (s->in_use + need <= s->budget) {
           if (it != s->pending.begin() && !(small_only && s->pending.front()->n >= kUrgentRows))
             s->pending.front()->skipped++;
@@ -410,7 +419,7 @@ void worker(evoc_gpu_server* s, int lane) {
       // out gives them back.
       if (!s->pending.empty() && mine.total() > 0) {
         const Job* head = s->pending.front().get();
-        const int64_t alone = int64_t(evoc::grown_sizes(evoc::CtxSizes{}, head->need).total());
+        const int64_t alone = int64_t(evoc::grown_sizes(evoc::CtxSizes{}, head->need_lean).total());
         if (s->in_use - int64_t(mine.total()) + head->row_bytes_total + head->out_bytes + alone <= s->budget) {
           trim = true;
           break;
@@ -612,7 +621,8 @@ int evoc_gpu_server_submit(evoc_gpu_server* s, const evoc_gpu_opts* opts, int32_
   j->src_on_device = j->opts.buffers_on_device != 0;
   j->row_bytes_total = j->src_on_device ? 0 : in_bytes;
   j->out_bytes = n * int64_t(j->keff) * 8;
-  evoc::knn_buffer_needs(s->ctxs[0], j->opts, dtype, n, dim, k, &j->need);
+  evoc::knn_buffer_needs(s->ctxs[0], j->opts, dtype, n, dim, k, false, &j->need);
+  evoc::knn_buffer_needs(s->ctxs[0], j->opts, dtype, n, dim, k, true, &j->need_lean);
   j->form = j->opts.form == EVOC_FORM_AUTO
                 ? (dtype == EVOC_DTYPE_F32 ? EVOC_FORM_BF16_RERANK : EVOC_FORM_EXACT_INT)
                 : j->opts.form;
@@ -623,7 +633,7 @@ int evoc_gpu_server_submit(evoc_gpu_server* s, const evoc_gpu_opts* opts, int32_
     // (the batched forms do not read the tau seed)
     j->batch_ok = n <= kBatchRows && evoc::batch_buffer_needs(j->opts, dtype, 1, &n1, &d1, k, &bneed);
   }
-  const int64_t alone = int64_t(evoc::grown_sizes(evoc::CtxSizes{}, j->need).total());
+  const int64_t alone = int64_t(evoc::grown_sizes(evoc::CtxSizes{}, j->need_lean).total());
   if (j->row_bytes_total + j->out_bytes + alone > s->budget) {
     std::lock_guard<std::mutex> lock(s->mu);
     s->rejected++;
@@ -660,7 +670,7 @@ int evoc_gpu_server_request_bytes(evoc_gpu_server* s, const evoc_gpu_opts* opts,
   }
   const int64_t keff = std::max<int64_t>(1, std::min<int64_t>(k, n - 1));
   evoc::CtxSizes need;
-  evoc::knn_buffer_needs(s->ctxs[0], o, dtype, n, dim, k, &need);
+  evoc::knn_buffer_needs(s->ctxs[0], o, dtype, n, dim, k, true, &need);
   if (resident) *resident = (o.buffers_on_device ? 0 : n * dim * elem_size(dtype)) + n * keff * 8;
   if (workspace) *workspace = int64_t(evoc::grown_sizes(evoc::CtxSizes{}, need).total());
   return EVOC_OK;

@@ -493,7 +493,8 @@ int evoc_gpu_knn_f32_noalloc(const float* rows, int64_t n, int64_t ld, int32_t k
  * scratch), so several requests are on the device at once.  A lane admits the
  * oldest pending request that fits the budget: n*dim*size(dtype) for the rows
  * + n*k_eff*8 for the graph + what the lane's buffers must grow by for that
- * shape (lane buffers are kept between requests and counted once; an idle lane
+ * shape, with the memory of tile lists and of the small form where the budget
+ * has it and without where not (lane buffers are kept between requests and counted once; an idle lane
  * frees them when they alone keep the oldest request out).  A request passed
  * over 16 times by later ones is admitted next.  Under backlog -- at least 4
  * compatible small requests pending (f32 with the BF16+rerank form or i8 with
@@ -565,8 +566,8 @@ int evoc_gpu_server_submit(evoc_gpu_server* server, const evoc_gpu_opts* opts, i
                            int64_t n, int64_t dim, int32_t k, const int64_t* rng_state, int32_t flags,
                            int64_t* job_id);
 /* Bytes a request is admitted against: *resident = rows (unless on the
- * device) + graph; *workspace = lane buffers it needs on a lane that holds
- * none.  A request fits an otherwise empty server when their sum is at most
+ * device) + graph; *workspace = lane buffers it cannot do without on a lane
+ * that holds none.  A request fits an otherwise empty server when their sum is at most
  * the budget. */
 int evoc_gpu_server_request_bytes(evoc_gpu_server* server, const evoc_gpu_opts* opts, int32_t dtype, int64_t n,
                                   int64_t dim, int32_t k, int64_t* resident, int64_t* workspace);
