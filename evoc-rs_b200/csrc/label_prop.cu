@@ -1956,12 +1956,22 @@ cudaError_t launch_ne_schedule(const float* w, int64_t m, int32_t n_epochs, floa
 }
 
 namespace {
+// Shared memory of a CTA: the warps' staging, or a heavy row's two tiles.
+template <int MAXD>
+size_t ne_smem(int ncomp) {
+  using Shape = NeShape<MAXD>;
+  return std::max(size_t(Shape::kWarps) * ne_stage_floats(ncomp) * 4,
+                  size_t(Shape::kTile) * (2 * (kSlots * ncomp + 2) + kSlots) * 4);
+}
+
 template <int MAXD>
 cudaError_t run_ne_epoch(NeEpoch E, int sms, cudaStream_t s) {
   using Shape = NeShape<MAXD>;
-  const size_t smem = std::max(size_t(Shape::kWarps) * ne_stage_floats(E.ncomp) * 4,
-                               size_t(Shape::kTile) * (2 * (kSlots * E.ncomp + 2) + kSlots) * 4);
-  cudaError_t e = cudaFuncSetAttribute(ne_epoch_kernel<MAXD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const size_t smem = ne_smem<MAXD>(E.ncomp);
+  // The limit is the widest rows', not this call's: concurrent callers with
+  // other widths must not lower it between this call and the launch.
+  cudaError_t e = cudaFuncSetAttribute(ne_epoch_kernel<MAXD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)ne_smem<MAXD>(MAXD));
   if (e != cudaSuccess) return e;
   int resident = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, ne_epoch_kernel<MAXD>, Shape::kWarps * 32, smem);
