@@ -1151,7 +1151,7 @@ int fuzzy_impl(evoc_gpu_ctx* ctx, const int32_t* idx, const float* dist, int64_t
     {
       Stage st(ctx, "union_count");
       EVOC_TRY(evoc::launch_fuzzy_union_count(n, k, symmetrize, w, d_indptr, ctx->sms, ctx->stream), "union count");
-      ctx->launches += symmetrize ? 9 : 3;
+      ctx->launches += (symmetrize ? 3 : 0) + (symmetrize ? 2 : 1) * evoc::scan_counts_launches(n);
     }
     EVOC_TRY(cudaMemcpyAsync(&total_nnz, d_indptr + n, 8, cudaMemcpyDeviceToHost, ctx->stream), "read nnz");
     EVOC_TRY(cudaStreamSynchronize(ctx->stream), "union count");
@@ -1291,7 +1291,7 @@ int run_nndescent(evoc_gpu_ctx* ctx, const evoc_gpu_opts& opts, const Job& j, in
     Stage st(ctx, "nnd_iteration");
     EVOC_TRY(cudaMemsetAsync(a.changes, 0, 8, ctx->stream), "clear changes");
     EVOC_TRY(evoc::launch_nnd_iteration(a, cur, it, ctx->stream), "NN-descent iteration");
-    ctx->launches += 7;
+    ctx->launches += 6 + evoc::scan_counts_launches(n);
     cur ^= 1;
     unsigned long long ch = 0;
     double sum = 0.0;

@@ -324,6 +324,8 @@ cudaError_t launch_fuzzy_union_write(int64_t n, int k, int symmetrize, const Fuz
 
 namespace evoc {
 // graph.cu: out[0] = 0, out[i+1] = cnt[0] + ... + cnt[i].
+constexpr int64_t kScanOneBlock = 4096;
+inline int scan_counts_launches(int64_t n) { return n <= 0 ? 0 : n <= kScanOneBlock ? 1 : 3; }
 cudaError_t launch_scan_counts(const int32_t* cnt, int64_t n, int64_t* out, cudaStream_t stream);
 cudaError_t launch_scan_counts(const int64_t* cnt, int64_t n, int64_t* out, cudaStream_t stream);
 // jaccard.cu: per-row popcounts of rows of ldw 32-bit words.

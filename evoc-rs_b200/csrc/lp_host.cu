@@ -20,6 +20,7 @@
 
 #include "../../include/evoc_gpu.h"
 #include "ctx.h"
+#include "kernels.h"
 #include "lp.h"
 
 namespace {
@@ -541,7 +542,7 @@ int lp_init_level(evoc_gpu_ctx* ctx, const lp::ReduceScratch& W, const lp::Csr& 
     Stage st(ctx, "reduced_graph");
     EVOC_TRY(lp::launch_reduce_graph(g, part, xnorm, n_parts, W, r_indptr, r_indices, r_data, r_nnz, s),
              "reduced graph");
-    ctx->launches += 12;
+    ctx->launches += 11 + evoc::scan_counts_launches(n_parts);
   }
   cudaError_t e;
   const int64_t rnnz = read_i64(ctx, r_nnz, &e);
@@ -592,7 +593,7 @@ int lp_init_level(evoc_gpu_ctx* ctx, const lp::ReduceScratch& W, const lp::Csr& 
   {
     Stage st(ctx, "hadamard_symmetric");
     EVOC_TRY(lp::launch_hadamard_sym(g, W, s_indptr, s_indices, s_data, s_nnz, s), "hadamard_symmetric");
-    ctx->launches += 6;
+    ctx->launches += 5 + evoc::scan_counts_launches(g.n);
   }
   const int64_t snnz = read_i64(ctx, s_nnz, &e);
   EVOC_TRY(e, "hadamard_symmetric");
