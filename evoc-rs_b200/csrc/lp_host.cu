@@ -23,6 +23,15 @@
 #include "kernels.h"
 #include "lp.h"
 
+// Loops that are worth the host's wide vectors: on x86 with GCC and glibc a copy
+// for AVX2 is chosen when the library is loaded; other hosts (the GB200's is
+// aarch64) build the one plain copy.
+#if defined(__x86_64__) && defined(__GNUC__) && !defined(__clang__) && defined(__GLIBC__)
+#define EVOC_WIDE_HOST __attribute__((target_clones("avx2", "default"), optimize("tree-vectorize")))
+#else
+#define EVOC_WIDE_HOST
+#endif
+
 namespace {
 
 using evoc::cuda_fail;
@@ -40,7 +49,7 @@ struct Mt {
   // The 624-word state update, in place: words 0..226 mix with the old words
   // 397 ahead, words 227..622 with the new words 227 behind, word 623 with
   // the new word 396 (split so no index needs a modulo).
-  __attribute__((target_clones("avx2", "default"), optimize("tree-vectorize"))) void regen() {
+  EVOC_WIDE_HOST void regen() {
     constexpr uint32_t kUp = 0x80000000u, kLo = 0x7fffffffu, kA = 0x9908b0dfu;
     uint32_t* k = s->key;
     auto mix = [&](int i, uint32_t next, uint32_t far) {
@@ -53,7 +62,7 @@ struct Mt {
     mix(623, k[0], k[396]);
     s->pos = 0;
   }
-  __attribute__((target_clones("avx2", "default"), optimize("tree-vectorize"))) void temper_block() {
+  EVOC_WIDE_HOST void temper_block() {
     for (int i = 0; i < 624; i++) {
       uint32_t y = s->key[i];
       y ^= y >> 11;
