@@ -104,8 +104,13 @@ struct evoc_gpu_ctx {
   };
   std::vector<BatchGraph> batch_graphs;  // captured batch pipelines, replayed per batch
   bool use_graphs = true;                // EVOC_NO_GRAPHS=1 launches the kernels directly
-  // Autotuned scan variants: (scan mode, keep, row bytes, floor(log2 n)) -> variant.
-  std::map<std::tuple<int, int, int64_t, int>, int> tune;
+  // Autotuned scan variants: (scan mode, keep, row bytes, floor(log2 n)) -> variant (kTunedSmall: the small
+  // form won), and whether it also stands in for the small form where that would serve.
+  struct Tuned {
+    int variant;
+    bool over_small;
+  };
+  std::map<std::tuple<int, int, int64_t, int>, Tuned> tune;
   uint64_t timeout_ns = 4000000000ull;  // longest a pipeline wait inside a kernel may take
   uint64_t delay_ns = 0;  // tests of the timeout path: the scan's producer starts this late
   bool sync_check = false;  // EVOC_SYNC_CHECK=1: wait for and check every kernel stage (fault diagnosis)

@@ -78,10 +78,21 @@ int ilog2(int64_t v) {
   return l;
 }
 
-// The autotuned scan variant for this shape, or -1 (automatic).
+// What the tuner calls the small form (small.cu) beside the scan's variants.
+constexpr int kTunedSmall = evoc::kScanVariants;
+
+// Whether the small form serves these rows.
+bool small_feasible(int mode, int64_t n, int64_t keep) {
+  return evoc::small_scan_feasible(mode, n, int(std::min<int64_t>(keep, 1 << 20)));
+}
+
+// The autotuned scan variant for this shape, or -1 (automatic: the small form
+// where it serves).  An entry may come from another n of the same power of two:
+// one tuned where the small form does not serve says nothing against it.
 int tuned_variant(const evoc_gpu_ctx* ctx, int mode, int keep, int64_t row_bytes, int64_t n) {
-  auto it = ctx->tune.find(std::make_tuple(mode, keep, row_bytes, ilog2(n)));
-  return it == ctx->tune.end() ? -1 : it->second;
+  const auto it = ctx->tune.find(std::make_tuple(mode, keep, row_bytes, ilog2(n)));
+  if (it == ctx->tune.end() || it->second.variant == kTunedSmall) return -1;
+  return !it->second.over_small && small_feasible(mode, n, keep) ? -1 : it->second.variant;
 }
 
 int scan_grid(const evoc_gpu_ctx* ctx, int64_t n_q) {
@@ -104,8 +115,7 @@ int main_scan_grid(const evoc_gpu_ctx* ctx, int64_t n_q, int keep, int variant) 
 // Whether a request's scan takes the small form (small.cu): few enough rows,
 // no tuned variant, no delayed producer (a test's).
 bool use_small(const evoc_gpu_ctx* ctx, int mode, int64_t n, int64_t keep, int variant) {
-  return variant < 0 && ctx->delay_ns == 0 && !ctx->lean &&
-         evoc::small_scan_feasible(mode, n, int(std::min<int64_t>(keep, 1 << 20)));
+  return variant < 0 && ctx->delay_ns == 0 && !ctx->lean && small_feasible(mode, n, keep);
 }
 
 // The same with room for its scores.
@@ -1807,13 +1817,13 @@ int tune_load_impl(evoc_gpu_ctx* ctx, const char* path) {
   std::string line;
   int loaded = 0;
   while (std::getline(f, line)) {
-    int ver = 0, mode = 0, keep = 0, l2 = 0, v = 0;
+    int ver = 0, mode = 0, keep = 0, l2 = 0, v = 0, over = 1;  // a line without the last field: over the small form
     long long rb = 0;
     double ms = 0.0;
-    if (std::sscanf(line.c_str(), "evoc-tune %d mode=%d keep=%d row_bytes=%lld log2n=%d variant=%d ms=%lf", &ver,
-                    &mode, &keep, &rb, &l2, &v, &ms) == 7 &&
-        ver == 1 && v >= 0 && v < evoc::kScanVariants) {
-      ctx->tune[std::make_tuple(mode, keep, int64_t(rb), l2)] = v;
+    if (std::sscanf(line.c_str(), "evoc-tune %d mode=%d keep=%d row_bytes=%lld log2n=%d variant=%d ms=%lf over_small=%d",
+                    &ver, &mode, &keep, &rb, &l2, &v, &ms, &over) >= 7 &&
+        ver == 1 && v >= 0 && v <= kTunedSmall) {
+      ctx->tune[std::make_tuple(mode, keep, int64_t(rb), l2)] = {v, over != 0};
       loaded++;
     }
   }
@@ -1863,17 +1873,19 @@ int autotune_impl(evoc_gpu_ctx* ctx, int32_t dtype, int32_t form_in, int64_t n, 
   const int64_t nt = std::min<int64_t>(n, n >= 1000000 ? 262144 : 65536);
   const int64_t rows = evoc::padded_rows(nt);
   EVOC_TRY(ctx->xb.ensure(size_t(rows * row_bytes)), "alloc tuning rows");
-  const int32_t* pc = nullptr;
+  const int32_t *pc = nullptr, *pc_least = nullptr;
   if (mode == evoc::kScanJaccard) {
     const int64_t ldp = round_up(dim, 64);
     EVOC_TRY(ctx->x.ensure(size_t(rows * ldp)), "alloc tuning bits");
     EVOC_TRY(evoc::launch_fill_random(2, ctx->x.p, rows, ldp, nt, dim, 0x7157u, ctx->sms, ctx->stream), "fill");
-    EVOC_TRY(ctx->popc.ensure(size_t(nt) * 4), "alloc popcounts");
+    EVOC_TRY(ctx->popc.ensure(popcount_words(nt) * 4), "alloc popcounts");
     EVOC_TRY(evoc::launch_popcount_rows(ctx->x.p, nt, int(ldp / 4), ctx->popc.as<int32_t>(), ctx->sms, ctx->stream),
              "popcounts");
     EVOC_TRY(evoc::launch_expand_bits(ctx->x.p, nt, ldp, dim, ctx->xb.p, rows, row_bytes, ctx->sms, ctx->stream),
              "expand bits");
     pc = ctx->popc.as<int32_t>();
+    pc_least = ctx->popc.as<int32_t>() + nt;
+    EVOC_TRY(evoc::launch_least_popcounts(pc, nt, ctx->popc.as<int32_t>() + nt, ctx->sms, ctx->stream), "popcounts");
   } else {
     const int64_t bytes = mode == evoc::kScanHalf ? dim * 2 : dim;
     EVOC_TRY(evoc::launch_fill_random(mode == evoc::kScanHalf ? 0 : 1, ctx->xb.p, rows, row_bytes, nt, bytes, 0x7157u,
@@ -1883,7 +1895,10 @@ int autotune_impl(evoc_gpu_ctx* ctx, int32_t dtype, int32_t form_in, int64_t n, 
   const int grid = scan_grid(ctx, nt);
   EVOC_TRY(ctx->cand.ensure(size_t(nt) * size_t(keep) * 4), "alloc tuning outputs");
   EVOC_TRY(ctx->out_dist.ensure(size_t(nt) * size_t(keep) * 4), "alloc tuning outputs");
-  EVOC_TRY(ctx->scratch.ensure(size_t(grid) * 256 * size_t(keep) * 8), "alloc scratch");
+  const bool small = small_feasible(mode, n, keep);  // then nt == n
+  EVOC_TRY(ctx->scratch.ensure(std::max(size_t(grid) * 256 * size_t(keep) * 8,
+                                        small ? evoc::small_scan_bytes(nt, nt) : 0)),
+           "alloc scratch");
   EVOC_TRY(ctx->flag.ensure(64), "alloc flag");
   int* status = ctx->flag.as<int>() + 1;
   cudaEvent_t e0, e1;
@@ -1892,15 +1907,20 @@ int autotune_impl(evoc_gpu_ctx* ctx, int32_t dtype, int32_t form_in, int64_t n, 
   std::string rep;
   // The automatic choice stays unless another variant is clearly faster:
   // timings within a few percent are noise at this sample size.
-  const int automatic = evoc::tc_scan_automatic_variant(mode, keep);
-  std::vector<float> times(evoc::kScanVariants, -1.0f);
-  for (int v = 0; v < evoc::kScanVariants; v++) {
-    if (!evoc::tc_scan_variant_feasible(v, keep, true)) continue;
+  const int automatic = small ? kTunedSmall : evoc::tc_scan_automatic_variant(mode, keep);
+  std::vector<float> times(kTunedSmall + 1, -1.0f);
+  for (int v = 0; v <= kTunedSmall; v++) {
+    if (v == kTunedSmall ? !small : !evoc::tc_scan_variant_feasible(v, keep, true)) continue;
     auto run = [&]() {
+      if (v == kTunedSmall)
+        return evoc::launch_small_scan(mode, ctx->xb.p, rows, nt, 0, nt, row_bytes, keep, final_mode, out_dtype,
+                                       ctx->scratch.p, ctx->cand.as<int32_t>(), nullptr,
+                                       final_mode ? ctx->out_dist.as<float>() : nullptr, nullptr, status,
+                                       ctx->timeout_ns, pc, evoc::kHalfF16, ctx->sms, ctx->stream);
       return evoc::launch_tc_scan(mode, ctx->xb.p, rows, 0, nt, ctx->xb.p, rows, nt, row_bytes, keep,
                                   ctx->scratch.as<uint64_t>(), grid, 1, final_mode, out_dtype, ctx->cand.as<int32_t>(),
                                   nullptr, final_mode ? ctx->out_dist.as<float>() : nullptr, status, ctx->timeout_ns,
-                                  pc, ctx->stream, v);
+                                  pc, ctx->stream, v, evoc::kHalfF16, nullptr, nullptr, 0, 0, pc_least);
     };
     cudaError_t e = cudaMemsetAsync(status, 0, sizeof(int), ctx->stream);
     if (e == cudaSuccess) e = run();  // warm-up
@@ -1919,24 +1939,25 @@ int autotune_impl(evoc_gpu_ctx* ctx, int32_t dtype, int32_t form_in, int64_t n, 
     cudaEventElapsedTime(&ms, e0, e1);
     ms /= 2.0f;
     char buf[160];
-    std::snprintf(buf, sizeof(buf), "%d %.3f ms %s%s\n", v, double(ms), evoc::tc_scan_variant_name(v),
-                  st ? " (timed out)" : "");
+    std::snprintf(buf, sizeof(buf), "%d %.3f ms %s%s\n", v, double(ms),
+                  v == kTunedSmall ? "small form" : evoc::tc_scan_variant_name(v), st ? " (timed out)" : "");
     rep += buf;
     if (st == 0) times[size_t(v)] = ms;
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   int best = (automatic >= 0 && times[size_t(automatic)] >= 0.0f) ? automatic : -1;
-  for (int v = 0; v < evoc::kScanVariants; v++) {
+  for (int v = 0; v <= kTunedSmall; v++) {
     if (times[size_t(v)] < 0.0f) continue;
     if (best < 0 || times[size_t(v)] < 0.97f * times[size_t(best)]) best = v;
   }
   if (best < 0) return fail(ctx, EVOC_ERR_TIMEOUT, "no variant completed");
   const float best_ms = times[size_t(best)];
-  ctx->tune[std::make_tuple(mode, keep, row_bytes, ilog2(n))] = best;
+  ctx->tune[std::make_tuple(mode, keep, row_bytes, ilog2(n))] = {best, small};
   char line[200];
-  std::snprintf(line, sizeof(line), "evoc-tune 1 mode=%d keep=%d row_bytes=%lld log2n=%d variant=%d ms=%.3f\n", mode,
-                keep, static_cast<long long>(row_bytes), ilog2(n), best, double(best_ms));
+  std::snprintf(line, sizeof(line),
+                "evoc-tune 1 mode=%d keep=%d row_bytes=%lld log2n=%d variant=%d ms=%.3f over_small=%d\n", mode, keep,
+                static_cast<long long>(row_bytes), ilog2(n), best, double(best_ms), small ? 1 : 0);
   rep += std::string("chosen: ") + line;
   if (cache_path && cache_path[0]) {
     std::lock_guard<std::mutex> flock(g_tune_file_mu);

@@ -158,9 +158,11 @@ int evoc_gpu_knn_graph_batch(evoc_gpu_ctx* ctx, const evoc_gpu_opts* opts, int32
 /*
  * Autotuner.  Times the tensor-core scan's kernel variants (pipeline depth,
  * epilogue warp groups, heaps in shared or global memory) for requests of
- * this shape on synthetic rows (a sample of up to 65,536 rows), keeps the
- * fastest for this context -- later calls with the same dtype, form, k, dim
- * and floor(log2 n) use it -- and, when cache_path is not NULL, appends it to
+ * this shape on synthetic rows (a sample of up to 65,536 rows), and the small
+ * form where it serves n rows; keeps the fastest for this context -- later
+ * calls with the same dtype, form, k, dim and floor(log2 n) use it, but for
+ * whole graphs that take tile lists, and rows that the small form serves where
+ * n was too large for it -- and, when cache_path is not NULL, appends it to
  * that file.  A context created while EVOC_TUNE_CACHE names such a file loads
  * it.  Only the tensor-core forms are tuned (f32 BF16_RERANK, i8 and u8
  * EXACT_INT); every variant gives the same results.  report (may be NULL)
