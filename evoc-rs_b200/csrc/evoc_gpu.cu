@@ -919,7 +919,7 @@ int run_bf16_rerank(evoc_gpu_ctx* ctx, const evoc_gpu_opts& opts, const Job& j, 
                                      certify ? cf(CL.bound) : nullptr, j.status, ctx->timeout_ns, nullptr, half,
                                      ctx->sms, ctx->stream),
              "small scan");
-    ctx->launches += 2;
+    ctx->launches += evoc::small_scan_launches(j.nq, j.n);
   } else if (!lists) {
     Stage st(ctx, "bf16_scan");
     EVOC_TRY(ctx->scratch.ensure(scan_scratch_bytes(ctx, j.nq, C)), "alloc scratch");
@@ -990,7 +990,7 @@ int run_int8(evoc_gpu_ctx* ctx, const Job& j, int64_t ldb) {
                                      ctx->scratch.p, j.idx, j.raw, j.dist, nullptr, j.status, ctx->timeout_ns, nullptr,
                                      evoc::kHalfF16, ctx->sms, ctx->stream),
              "small scan");
-    ctx->launches += 2;
+    ctx->launches += evoc::small_scan_launches(j.nq, j.n);
     return EVOC_OK;
   }
   EVOC_TRY(ctx->scratch.ensure(size_t(scan_grid(ctx, j.nq)) * 256 * size_t(j.keff) * 8), "alloc scratch");
@@ -1037,7 +1037,7 @@ int run_jaccard_tc(evoc_gpu_ctx* ctx, const Job& j, int64_t ldb, int64_t nbytes)
                                      EVOC_DTYPE_U8, ctx->scratch.p, j.idx, j.raw, j.dist, nullptr, j.status,
                                      ctx->timeout_ns, ctx->popc.as<int32_t>(), evoc::kHalfF16, ctx->sms, ctx->stream),
              "small scan");
-    ctx->launches += 2;
+    ctx->launches += evoc::small_scan_launches(j.nq, j.n);
     return EVOC_OK;
   }
   const int grid = scan_grid(ctx, j.nq);

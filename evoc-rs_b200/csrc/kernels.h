@@ -205,6 +205,7 @@ cudaError_t launch_prune_lists(int mode, int64_t n, int64_t group_rows, int grou
 constexpr int64_t kSmallRows = 5000;
 bool small_scan_feasible(int mode, int64_t n_k, int keep);
 size_t small_scan_bytes(int64_t n_q, int64_t n_k);
+int small_scan_launches(int64_t n_q, int64_t n_k);
 cudaError_t launch_small_scan(int mode, const void* X, int64_t rows_mem, int64_t n, int64_t q_row0, int64_t n_q,
                               int64_t row_bytes, int keep, int final_mode, int dtype, void* scores, int32_t* out_idx,
                               float* out_raw, float* out_dist, float* out_bound, int* status, uint64_t timeout_ns,

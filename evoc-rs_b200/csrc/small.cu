@@ -214,6 +214,11 @@ size_t small_scan_bytes(int64_t n_q, int64_t n_k) {
   return size_t(score_rows(n_q, n_k)) * size_t(padded_rows(n_k)) * 4;
 }
 
+int small_scan_launches(int64_t n_q, int64_t n_k) {
+  const int64_t step = score_rows(n_q, n_k);
+  return 2 * int((n_q + step - 1) / step);
+}
+
 cudaError_t launch_small_scan(int mode, const void* X, int64_t rows_mem, int64_t n, int64_t q_row0, int64_t n_q,
                               int64_t row_bytes, int keep, int final_mode, int dtype, void* scores, int32_t* out_idx,
                               float* out_raw, float* out_dist, float* out_bound, int* status, uint64_t timeout_ns,
