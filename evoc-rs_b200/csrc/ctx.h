@@ -90,6 +90,9 @@ struct evoc_gpu_ctx {
   // leaves it larger than kKeepLists gives it back.
   evoc::DevBuf prune;
   static constexpr size_t kKeepLists = size_t(4) << 30;
+  // Most groups and segments of the lists (0: the kernels' limits); fewer make groups of several tiles and
+  // arrays too short for every cut out of a small set (tests; EVOC_LIST_LIMITS=groups,segments).
+  int list_groups = 0, list_segments = 0;
   bool lean = false;  // plain scans only, without the memory of lists and small forms (a server short of budget)
   evoc::DevBuf batch_ws, batch_tab;  // batches: per-request work arena, device tables
   void* batch_host = nullptr;  // pinned staging of the tables

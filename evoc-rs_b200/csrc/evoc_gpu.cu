@@ -229,10 +229,10 @@ constexpr int64_t kStrayPivots = 2048;
 
 int64_t list_pivots(int64_t n) { return std::max<int64_t>(2, std::min<int64_t>(n / 512, 2048)); }
 
-// Tiles per group as a power of two: at most kPruneGroups groups.
-int prune_lg(int64_t n) {
+// Tiles per group as a power of two: at most `most` groups.
+int prune_lg(int64_t n, int most) {
   int lg = 0;
-  while ((((n + 255) / 256 + (int64_t(1) << lg) - 1) >> lg) > evoc::kPruneGroups) lg++;
+  while ((((n + 255) / 256 + (int64_t(1) << lg) - 1) >> lg) > most) lg++;
   return lg;
 }
 
@@ -245,13 +245,14 @@ struct PruneLayout {
 
 // row_bytes: of the operand rows; xs_bytes: of the rows copied into scanned
 // order (the operand rows; binary data: the packed rows).
-PruneLayout prune_layout(int64_t n, int64_t row_bytes, int64_t xs_bytes) {
+PruneLayout prune_layout(const evoc_gpu_ctx* ctx, int64_t n, int64_t row_bytes, int64_t xs_bytes) {
   PruneLayout L{};
   const int64_t piv = list_pivots(n) + kStrayPivots;
-  L.lg = prune_lg(n);
+  L.lg = prune_lg(n, ctx->list_groups ? ctx->list_groups : evoc::kPruneGroups);
   L.group_rows = int64_t(256) << L.lg;
   L.groups = (n + L.group_rows - 1) / L.group_rows;
-  L.segments = std::min<int64_t>(L.groups + piv, evoc::kPruneSegments);
+  L.segments = std::min<int64_t>(L.groups + piv, ctx->list_segments ? std::max<int64_t>(ctx->list_segments, L.groups)
+                                                                     : evoc::kPruneSegments);
   L.ld = round_up(std::max(L.segments, piv), 256);
   size_t off = 0;
   auto take = [&](size_t bytes) {
@@ -352,7 +353,7 @@ int list_scan(evoc_gpu_ctx* ctx, const Job& j, int mode, const void* rows, int64
     const int32_t near = read_count(ctx, fit, &rc);
     if (rc || float(near) < rule.sample * float(sample.rows)) return rc;
   }
-  const PruneLayout L = prune_layout(n, row_bytes, binary ? ldp : row_bytes);
+  const PruneLayout L = prune_layout(ctx, n, row_bytes, binary ? ldp : row_bytes);
   // All the memory of the lists now: where there is none the full scan does without, and from here
   // on no allocation takes the arena away.
   const int64_t piv_max = piv1 + kStrayPivots;
@@ -2008,6 +2009,13 @@ int evoc_gpu_ctx_create(int device, evoc_gpu_ctx** out) {
     const long long r = std::atoll(v);
     ctx->sym_min_rows = r < 0 ? 0 : r;
   }
+  if (const char* v = std::getenv("EVOC_LIST_LIMITS")) {
+    int groups = 0, segments = 0;
+    if (std::sscanf(v, "%d,%d", &groups, &segments) >= 1) {
+      ctx->list_groups = std::min(std::max(groups, 0), evoc::kPruneGroups);
+      ctx->list_segments = std::min(std::max(segments, 0), evoc::kPruneSegments);
+    }
+  }
   if (const char* v = std::getenv("EVOC_TUNE_CACHE"))
     if (v[0]) tune_load_impl(ctx, v);
   e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
@@ -2197,7 +2205,7 @@ void knn_buffer_needs(const evoc_gpu_ctx* ctx, const evoc_gpu_opts& opts, int32_
     at_least(kBufHist, size_t(piv + kStrayPivots) * 4);
     at_least(kBufCursor, size_t(piv + kStrayPivots) * 4);
     at_least(kBufScratch, sample_fit_bytes(list_sample(n, piv)));
-    b[kBufPrune] = prune_layout(n, row_bytes, xs_bytes).total;
+    b[kBufPrune] = prune_layout(ctx, n, row_bytes, xs_bytes).total;
   };
   auto nnd = [&]() {
     size_t sizes[kNndParts];
