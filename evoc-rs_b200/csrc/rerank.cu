@@ -272,17 +272,20 @@ rerank_f32_kernel(const float* __restrict__ X, int ld, int d, int64_t n, int64_t
   }
 }
 
-// The same with the candidate rows brought into shared memory by bulk copies:
-// every warp keeps a ring of `slots` rows in flight, far more than registers
-// could hold, and takes its products from there in the same order (so the
-// results are the same bit for bit).  Bound by L2 bandwidth: 6.8 TB/s of
+// The same with the candidate rows brought into shared memory by bulk copies,
+// one instruction a row: every warp keeps a ring of `slots` rows (an even
+// number: four up to a stride of 672 floats, two above) and takes its products
+// from there in the same order (so the results are the same bit for bit), two
+// rows at a time, their copies sent again together.  16 warps an SM keep 32 to
+// 64 rows in flight that way.  Bound by L2 bandwidth: 6.8 TB/s of
 // gathered rows.  1,000,000 x 768 with 60 candidates 27 ms (loads through
-// registers: 38), 200,000 x 768 with 75 the same 6.4; below 512 features the
+// registers: 38), 200,000 x 768 with 75 the same 6.4; below a stride of 512 the
 // copies are too short and the few warps show (20,011 x 384: 0.34 ms against
-// 0.19, 50,000 x 200: 0.77 against 0.34), above 1,600 two rows a warp no
-// longer fit.
+// 0.19, 50,000 x 200: 0.77 against 0.34).  It ends where two rows, the query row
+// and the keys of 16 warps no longer fit an SM: above a stride of 1,136 with up
+// to 64 candidates, 1,088 with up to 128, 1,008 with more.
 constexpr int BW = 16;  // warps per block, one block per SM
-constexpr int kBulkMin = 512, kBulkMax = 1600;  // row lengths taken
+constexpr int kBulkMin = 512;  // smallest row stride taken
 
 __global__ void __launch_bounds__(BW * 32, 1)
 rerank_bulk_kernel(const float* __restrict__ X, int ld, int d, int64_t n, int64_t n_keys, int64_t q_row0,
@@ -447,7 +450,7 @@ cudaError_t launch_rerank_f32(const float* X, int ld, int d, int64_t n, int64_t 
   while (P < C || P < 2) P <<= 1;
   const size_t limit = 227 * 1024 - 1024, fixed = size_t(ld) * 4 + size_t(P) * 8 + 32 * 8;
   const int64_t slots = (int64_t(limit / BW) - int64_t(fixed)) / (int64_t(ld) * 4 + 8);
-  if (status && ld >= kBulkMin && ld <= kBulkMax && slots >= 2) {
+  if (status && ld >= kBulkMin && slots >= 2) {
     const int s = int(std::min<int64_t>(slots & ~int64_t(1), 16));
     const size_t smem = BW * (fixed + size_t(s) * (size_t(ld) * 4 + 8));
     const cudaError_t e = cudaFuncSetAttribute(rerank_bulk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
