@@ -27,7 +27,8 @@ cudaError_t launch_validate_csr(const Csr& g, int32_t* bad, cudaStream_t s);
 // Largest row length -> *out (device int64).
 cudaError_t launch_max_degree(const int64_t* indptr, int64_t n, int64_t* out, cudaStream_t s);
 
-// Sets labels[idx[i]] = i for i in order (seeds from host draws): one thread, in order.
+// Sets labels[idx[i]] = i over labels that are all -1 (seeds from host draws); the last i of a repeated
+// index stays, as if they were set in order.
 cudaError_t launch_seed_labels(int32_t* labels, const int64_t* idx, int64_t count, cudaStream_t s);
 
 // One label_prop_iteration sweep.  Rows whose table outgrows shared memory go

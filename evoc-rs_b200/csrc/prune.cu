@@ -34,9 +34,14 @@
 // Slack.  The products with the centres and the scores the bound is compared
 // with are tensor-core sums: at most e = (L/4 + 2) 2^-21 |x||y| off for 16-bit
 // operands of length L, exact for integers.  The bound adds up five such
-// terms of size at most N^2 (N the largest row norm); it is given 16 e N^2 and
-// 1e-5 N^2 more for the f32 arithmetic here.  For binary rows the bound on
-// the intersection becomes one on J through the segments' smallest popcounts.
+// terms of size at most N^2 (N the largest row norm).  The a_x are off by the
+// f32 sums that make them, (L/32 + L/512 + 28) 2^-24 of |x| / |m|, and stand in
+// three terms.  16-bit rows get 16 e N^2, of which 11 e cover the latter;
+// integer rows 8 (L/32 + L/512) 2^-24 N^2 (their sums are exact up to about
+// 1,040 features); both 1e-5 N^2 for the operations on the sums.  The |x'|
+// carry an allowance of their own (segment_stats_kernel).  For binary rows the
+// bound on the intersection becomes one on J through the segments' smallest
+// popcounts.
 //
 // Replaces nothing in the reference, which prunes by its RP forest and
 // NN-descent (src/nndescent/float.rs:775-879) without a guarantee.
@@ -774,6 +779,10 @@ segment_stats_kernel(const uint8_t* __restrict__ rows, int64_t row_bytes, Segmen
   msq = 0.0f;
   for (int w = 0; w < kStatThreads / 32; w++) msq += red[w][0];
   __syncthreads();
+  // |x'|^2 = sq - dot^2 / msq cancels, so the sums' rounding counts against |x|^2: sq is off by
+  // (L/32 + 5) u of it (a lane's chain and five additions), dot^2 by twice that, msq by (L/512 + 23) u;
+  // the last operations take 9 u more.
+  const float allowance = (3.0f * float((len + 31) / 32) + float(len) / 512.0f + 48.0f) * 0x1p-24f;
   float a0 = FLT_MAX, a1 = -FLT_MAX, rho = 0.0f, nsq = 0.0f, sq0 = FLT_MAX;
   for (int64_t r = r0 + warp; r < r1; r += kStatThreads / 32) {
     const uint8_t* row = rows + r * row_bytes;
@@ -795,8 +804,7 @@ segment_stats_kernel(const uint8_t* __restrict__ rows, int64_t row_bytes, Segmen
     const float a = msq > 0.0f ? dot / msq : 0.0f;
     a0 = fminf(a0, a);
     a1 = fmaxf(a1, a);
-    // the subtraction cancels: 4e-6 |x|^2 covers the sums' rounding
-    rho = fmaxf(rho, sqrtf(fmaxf(sq - a * dot, 0.0f) + 4e-6f * sq));
+    rho = fmaxf(rho, sqrtf(fmaxf(sq - a * dot, 0.0f) + allowance * sq));
     nsq = fmaxf(nsq, sq);
     sq0 = fminf(sq0, sq);
   }
@@ -841,7 +849,9 @@ decide_kernel(int mode, Segments seg, const int32_t* __restrict__ group_of, int 
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5, g = blockIdx.x;
   for (int i = t; i < kPruneGroups / 32; i += kDecideThreads) hit[i] = 0u;
   const float nn = __uint_as_float(*st.top);
-  const float e = mode == kScanHalf ? (float(half_len) / 4.0f + 2.0f) * 0x1p-21f * 16.0f : 0.0f;
+  // 16-bit: 16 e; integers, whose products are exact: eight times what their f32 sums are off by
+  const float e = mode == kScanHalf ? (float(half_len) / 4.0f + 2.0f) * 0x1p-21f * 16.0f
+                                    : 8.0f * (float(half_len) / 16.0f + float(half_len) / 256.0f) * 0x1p-24f;
   const float slack = (e + 1e-5f) * nn;
   auto value = [&](int32_t u) { return mode == kScanHalf ? __int_as_float(u) : float(u); };
   __syncthreads();
