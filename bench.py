@@ -497,14 +497,17 @@ def sampled_exact_check(x, oi, oraw, k, kind, rows=128):
     return {"rows": int(len(q)), "indices_exact": ok_i, "raw_exact": ok_r}
 
 
-def exhaustive_only(roofline):
-    """A scan over tile lists multiplies a part of the pairs only, so a rate over all n^2 of them
-    (and the traffic of a scan that reads every tile) is no share of any peak."""
+def over_lists(roofline, lists):
+    """A scan over tile lists multiplies a part of the tiles only: the rate is that of the tiles it
+    multiplied (and the traffic of a scan that reads every tile is not its own)."""
+    kept = lists["tiles"] / lists["all_tiles"]
     roofline["exhaustive_equivalent"] = roofline["achieved"]
     roofline["note"] = "scan over tile lists: key tiles that provably hold no neighbour are not multiplied"
-    for key in ("achieved", "frac", "frac_of_burst", "traffic"):
+    roofline["tiles"], roofline["tiles_kept"] = lists["tiles"], kept
+    for key in ("achieved", "frac", "frac_of_burst"):
         if key in roofline:
-            roofline[key] = None
+            roofline[key] *= kept
+    roofline["traffic"] = None
 
 
 def exact_int_leg(workload, n, d, k, dev, local, rank, world, pg, steps, warmup, e2e_steps, check_rows, cpu_rows,
@@ -561,6 +564,7 @@ def exact_int_leg(workload, n, d, k, dev, local, rank, world, pg, steps, warmup,
     if pg:
         pg.barrier()
     clk = clocks.stop()
+    lists = ctx.list_stats()  # of the last timed step
     ms_step = ev0.elapsed_time(ev1) / steps
     if pg:
         t = torch.tensor([ms_step], device=dev)
@@ -599,8 +603,8 @@ def exact_int_leg(workload, n, d, k, dev, local, rank, world, pg, steps, warmup,
                 "kernel": f"tc_scan_kernel ({'int8' if i8 else 'Jaccard on 0/1 int8'}, fused top-k)",
                 "peak_kind": peak_kind, "peak_burst": peak_burst, "frac_of_burst": achieved / peak_burst,
                 "launch_ms": scan_ms, "ops_per_launch": ops_per_pair * n * n}
-    if "tile_lists" in stage_ms:
-        exhaustive_only(roofline)
+    if lists["all_tiles"]:
+        over_lists(roofline, lists)
 
     cpu = None
     if rank == 0 and world == 1 and cpu_rows > 0:
@@ -779,7 +783,8 @@ def blobs_leg(dev, local, steps=20, warmup=5):
                      "peak": float(peaks.get("bf16_tflops")), "peak_kind": f"{peak_kind} bf16 burst",
                      "frac": flops / (scan_ms / 1e3) / 1e12 / float(peaks.get("bf16_tflops")),
                      "launch_ms": scan_ms, "traffic": None,
-                     "note": "16 query blocks of 128 rows: 16 of 148 SMs busy, launch/latency-bound by size"},
+                     "note": "scores written by one product on all SMs, each row's nearest selected from them; "
+                             "launch/latency-bound by size"},
         "e2e": {"value": n * k / (e2e_ms / 1000.0), "unit": UNIT, "h2d_bytes_per_step": n * d * 4,
                 "d2h_bytes_per_step": n * k * 8, "ms_per_step": e2e_ms},
         "cpu_baseline": {"value": n * k / t, "unit": UNIT, "cores": 1, "kind": "reference" if ref else "port",
@@ -1003,6 +1008,7 @@ def run_ours(args, world, rank, local):
     if pg:
         pg.barrier()
     clk = clocks.stop()
+    lists = ctx.list_stats()  # of the last timed step
     cert = ctx.certify_counts() if form == "bf16_rerank" else None
     sym = ctx.symmetric_stats() if form == "bf16_rerank" else None
     total_ms = ev0.elapsed_time(ev1)
@@ -1127,8 +1133,8 @@ def run_ours(args, world, rank, local):
                     "kernel": kernel, "algorithmic_flops": flops,
                     "peak_kind": f"{peak_kind} bf16 sustained (burst {peaks.get('bf16_tflops')})",
                     "launch_ms": scan_ms}
-        if "tile_lists" in stage_ms:
-            exhaustive_only(roofline)
+        if lists["all_tiles"]:
+            over_lists(roofline, lists)
     else:
         it_ms = stage_ms.get("nnd_iteration", [float("nan")])
         nst = ctx.nndescent_stats()  # of the last timed step

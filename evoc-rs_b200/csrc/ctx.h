@@ -93,6 +93,7 @@ struct evoc_gpu_ctx {
   // Most groups and segments of the lists (0: the kernels' limits); fewer make groups of several tiles and
   // arrays too short for every cut out of a small set (tests; EVOC_LIST_LIMITS=groups,segments).
   int list_groups = 0, list_segments = 0;
+  int64_t list_tiles = 0, list_tiles_all = 0;  // last call: tiles its list scan multiplied, of how many (0: none taken)
   bool lean = false;  // plain scans only, without the memory of lists and small forms (a server short of budget)
   evoc::DevBuf batch_ws, batch_tab;  // batches: per-request work arena, device tables
   void* batch_host = nullptr;  // pinned staging of the tables

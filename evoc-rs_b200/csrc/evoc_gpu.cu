@@ -130,7 +130,7 @@ struct Job {
   int32_t* idx;
   float* raw;
   float* dist;
-  int* status;
+  int* status;  // followed by 8 bytes, cleared, for the tiles a list scan multiplies
 };
 
 int run_fp32(evoc_gpu_ctx* ctx, const Job& j, int ld) {
@@ -363,6 +363,7 @@ int list_scan(evoc_gpu_ctx* ctx, const Job& j, int mode, const void* rows, int64
       !ctx->prune.room(L.total))
     return EVOC_OK;
   *taken = true;
+  ctx->list_tiles_all = (n + 127) / 128 * ((n + 255) / 256);
   uint8_t* b = ctx->prune.as<uint8_t>();
   auto f = [&](size_t off) { return reinterpret_cast<float*>(b + off); };
   auto i32 = [&](size_t off) { return reinterpret_cast<int32_t*>(b + off); };
@@ -489,7 +490,8 @@ int list_scan(evoc_gpu_ctx* ctx, const Job& j, int mode, const void* rows, int64
              "seeds");
     EVOC_TRY(evoc::launch_prune_lists(mode, n, L.group_rows, int(L.groups), seg, i32(L.group_of), segments, L.ld,
                                       i32(L.u), f(L.g), ps, f(L.seed), int(row_bytes / 2), i32(L.list), i32(L.len),
-                                      i32(L.blocks), ctx->stream),
+                                      i32(L.blocks), reinterpret_cast<unsigned long long*>(j.status + 1),
+                                      ctx->stream),
              "tile lists");
     ctx->launches += 6;
   }
@@ -1346,6 +1348,7 @@ int knn_impl(evoc_gpu_ctx* ctx, const evoc_gpu_opts* opts_in, int32_t dtype, con
   ctx->launches = 0;
   ctx->cert_checked = ctx->cert_second = ctx->cert_exact = 0;
   ctx->sym_sample = ctx->sym_cap = ctx->sym_max_offers = ctx->sym_overflow = 0;
+  ctx->list_tiles = ctx->list_tiles_all = 0;
   evoc_gpu_opts opts;
   evoc_gpu_default_opts(&opts);
   if (opts_in) {
@@ -1390,7 +1393,7 @@ int knn_impl(evoc_gpu_ctx* ctx, const evoc_gpu_opts* opts_in, int32_t dtype, con
     }
   }
   EVOC_TRY(ctx->flag.ensure(64), "alloc flag");
-  int* d_flags = ctx->flag.as<int>();  // [0] prepare_float, [1] scan status
+  int* d_flags = ctx->flag.as<int>();  // [0] some row is not of unit length, [1] scan status, [2..3] tiles
   EVOC_TRY(cudaMemsetAsync(d_flags, 0, 64, ctx->stream), "clear flags");
   job.status = d_flags + 1;
   int rc = EVOC_OK;
@@ -1446,7 +1449,7 @@ int knn_impl(evoc_gpu_ctx* ctx, const evoc_gpu_opts* opts_in, int32_t dtype, con
     else rc = run_nndescent(ctx, opts, job, EVOC_DTYPE_U8, ldb, ctx->x.p, 0, int(dim), rng_state);
   }
   if (rc) return rc;
-  int flags[2] = {0, 0};
+  int flags[4] = {0, 0, 0, 0};
   if (!on_dev) {
     Stage st(ctx, "d2h_out");
     EVOC_TRY(cudaMemcpyAsync(out_idx, job.idx, out_elems * 4, cudaMemcpyDeviceToHost, ctx->stream), "download idx");
@@ -1460,6 +1463,7 @@ int knn_impl(evoc_gpu_ctx* ctx, const evoc_gpu_opts* opts_in, int32_t dtype, con
   total.end();
   EVOC_TRY(cudaStreamSynchronize(ctx->stream), "knn_graph");
   if (ctx->prune.bytes > evoc_gpu_ctx::kKeepLists) ctx->prune.release();
+  std::memcpy(&ctx->list_tiles, flags + 2, 8);
   if (flags[1] == evoc::kStatusBadOrder || flags[1] == evoc::kStatusBadCandidate)
     return fail(ctx, EVOC_ERR_CUDA, "device self-check failed (code " + std::to_string(flags[1]) + ")");
   if (flags[1] != 0)
@@ -1575,6 +1579,7 @@ int knn_batch_impl(evoc_gpu_ctx* ctx, const evoc_gpu_opts* opts_in, int32_t dtyp
   ctx->launches = 0;
   ctx->cert_checked = ctx->cert_second = ctx->cert_exact = 0;
   ctx->sym_sample = ctx->sym_cap = ctx->sym_max_offers = ctx->sym_overflow = 0;
+  ctx->list_tiles = ctx->list_tiles_all = 0;
   evoc_gpu_opts opts;
   evoc_gpu_default_opts(&opts);
   if (opts_in) {
@@ -2114,6 +2119,13 @@ int evoc_gpu_last_symmetric(const evoc_gpu_ctx* ctx, int64_t* sample_rows, int64
   if (mailbox_cap) *mailbox_cap = ctx->sym_cap;
   if (max_offers) *max_offers = ctx->sym_max_offers;
   if (overflowed) *overflowed = ctx->sym_overflow;
+  return EVOC_OK;
+}
+
+int evoc_gpu_last_lists(const evoc_gpu_ctx* ctx, int64_t* tiles, int64_t* all_tiles) {
+  if (!ctx) return EVOC_ERR_ARG;
+  if (tiles) *tiles = ctx->list_tiles;
+  if (all_tiles) *all_tiles = ctx->list_tiles_all;
   return EVOC_OK;
 }
 

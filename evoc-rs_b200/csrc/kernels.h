@@ -198,7 +198,7 @@ cudaError_t launch_segment_stats(int mode, const void* rows, int64_t row_bytes, 
 cudaError_t launch_prune_lists(int mode, int64_t n, int64_t group_rows, int groups, const Segments& seg,
                                const int32_t* group_of, int segments, int64_t ld, const int32_t* U, const float* G,
                                const PruneStats& st, const float* T, int half_len, int32_t* list, int32_t* len,
-                               int32_t* block_order, cudaStream_t stream);
+                               int32_t* block_order, unsigned long long* tiles, cudaStream_t stream);
 
 // small.cu: the scan of query rows q_row0 .. q_row0+n_q-1 of X against its first n rows (self rule) for
 // sets of at most kSmallRows rows: scores holds small_scan_bytes.  Outputs as launch_tc_scan's.

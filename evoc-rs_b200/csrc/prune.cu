@@ -910,15 +910,22 @@ decide_kernel(int mode, Segments seg, const int32_t* __restrict__ group_of, int 
 
 // The query blocks by descending list length (counting sort in one block):
 // dealt in turns forth and back, every CTA then gets about the same work.
+// *total: the tiles of all blocks.
 __global__ void __launch_bounds__(1024)
 block_order_kernel(const int32_t* __restrict__ len, int groups, int64_t n_blocks, int blocks_per_group,
-                   int32_t* __restrict__ order) {
+                   int32_t* __restrict__ order, unsigned long long* __restrict__ total) {
   extern __shared__ int32_t bins[];  // groups + 1, longest first
   __shared__ int32_t part[1024];
   const int t = threadIdx.x, nb = groups + 1;
   for (int b = t; b < nb; b += blockDim.x) bins[b] = 0;
   __syncthreads();
-  for (int64_t q = t; q < n_blocks; q += blockDim.x) atomicAdd(&bins[groups - len[q / blocks_per_group]], 1);
+  unsigned long long tiles = 0;
+  for (int64_t q = t; q < n_blocks; q += blockDim.x) {
+    const int32_t l = len[q / blocks_per_group];
+    atomicAdd(&bins[groups - l], 1);
+    tiles += (unsigned long long)(l) * unsigned(blocks_per_group / 2);  // a tile: two blocks of rows
+  }
+  atomicAdd(total, tiles);
   __syncthreads();
   const int per = (nb + blockDim.x - 1) / blockDim.x;
   int32_t s = 0;
@@ -1141,12 +1148,12 @@ cudaError_t launch_segment_stats(int mode, const void* rows, int64_t row_bytes, 
 cudaError_t launch_prune_lists(int mode, int64_t n, int64_t group_rows, int groups, const Segments& seg,
                                const int32_t* group_of, int segments, int64_t ld, const int32_t* U, const float* G,
                                const PruneStats& st, const float* T, int half_len, int32_t* list, int32_t* len,
-                               int32_t* block_order, cudaStream_t stream) {
+                               int32_t* block_order, unsigned long long* tiles, cudaStream_t stream) {
   if (groups < 1 || groups > kPruneGroups || segments < groups) return cudaErrorInvalidValue;
   decide_kernel<<<unsigned(groups), kDecideThreads, 0, stream>>>(mode, seg, group_of, segments, groups, ld, U, G, st,
                                                                  T, half_len, list, len);
   block_order_kernel<<<1, 1024, size_t(groups + 1) * 4, stream>>>(len, groups, (n + BM - 1) / BM,
-                                                                  int(group_rows / BM), block_order);
+                                                                  int(group_rows / BM), block_order, tiles);
   return cudaGetLastError();
 }
 

@@ -93,6 +93,7 @@ def lib():
             L.evoc_gpu_set_symmetric_scan.argtypes = [P, C.c_int64]
             L.evoc_gpu_last_symmetric.argtypes = [P, C.POINTER(i64), C.POINTER(i64), C.POINTER(i64),
                                                   C.POINTER(i64)]
+            L.evoc_gpu_last_lists.argtypes = [P, C.POINTER(i64), C.POINTER(i64)]
             _bind_optional(L)
             _lib = L
     return _lib
@@ -309,6 +310,13 @@ class Context:
         a, b, c, d = C.c_int64(0), C.c_int64(0), C.c_int64(0), C.c_int64(0)
         lib().evoc_gpu_last_symmetric(self.h, C.byref(a), C.byref(b), C.byref(c), C.byref(d))
         return {"sample_rows": a.value, "mailbox_cap": b.value, "max_offers": c.value, "overflowed": d.value}
+
+    def list_stats(self) -> dict:
+        """Tiles of scores the last call's scan over tile lists multiplied, and those of the full scan
+        (both 0: not taken)."""
+        a, b = C.c_int64(0), C.c_int64(0)
+        lib().evoc_gpu_last_lists(self.h, C.byref(a), C.byref(b))
+        return {"tiles": a.value, "all_tiles": b.value}
 
     def close(self) -> None:
         if self.h:

@@ -445,6 +445,11 @@ int evoc_gpu_set_symmetric_scan(evoc_gpu_ctx* ctx, int64_t min_rows);
 int evoc_gpu_last_symmetric(const evoc_gpu_ctx* ctx, int64_t* sample_rows, int64_t* mailbox_cap,
                             int64_t* max_offers, int64_t* overflowed);
 
+/* The last call's scan over tile lists: the 128 x 256 tiles of scores it
+ * multiplied and those of the full scan (both 0 when the call did not take
+ * lists).  Either pointer may be NULL. */
+int evoc_gpu_last_lists(const evoc_gpu_ctx* ctx, int64_t* tiles, int64_t* all_tiles);
+
 /* The last NN-descent call on this context: iterations run, distances its
  * joins computed, and the bytes of each row those distances gathered (the
  * join's algorithmic traffic is distance_evals x row_bytes).  No counterpart
