@@ -307,6 +307,11 @@ bool use_lists(const evoc_gpu_ctx* ctx, int64_t n, int64_t r0, int64_t nq, int64
 // to row; their bound needs twice as much (bit rows that keep 0.66, 1,024 bits
 // with a twentieth flipped, skip no tile at all).
 //
+// Rows of few dimensions have a pivot near by without clusters, but not all
+// rows of a tile have: their bound keeps every tile up to cosines of 0.6 or so
+// (200,000 x 32 without clusters: int8 17.4 against 15.3 ms, f32 29.7 against
+// 27.0), hence less than a half, and less for the cheaper integer scan.
+//
 // Up to two rounds of query blocks the plan is a third of a f32 scan and more
 // of an integer one, so fewer tiles may be left: rows nearer to their pivot
 // (24,000 x 96 f32, 50 clusters about a common mean: 1.67 against 1.49 ms), and
@@ -322,8 +327,8 @@ struct FitRule {
 FitRule fit_rule(const evoc_gpu_ctx* ctx, int mode, int64_t n) {
   const bool few = n <= int64_t(256) * ctx->sms;
   if (mode == evoc::kScanJaccard) return few ? FitRule{0.2f, 0.75f} : FitRule{0.25f, 0.5f};
-  if (!few) return {0.5f, 0.25f};
-  return {0.3f, mode == evoc::kScanInt8 ? 0.75f : 0.25f};
+  if (mode == evoc::kScanInt8) return few ? FitRule{0.3f, 0.75f} : FitRule{0.35f, 0.25f};
+  return {few ? 0.3f : 0.4f, 0.25f};
 }
 
 // Plans the lists of a self-join of all rows and scans over them; *taken is

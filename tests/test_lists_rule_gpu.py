@@ -56,6 +56,9 @@ def _call(x, k, rows=None):
     ("i8", 24000, 96, 200, 0.0, False),     # pivots in a fifth of the clusters
     ("i8", 60000, 96, 50, 0.0, True),
     ("i8", 60000, 96, 0, 1.0, False),
+    ("f32", 60000, 32, 0, 0.0, False),      # few dimensions: pivots near by without clusters
+    ("i8", 60000, 32, 0, 0.0, False),
+    ("i8", 60000, 32, 50, 0.0, True),
     ("bits", 60000, 512, 20, 0.0, True),
     ("bits", 60000, 512, 1000, 0.0, False),
     ("bits", 60000, 512, 1, 0.0, False),    # dense rows of one prototype
