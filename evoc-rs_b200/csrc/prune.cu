@@ -553,8 +553,10 @@ __global__ void sample_fit_kernel(const float* __restrict__ products, int64_t ld
   if (i >= s.rows) return;
   const float* row = products + i * ld;
   const float own = sq ? rsqrtf(fmaxf(float(sq[i]), 1.0f)) : 1.0f;  // f32 rows have unit length
+  const int64_t self = s.first + i * s.stride;
   float most = 0.0f, sum = 0.0f;
   for (int p = lane; p < s.pivots; p += 32) {
+    if (p * s.pivot_stride == self) continue;  // the row itself is a pivot
     const float c = row[p] * own * (sq ? rsqrtf(fmaxf(float(sq[s.rows + p]), 1.0f)) : 1.0f);
     most = fmaxf(most, c);
     sum += c;

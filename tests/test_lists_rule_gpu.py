@@ -69,3 +69,23 @@ def test_who_takes_the_lists(kind, n, d, clusters, mean, lists):
     assert ("tile_lists" in stages) == lists
     part = _call(x, 15, (0, 1000))
     assert np.array_equal(ind[:1000], part[0]) and np.array_equal(dst[:1000].view(np.uint32), part[1].view(np.uint32))
+
+
+def test_sampled_rows_that_are_pivots():
+    """At 2^20 rows every sampled row is one of the pivots; that is no sign of clusters."""
+    n, d, k = 1 << 20, 64, 5
+    x = torch.randn(n, d, generator=torch.Generator(device="cuda").manual_seed(1), device="cuda")
+    x = torch.clamp(torch.round(127 * x / x.norm(dim=1, keepdim=True)), -127, 127).to(torch.int8)
+    ind, dst = torch.empty(n, k, dtype=torch.int32, device="cuda"), torch.empty(n, k, device="cuda")
+    torch.cuda.synchronize()
+    ctx = _lib.Context(0)
+    try:
+        o = _lib.default_opts()
+        o.buffers_on_device = 1
+        p = C.c_void_p
+        st = _lib.lib().evoc_gpu_knn_graph(ctx.h, C.byref(o), 1, p(x.data_ptr()), n, d, k, None, p(ind.data_ptr()),
+                                           p(dst.data_ptr()), None)
+        assert st == 0, ctx.last_error()
+        assert ctx.list_stats() == {"tiles": 0, "all_tiles": 0}
+    finally:
+        ctx.close()
