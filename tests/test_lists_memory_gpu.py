@@ -2,6 +2,7 @@
 memory that needs, and gives the same graph.  The GPU's memory is filled by an allocation of torch's;
 a server is given a budget that holds the plain scan only."""
 import ctypes as C
+import gc
 
 import numpy as np
 import pytest
@@ -47,9 +48,18 @@ class _Call:
 
 
 def _fill(leave):
+    gc.collect()
     torch.cuda.empty_cache()
     free, _ = torch.cuda.mem_get_info()
     return torch.empty(max(free - leave, 1), dtype=torch.uint8, device="cuda")
+
+
+@pytest.fixture(autouse=True)
+def _nothing_held():
+    """Contexts that earlier tests share hold pools of freed memory, which the driver would hand out."""
+    for ctx in list(_lib._contexts.values()):
+        ctx.close()
+    _lib._contexts.clear()
 
 
 @pytest.mark.parametrize("kind", ["f32", "i8"])
