@@ -311,12 +311,13 @@ __device__ __forceinline__ uint32_t chunk_mask(const uint32_t (&v)[32], uint32_t
 // (130 candidates) 5.65 (4.3) and at 100 (250) 11.0 (7.0).  Binary rows gain
 // by the set up to kBitsSet keys (k = 130, 300 and 1,000: 6.2, 19.0 and 136
 // against 8.5, 20.5 and 122).  Beside two stages in shared memory (84 to 128
-// keys) the two are level at 100 keys and the heap is ahead at 128 (10,000 x
-// 128 int8: 1.57 against 1.64 ms).
+// keys) the set is ahead at 83 keys (9,653 x 821 f32: 1.52 against 1.56 ms),
+// the two are level at 100 and the heap is ahead at 128 (10,000 x 128 int8: 1.57
+// against 1.64 ms): kNearSet.
 constexpr int kBitsSet = 384;
-template <int MODE, int STAGES, int GROUPS, bool kSmemHeap, bool kList>
-constexpr bool takes_heap =
-    GROUPS == 4 || !kSmemHeap || (STAGES == 2 && GROUPS == 1 && MODE != kModeJaccard && !kList);
+constexpr int kNearSet = 104;
+template <int GROUPS, bool kSmemHeap>
+constexpr bool takes_heap = GROUPS == 4 || !kSmemHeap;
 
 // Symmetric mode, mirror side.  The keys for later rows wait in a per-warp
 // shared-memory stage and go to the mailboxes kMirrorStage at a time: one
@@ -540,7 +541,7 @@ __device__ __forceinline__ bool epilogue_vote(int nthreads, bool ok) {
 }  // namespace
 
 template <int MODE, int STAGES, int GROUPS, bool kSmemHeap, bool kBatch, bool kPair = false, bool kSym = false,
-          bool kList = false, bool kHeap = takes_heap<MODE, STAGES, GROUPS, kSmemHeap, kList>>
+          bool kList = false, bool kHeap = takes_heap<GROUPS, kSmemHeap>>
 __global__ void __launch_bounds__(64 + GROUPS * 128, 1)
 tc_scan_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const ScanParams p) {
   using namespace sm100;
@@ -967,7 +968,7 @@ size_t tc_scan_smem_bytes() { return smem_bytes(4, 1, 0); }
 
 namespace {
 template <int MODE, int STAGES, int GROUPS, bool kSmemHeap, bool kBatch = false,
-          bool kHeap = takes_heap<MODE, STAGES, GROUPS, kSmemHeap, false>>
+          bool kHeap = takes_heap<GROUPS, kSmemHeap>>
 cudaError_t launch_variant(const CUtensorMap& ma, const CUtensorMap& mb, const ScanParams& p, int grid, size_t smem,
                            cudaStream_t stream) {
   auto kern = tc_scan_kernel<MODE, STAGES, GROUPS, kSmemHeap, kBatch, false, false, false, kHeap>;
@@ -1045,6 +1046,14 @@ cudaError_t launch_global(const CUtensorMap& ma, const CUtensorMap& mb, ScanPara
 }
 
 template <int MODE>
+cudaError_t launch_two_stages(const CUtensorMap& ma, const CUtensorMap& mb, const ScanParams& p, int grid, size_t smem,
+                              cudaStream_t stream) {
+  if (MODE != kModeJaccard && p.keep > kNearSet)
+    return launch_variant<MODE, 2, 1, true, false, MODE != kModeJaccard>(ma, mb, p, grid, smem, stream);
+  return launch_variant<MODE, 2, 1, true>(ma, mb, p, grid, smem, stream);
+}
+
+template <int MODE>
 cudaError_t launch_forced(const CUtensorMap& ma, const CUtensorMap& mb, ScanParams p, int grid, int v,
                           cudaStream_t stream) {
   const int odd = p.keep | 1;
@@ -1063,7 +1072,7 @@ cudaError_t launch_forced(const CUtensorMap& ma, const CUtensorMap& mb, ScanPara
     case 11: return launch_variant<MODE, 2, 4, true>(ma, mb, p, grid, smem_bytes(2, 4, odd), stream);
     case 12: return launch_pair<MODE, 5, 1>(ma, mb, p, grid, smem_bytes(5, 1, odd, true), stream);
     case 13: return launch_pair<MODE, 2, 2>(ma, mb, p, grid, smem_bytes(2, 2, odd, true), stream);
-    case 14: return launch_variant<MODE, 2, 1, true>(ma, mb, p, grid, smem_bytes(2, 1, odd), stream);
+    case 14: return launch_two_stages<MODE>(ma, mb, p, grid, smem_bytes(2, 1, odd), stream);
     default: return launch_global<MODE>(ma, mb, p, grid, stream);
   }
 }
@@ -1097,7 +1106,7 @@ cudaError_t launch_mode(const CUtensorMap& ma, const CUtensorMap& mb, ScanParams
   // heaps in shared memory beside two stages beat heaps in global memory by
   // far (each heap insert is a chain of dependent loads)
   if (smem_bytes(2, 1, odd) <= SMEM_LIMIT)
-    return launch_variant<MODE, 2, 1, true>(ma, mb, p, grid, smem_bytes(2, 1, odd), stream);
+    return launch_two_stages<MODE>(ma, mb, p, grid, smem_bytes(2, 1, odd), stream);
   if (!p.scratch) return cudaErrorInvalidValue;
   return launch_global<MODE>(ma, mb, p, grid, stream);
 }
