@@ -312,14 +312,18 @@ bool use_lists(const evoc_gpu_ctx* ctx, int64_t n, int64_t r0, int64_t nq, int64
 // (200,000 x 32 without clusters: int8 17.4 against 15.3 ms, f32 29.7 against
 // 27.0), hence less than a half, and less for the cheaper integer scan.
 //
+// Rows whose cluster has no pivot get one in the second round if the others can
+// be told from them, so a fifth of the sample is enough: 44,000 x 128 f32 in 200
+// clusters (0.32 of the sample) 1.8 to 2.5 against 3.1 ms, 400 (0.18) 2.8 to 3.5,
+// 800 (0.08) 3.8 to 4.6; int8 1.2 to 1.5, 1.6 to 1.9 and 2.0 to 2.5 against 1.6.
 // Up to two rounds of query blocks the plan is a third of a f32 scan and more
 // of an integer one, so fewer tiles may be left: rows nearer to their pivot
 // (24,000 x 96 f32, 50 clusters about a common mean: 1.67 against 1.49 ms), and
-// for integer scans, which are cheaper, pivots in most clusters (24,000 x 96
-// int8: 20 clusters 0.61 against 0.76 ms, 50 about a mean 0.95).  Binary rows
-// whose pivots miss most clusters lose at any size (60,000 x 1,024 bits: 300
-// clusters 6.3 against 5.5 ms, 100 3.8 against 5.7).  A sample that declines
-// costs 35 us.
+// for integer scans, which are cheaper, pivots in most clusters (28,000 x 128
+// int8, 50 clusters (0.66) 0.63 against 0.83 ms, 100 (0.40) 0.75 to 1.02, 200
+// (0.23) 0.92 to 1.04).  Binary rows whose pivots miss most clusters lose at any
+// size (70,000 x 512 bits in 100 clusters (0.76) 3.5 to 4.6 against 6.2 ms, 200
+// (0.51) 5.7 to 7.2, 400 (0.29) 7.5 to 8.1).  A sample that declines costs 35 us.
 struct FitRule {
   float part;    // of the distance to the pivots' mean (1 - cosine) that the nearest pivot's may be
   float sample;  // share of the sample that must be as near
@@ -327,8 +331,8 @@ struct FitRule {
 FitRule fit_rule(const evoc_gpu_ctx* ctx, int mode, int64_t n) {
   const bool few = n <= int64_t(256) * ctx->sms;
   if (mode == evoc::kScanJaccard) return few ? FitRule{0.2f, 0.75f} : FitRule{0.25f, 0.5f};
-  if (mode == evoc::kScanInt8) return few ? FitRule{0.3f, 0.75f} : FitRule{0.35f, 0.25f};
-  return {few ? 0.3f : 0.4f, 0.25f};
+  if (mode == evoc::kScanInt8) return few ? FitRule{0.3f, 0.5f} : FitRule{0.35f, 0.2f};
+  return {few ? 0.3f : 0.4f, 0.2f};
 }
 
 // Plans the lists of a self-join of all rows and scans over them; *taken is
