@@ -2,7 +2,7 @@
 //
 // A batch lives in device tables: a header with the counts and one status
 // word, one BatchRowJob per request for the row kernels (copy and pad,
-// prepare_float, 16-bit conversion, FP32 rerank), one ScanJob per request for
+// row preparation, FP32 rerank), one ScanJob per request for
 // the tensor-core scan (its two tensor maps and scan parameters) and a
 // work-list of (request, 128-row query block) items.  Every kernel reads its
 // counts and pointers from these tables, so its launch parameters do not
@@ -38,7 +38,7 @@ struct BatchRowJob {
   float* x;                // f32 padded rows (f32 requests)
   uint8_t* xb;             // 16-bit or int8 padded rows
   float* norms;            // f32 row norms (f32 requests)
-  int32_t* flag;           // prepare_float: some row's norm is off by > 1e-5
+  int32_t* flag;           // some row's norm is off by > 1e-5
   int32_t* cand;           // n x C scan candidates (f32 requests)
   int32_t C, keff;         // candidates kept per row, neighbours returned
   int32_t* out_idx;
@@ -85,7 +85,7 @@ cudaError_t prepare_tc_scan_batch(int mode, int max_keep);
 cudaError_t launch_tc_scan_batch(int mode, BatchHeader* hdr, const ScanJob* jobs, const ScanItem* items,
                                  int max_keep, int grid, uint64_t timeout_ns, cudaStream_t stream, int half_type);
 
-// prep.cu.  f32 requests: copy + pad into x, prepare_float, 16-bit rows into
+// prep.cu.  f32 requests: copy + pad into x, normalisation, 16-bit rows into
 // xb (with the certificate's norms).  i8 requests: copy + pad into xb.
 // Grids are sized by the caller for the batch (grid-stride loops cover any
 // count), so a small batch occupies a few SMs and runs beside other work.
