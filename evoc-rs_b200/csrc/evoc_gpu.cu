@@ -1273,6 +1273,7 @@ int run_nndescent(evoc_gpu_ctx* ctx, const evoc_gpu_opts& opts, const Job& j, in
     a.label = ctx->labels.as<int32_t>();
     a.cell_end = ctx->cursor.as<int32_t>();
     a.cell_cnt = ctx->hist.as<int32_t>();
+    a.cells = int(pivot_count(n));
   }
   const size_t nk = size_t(n) * size_t(k);
   size_t sizes[kNndParts];

@@ -352,6 +352,7 @@ struct NndArgs {
   const int32_t* label;   // pivot cell of each row or null
   const int32_t* cell_end;
   const int32_t* cell_cnt;
+  int cells;
   uint64_t seed;
   uint64_t* keys[2];      // n x k sorted (raw, index) keys, double buffered
   uint8_t* isnew[2];      // n x k flags

@@ -212,7 +212,7 @@ template <int DT>
 __global__ void __launch_bounds__(NW * 32)
 nnd_init_kernel(const uint8_t* __restrict__ X, int64_t row_bytes, const int32_t* __restrict__ pc, int64_t n, int k,
                 const int32_t* __restrict__ order, const int32_t* __restrict__ label,
-                const int32_t* __restrict__ cell_end, const int32_t* __restrict__ cell_cnt, uint64_t seed,
+                const int32_t* __restrict__ cell_end, const int32_t* __restrict__ cell_cnt, int cells, uint64_t seed,
                 uint64_t* __restrict__ keys, uint8_t* __restrict__ isnew) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kr = label ? k / 3 : k;  // slots for random rows
@@ -223,7 +223,8 @@ nnd_init_kernel(const uint8_t* __restrict__ X, int64_t row_bytes, const int32_t*
     if (kc > 0) cell.insert(make_key(-1.0f, int32_t(u)), kc, lane);
     else rnd.insert(make_key(-1.0f, int32_t(u)), kr, lane);
     if (label && kc > 0) {
-      const int lb = label[u];
+      // a row that holds a NaN has no nearest pivot (-1); it was counted in the first cell
+      const int lb = label[u] < 0 || label[u] >= cells ? 0 : label[u];
       const int64_t cn = cell_cnt[lb], c0 = cell_end[lb] - cn;
       for (int t = 0; t < 2 * kc + 8 && cn > 1; t += 4) {
         int32_t b[4];
@@ -488,7 +489,8 @@ template <int DT>
 cudaError_t nnd_run(const NndArgs& a, cudaStream_t stream) {
   const int blocks = a.sms * 8;
   nnd_init_kernel<DT><<<blocks, NW * 32, 0, stream>>>(a.X, a.row_bytes, a.pc, a.n, a.k, a.order, a.label, a.cell_end,
-                                                      a.cell_cnt, a.seed, a.keys[0], a.isnew[0]);
+                                                      a.cell_cnt, a.cells, a.seed, a.keys[0],
+                                                      a.isnew[0]);
   return cudaGetLastError();
 }
 
