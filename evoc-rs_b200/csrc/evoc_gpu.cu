@@ -2053,7 +2053,8 @@ void evoc_gpu_ctx_destroy(evoc_gpu_ctx* ctx) {
                     &ctx->out_raw,  &ctx->out_dist, &ctx->xb,   &ctx->cand,   &ctx->labels,
                     &ctx->order,    &ctx->hist,    &ctx->cursor, &ctx->pivots, &ctx->popc,
                     &ctx->g_idx,    &ctx->g_dist,  &ctx->g_sigma, &ctx->g_rho, &ctx->g_indptr,
-                    &ctx->g_indices, &ctx->g_data, &ctx->g_work, &ctx->nnd_work, &ctx->cert, &ctx->repair, &ctx->prune};
+                    &ctx->g_indices, &ctx->g_data, &ctx->g_work, &ctx->nnd_work, &ctx->cert, &ctx->repair, &ctx->sym,
+                    &ctx->prune};
   for (DevBuf* b : bufs) b->release();
   for (auto& g : ctx->batch_graphs) cudaGraphExecDestroy(g.exec);
   ctx->batch_ws.release();
